@@ -16,6 +16,8 @@ SIGNATURES = {
     "actnn_compress_single": ['P', 'I', 'P', 'P', 'P', 'P', 'L', 'L', 'L', 'I', 'I', 'I', 'P', 'U', 'U', 'P'],
     "actnn_compress_mixed": ['P', 'P', 'P', 'P', 'P', 'P', 'P', 'P', 'L', 'L', 'L', 'L', 'I', 'I', 'F', 'F', 'P', 'I', 'D', 'I', 'P',
                              'U', 'U', 'P'],
+    "actnn_compress_mixed_samples": ['P'] * 8 + ['L', 'L', 'L', 'I', 'I', 'F', 'F', 'P', 'I', 'D', 'I', 'P', 'U', 'U', 'P'],
+    "actnn_unpack_mixed_samples": ['P', 'P', 'P', 'P', 'P', 'P', 'L', 'L', 'I', 'I', 'P'],
     "actnn_compress_mixed_static": ['P', 'P', 'P', 'P', 'P', 'P', 'P', 'L', 'L', 'L', 'I', 'I', 'F', 'F', 'P', 'I', 'D', 'I', 'P', 'U',
                                     'U', 'P'],
     "actnn_compress_mixed_prestat": ['P', 'P', 'P', 'P', 'P', 'P', 'P', 'P', 'P', 'P', 'L', 'L', 'L', 'I', 'I', 'F', 'F', 'P', 'I', 'D', 'I',

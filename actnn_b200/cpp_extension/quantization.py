@@ -115,6 +115,26 @@ def compress_mixed_precision(data, target_bits: int, initial_bits: int, range_fa
     check_cuda_tensor(data, "data", 3)
     n, g, gs = data.shape
     _check_group_size(gs)
+    return _compress_mixed(data, n, g, gs, None, target_bits, initial_bits, range_factor, coeff, grad_scale,
+                           stochastic, noise, philox, stat_dtype, minmax)
+
+
+def compress_mixed_samples(data, target_bits: int, initial_bits: int, range_factor: float, coeff: float = 1.0,
+                           grad_scale=None, stochastic=True, *, noise=None, philox=None, stat_dtype=None):
+    """``compress_mixed_precision`` of ``data [N, F]`` for any ``F``: the last group of 256 of every
+    sample is completed with zeros that exist only in the kernels, where the reference
+    concatenates a padded copy (actnn/actnn/qscheme.py:61-71).  ``noise``: ``[N, G, 256]``."""
+    check_cuda_tensor(data, "data", 2)
+    n, f = data.shape
+    if noise is not None and stochastic and noise.numel() != n * ((f + 255) // 256) * 256:
+        raise RuntimeError("noise must have as many elements as the padded data!")
+    return _compress_mixed(data, n, (f + 255) // 256, 256, f, target_bits, initial_bits, range_factor, coeff,
+                           grad_scale, stochastic, noise, philox, stat_dtype, None)
+
+
+def _compress_mixed(data, n, g, gs, features, target_bits, initial_bits, range_factor, coeff, grad_scale, stochastic,
+                    noise, philox, stat_dtype, minmax):
+    """The body of the two entries above; ``features`` is ``None`` for whole groups."""
     sdt = _stat_dtype(data.dtype, stat_dtype)
     total = min(initial_bits * n, max(int(target_bits), n))        # what the greedy ends with
     dev = data.device
@@ -127,7 +147,11 @@ def compress_mixed_precision(data, target_bits: int, initial_bits: int, range_fa
     if grad_scale is not None and (grad_scale.dtype != torch.float32 or not grad_scale.is_cuda
                                    or grad_scale.numel() != 1):
         raise RuntimeError("grad_scale must be a float32 CUDA tensor with one element!")
-    nz, seed, offset = _noise_args(data, stochastic, noise, philox)
+    if features is not None and noise is not None and stochastic:
+        check_cuda_tensor(noise, "noise", dtype=data.dtype)
+        nz, seed, offset = noise.data_ptr(), 0, 0
+    else:
+        nz, seed, offset = _noise_args(data, stochastic, noise, philox)
     if minmax is not None:
         gmn, gmx = minmax
         check_cuda_tensor(gmn, "min", dtype=data.dtype)
@@ -146,8 +170,10 @@ def compress_mixed_precision(data, target_bits: int, initial_bits: int, range_fa
         return packed, bits, scale, mn, C
     ws_bytes = 2 * ((n * g * data.element_size() + 255) // 256 * 256) + 256     # actnn_compress_mixed_workspace
     workspace = _lib.scratch(dev, ws_bytes)
-    _lib.call("actnn_compress_mixed", data, data.data_ptr(), packed.data_ptr(), scale.data_ptr(), mn.data_ptr(),
-              bits.data_ptr(), offsets.data_ptr(), C.data_ptr(), workspace.data_ptr(), ws_bytes, n, g, gs,
+    name, shape = ("actnn_compress_mixed", (n, g, gs)) if features is None else \
+        ("actnn_compress_mixed_samples", (n, features))
+    _lib.call(name, data, data.data_ptr(), packed.data_ptr(), scale.data_ptr(), mn.data_ptr(),
+              bits.data_ptr(), offsets.data_ptr(), C.data_ptr(), workspace.data_ptr(), ws_bytes, *shape,
               _lib.dtype_id(data.dtype), _lib.dtype_id(sdt), float(range_factor), float(coeff),
               _lib.ptr(grad_scale), int(initial_bits), float(target_bits), int(bool(stochastic)), nz, seed, offset,
               _lib.stream_of(data))
@@ -176,6 +202,28 @@ def unpack_mixed_precision(data, bits, scale, min, N, num_groups, group_size, *,
     _lib.call("actnn_unpack_mixed", data, data.data_ptr(), bits.data_ptr(), word_offsets.data_ptr(),
               scale.data_ptr(), min.data_ptr(), out.data_ptr(), N, num_groups, group_size,
               _lib.dtype_id(out_dtype), _lib.dtype_id(scale.dtype), _lib.stream_of(data))
+    return out
+
+
+def unpack_mixed_samples(data, bits, scale, min, shape, *, out_dtype=None):
+    """``unpack_mixed_precision`` of groups of 256 straight into a new tensor of ``shape``, whose
+    samples need not be whole groups (no padded intermediate)."""
+    check_cuda_tensor(data, "data", 1, torch.int32)
+    check_cuda_tensor(bits, "bits", 1, torch.int32)
+    check_cuda_tensor(scale, "scale", 3)
+    check_cuda_tensor(min, "min", 3, scale.dtype)
+    out_dtype = scale.dtype if out_dtype is None else out_dtype
+    _stat_dtype(out_dtype, scale.dtype)
+    n, g = scale.shape[0], scale.shape[1]
+    word_offsets = getattr(data, "word_offsets", None)
+    if word_offsets is None:
+        word_offsets = bits_prefix(bits, g, 256)
+    out = torch.empty(shape, dtype=out_dtype, device=data.device)
+    if out.shape[0] != n or bits.numel() != n or (out.numel() // n + 255) // 256 != g:
+        raise RuntimeError("unpack_mixed_samples: the statistics do not belong to a tensor of this shape")
+    _lib.call("actnn_unpack_mixed_samples", data, data.data_ptr(), bits.data_ptr(), word_offsets.data_ptr(),
+              scale.data_ptr(), min.data_ptr(), out.data_ptr(), n, out.numel() // n, _lib.dtype_id(out_dtype),
+              _lib.dtype_id(scale.dtype), _lib.stream_of(data))
     return out
 
 

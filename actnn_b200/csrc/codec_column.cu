@@ -1,0 +1,237 @@
+// The mixed-precision codec on [N, F] activations whose samples are not whole groups of 256, or not
+// a multiple of four groups: min / max, pack and unpack on the column mapping (column.cuh), reading
+// and writing the activation where it is.  (The reference pads every sample with a concatenation
+// and strips the padding with a copy, actnn/actnn/qscheme.py:61-71 and ops.py:137-139.)
+//
+// Bound by HBM at large sizes and by launches at small ones.  float16, compress and decompress of
+// 100 x 192 x 35 x 35 (918.75 groups a sample): 127.1 -> 60.6 us, of which the padded copy was 18 and the
+// cut-out copy 49; 8 x 16 x 14 x 14: 81.1 -> 46.4 us (seven kernels -> four).
+#include "column.cuh"
+
+namespace actnn {
+namespace {
+
+// min / max of every group.  `clear_word` (optional) is set to zero: the ticket of the next kernel.
+// Samples are walked from the last to the first, the order that leaves what the pack reads first
+// in the L2.
+template <typename T, bool EDGE>
+__global__ void __launch_bounds__(kColThreads)
+column_minimax_kernel(const T* __restrict__ data, ColumnShape sh, T* __restrict__ mn, T* __restrict__ mx,
+                      unsigned* __restrict__ clear_word) {
+  const int lane = threadIdx.x & 31;
+  if (clear_word && blockIdx.x == 0 && threadIdx.x == 0) *clear_word = 0u;
+  const ColumnTask t = column_task(sh);
+  if (!t.valid) return;
+  const ColumnOctets<EDGE> oct(sh, t, lane);
+  Oct<T> next[kBundle];
+  oct.template load<T>(data + (int64_t)(t.n1 - 1) * sh.F, next);
+  for (int n = t.n1 - 1; n >= t.n0; --n) {
+    Oct<T> x[kBundle];
+#pragma unroll
+    for (int gi = 0; gi < kBundle; ++gi) x[gi] = next[gi];
+    if (n > t.n0) oct.template load<T>(data + (int64_t)(n - 1) * sh.F, next);
+    float lo = 0.f, hi = 0.f;
+    bundle_minmax<T>(x, lane, lo, hi);
+    if (lane < t.count) {
+      const int64_t q = (int64_t)n * sh.G + t.g0 + lane;
+      store_scalar<T>(mn, q, lo);
+      store_scalar<T>(mx, q, hi);
+    }
+  }
+}
+
+// Scale, stochastic rounding and pack.  Eight samples at a time: lane 4i + g prepares group g of
+// the i-th of them (one division per lane for eight bundles).  The noise octets are formed before
+// the dispatch on the width, so the eight width variants stay short.
+template <typename T, typename ST, bool PHILOX, bool EDGE>
+__global__ void __launch_bounds__(kColThreads, 2)
+column_pack_kernel(const T* __restrict__ data, ColumnShape sh, const T* __restrict__ mn, const T* __restrict__ mx,
+                   const int32_t* __restrict__ bits, const int64_t* __restrict__ word_offsets,
+                   int32_t* __restrict__ packed, ST* __restrict__ scale, ST* __restrict__ mn_out,
+                   const T* __restrict__ noise, const NoiseKey key) {
+  const int lane = threadIdx.x & 31;
+  const ColumnTask t = column_task(sh);
+  if (!t.valid) return;
+  const ColumnOctets<EDGE> oct(sh, t, lane);
+  const TransposePlan plan = make_transpose_plan(lane);
+  Oct<T> next[kBundle];
+  oct.template load<T>(data + (int64_t)t.n0 * sh.F, next);
+  for (int nb = t.n0; nb < t.n1; nb += 8) {
+    const int n_l = nb + (lane >> 2), g_l = lane & 3;
+    int b_l = 0;
+    int64_t off_l = 0;
+    LaneParams<T> mine = {0u, 0u};
+    if (n_l < t.n1 && g_l < t.count) {
+      b_l = __ldg(bits + n_l);
+      if (b_l < 1 || b_l > 8) b_l = 0;                   // not a width: nothing written
+      off_l = __ldg(word_offsets + n_l) + (int64_t)t.g0 * 8 * b_l;
+      const int64_t q = (int64_t)n_l * sh.G + t.g0 + g_l;
+      const float gmn = load_scalar<T>(mn, q), gmx = load_scalar<T>(mx, q);
+      const GroupParams gp = prepare_group<T>(gmn, gmx, b_l);
+      store_scalar<ST>(scale, q, gp.scale);
+      store_scalar<ST>(mn_out, q, gmn);
+      mine = lane_params<T>(gp);
+    }
+    const int cnt = min(8, t.n1 - nb);
+    for (int i = 0; i < cnt; ++i) {
+      const int n = nb + i;
+      Oct<T> x[kBundle], nz[kBundle];
+#pragma unroll
+      for (int gi = 0; gi < kBundle; ++gi) x[gi] = next[gi];
+      if (n + 1 < t.n1) oct.template load<T>(data + (int64_t)(n + 1) * sh.F, next);
+      const int64_t q0 = (int64_t)n * sh.G + t.g0;
+      if constexpr (PHILOX) {
+        noise_bundle<T>(key, q0, lane, nz);
+      } else {                                           // an injected tensor shaped [N, G, 256], or none
+#pragma unroll
+        for (int gi = 0; gi < kBundle; ++gi)
+          nz[gi] = noise && gi < t.count ? load_oct<T>(noise + (q0 + gi) * kGroup + lane * kOct) : zero_oct<T>();
+      }
+      const int b = __shfl_sync(kFull, b_l, 4 * i);
+      const uint32_t olo = __shfl_sync(kFull, (uint32_t)off_l, 4 * i);
+      const uint32_t ohi = __shfl_sync(kFull, (uint32_t)((uint64_t)off_l >> 32), 4 * i);
+      int32_t* out = packed + (int64_t)(((uint64_t)ohi << 32) | olo);
+#define ACTNN_CASE(B) \
+      case B: pack_column_bundle<T, B>(x, nz, mine, 4 * i, t.count, out, plan, lane); break;
+      switch (b) {
+        ACTNN_CASE(1) ACTNN_CASE(2) ACTNN_CASE(3) ACTNN_CASE(4) ACTNN_CASE(5) ACTNN_CASE(6) ACTNN_CASE(7)
+        ACTNN_CASE(8)
+        default: break;
+      }
+#undef ACTNN_CASE
+    }
+  }
+}
+
+template <typename T, typename ST, bool EDGE>
+__global__ void __launch_bounds__(kColThreads, 3)
+column_unpack_kernel(const int32_t* __restrict__ packed, const int32_t* __restrict__ bits,
+                     const int64_t* __restrict__ word_offsets, const ST* __restrict__ scale,
+                     const ST* __restrict__ mn, ColumnShape sh, T* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const ColumnTask t = column_task(sh);
+  if (!t.valid) return;
+  const ColumnOctets<EDGE> oct(sh, t, lane);
+  const TransposePlan plan = make_transpose_plan(lane);
+  for (int nb = t.n0; nb < t.n1; nb += 32) {
+    const int nl = min(32, t.n1 - nb);
+    ColumnStream st;
+    st.open(t, nb, nl, bits, word_offsets, lane);
+    uint32_t wn[8];
+    float scn, mn_n;
+    int bn = st.fetch<ST>(t, sh.G, nb, 0, packed, scale, mn, lane, wn, scn, mn_n);
+    for (int i = 0; i < nl; ++i) {
+      uint32_t w[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w[k] = wn[k];
+      const int b = bn;
+      const float sc = scn, m = mn_n;
+      if (i + 1 < nl) bn = st.fetch<ST>(t, sh.G, nb, i + 1, packed, scale, mn, lane, wn, scn, mn_n);
+      if (b == 0) continue;                              // the pack wrote nothing for this sample either
+      Oct<T> x[kBundle];
+      decode_column<T>(b, w, sc, m, plan, lane, x);
+      oct.template store<T>(out + (int64_t)(nb + i) * sh.F, x);
+    }
+  }
+}
+
+constexpr int kPackWarps = 16, kUnpackWarps = 24, kMinimaxWarps = 32;     // resident warps per SM the grids are sized for
+
+template <typename T>
+int launch_minimax(const void* data, void* mn, void* mx, int64_t N, int64_t F, unsigned* clear_word, cudaStream_t s) {
+  const int al = octet_alignment(data, F, sizeof(T));
+  const ColumnShape sh = column_shape(N, F, al, kMinimaxWarps);
+  const bool edge = al != kOct || F % kGroup != 0;
+  auto kernel = edge ? column_minimax_kernel<T, true> : column_minimax_kernel<T, false>;
+  kernel<<<column_grid(sh), kColThreads, 0, s>>>((const T*)data, sh, (T*)mn, (T*)mx, clear_word);
+  return check_launch();
+}
+
+template <typename T, typename ST>
+int launch_pack(const void* data, const void* mn, const void* mx, const int32_t* bits, const int64_t* word_offsets,
+                int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t F, int stochastic, const void* noise,
+                uint64_t seed, uint64_t offset, cudaStream_t s) {
+  const int al = octet_alignment(data, F, sizeof(T));
+  const ColumnShape sh = column_shape(N, F, al, kPackWarps);
+  const bool edge = al != kOct || F % kGroup != 0;
+  const bool philox = stochastic && !noise;
+  const NoiseKey key = make_noise_key(seed, offset);
+  auto kernel = philox ? (edge ? column_pack_kernel<T, ST, true, true> : column_pack_kernel<T, ST, true, false>)
+                       : (edge ? column_pack_kernel<T, ST, false, true> : column_pack_kernel<T, ST, false, false>);
+  kernel<<<column_grid(sh), kColThreads, 0, s>>>((const T*)data, sh, (const T*)mn, (const T*)mx, bits, word_offsets,
+                                                 packed, (ST*)scale, (ST*)mn_out,
+                                                 (const T*)(stochastic ? noise : nullptr), key);
+  return check_launch();
+}
+
+template <typename T, typename ST>
+int launch_unpack(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets, const void* scale,
+                  const void* mn, void* out, int64_t N, int64_t F, cudaStream_t s) {
+  const int al = octet_alignment(out, F, sizeof(T));
+  const ColumnShape sh = column_shape(N, F, al, kUnpackWarps);
+  const bool edge = al != kOct || F % kGroup != 0;
+  auto kernel = edge ? column_unpack_kernel<T, ST, true> : column_unpack_kernel<T, ST, false>;
+  kernel<<<column_grid(sh), kColThreads, 0, s>>>(packed, bits, word_offsets, (const ST*)scale, (const ST*)mn, sh,
+                                                 (T*)out);
+  return check_launch();
+}
+
+}  // namespace
+
+int column_minimax(const void* data, void* mn, void* mx, int64_t N, int64_t F, int dtype, unsigned* clear_word,
+                   cudaStream_t s) {
+  if (!column_supported(N, F)) return ACTNN_ERR_SHAPE;
+  switch (dtype) {
+    case ACTNN_F32: return launch_minimax<float>(data, mn, mx, N, F, clear_word, s);
+    case ACTNN_F16: return launch_minimax<__half>(data, mn, mx, N, F, clear_word, s);
+    case ACTNN_BF16: return launch_minimax<__nv_bfloat16>(data, mn, mx, N, F, clear_word, s);
+    default: return ACTNN_ERR_DTYPE;
+  }
+}
+
+int column_pack(const void* data, const void* mn, const void* mx, const int32_t* bits, const int64_t* word_offsets,
+                int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t F, int dtype, int stat_dtype,
+                int stochastic, const void* noise, uint64_t seed, uint64_t offset, cudaStream_t s) {
+  if (!column_supported(N, F)) return ACTNN_ERR_SHAPE;
+  if (stochastic && noise && !aligned(noise, dtype == ACTNN_F32 ? 32 : 16)) return ACTNN_ERR_ALIGN;
+#define ACTNN_PACK(T, ST)                                                                                         \
+  return launch_pack<T, ST>(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, F, stochastic, noise, seed, \
+                            offset, s)
+  switch (dtype) {
+    case ACTNN_F16: ACTNN_PACK(__half, __half);
+    case ACTNN_BF16: ACTNN_PACK(__nv_bfloat16, __nv_bfloat16);
+    default:
+      if (stat_dtype == ACTNN_BF16) ACTNN_PACK(float, __nv_bfloat16);
+      ACTNN_PACK(float, float);
+  }
+#undef ACTNN_PACK
+}
+
+int column_unpack(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets, const void* scale,
+                  const void* mn, void* out, int64_t N, int64_t F, int dtype, int stat_dtype, cudaStream_t s) {
+  if (!column_supported(N, F)) return ACTNN_ERR_SHAPE;
+#define ACTNN_UNPACK(T, ST) return launch_unpack<T, ST>(packed, bits, word_offsets, scale, mn, out, N, F, s)
+  switch (dtype) {
+    case ACTNN_F16: ACTNN_UNPACK(__half, __half);
+    case ACTNN_BF16: ACTNN_UNPACK(__nv_bfloat16, __nv_bfloat16);
+    default:
+      if (stat_dtype == ACTNN_BF16) ACTNN_UNPACK(float, __nv_bfloat16);
+      ACTNN_UNPACK(float, float);
+  }
+#undef ACTNN_UNPACK
+}
+}  // namespace actnn
+
+using namespace actnn;
+
+extern "C" int actnn_unpack_mixed_samples(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets,
+                                          const void* scale, const void* mn, void* out, int64_t N, int64_t F,
+                                          int dtype, int stat_dtype, actnn_stream_t stream) {
+  if (N < 0 || F < 0) return ACTNN_ERR_SHAPE;
+  if (dtype < ACTNN_F32 || dtype > ACTNN_BF16) return ACTNN_ERR_DTYPE;
+  if (!(stat_dtype == dtype || (dtype == ACTNN_F32 && stat_dtype == ACTNN_BF16))) return ACTNN_ERR_DTYPE;
+  if (N == 0 || F == 0) return ACTNN_OK;
+  if (!packed || !bits || !word_offsets || !scale || !mn || !out) return ACTNN_ERR_NULL;
+  if (!aligned(out, dtype_size(dtype)) || !aligned(packed, 4)) return ACTNN_ERR_ALIGN;
+  return column_unpack(packed, bits, word_offsets, scale, mn, out, N, F, dtype, stat_dtype, (cudaStream_t)stream);
+}

@@ -11,12 +11,11 @@
 // string across the warp yields output words 32k .. 32k+31 of the bundle, lane w holding
 // word 32k + w, so every store is one fully coalesced 128-byte line.  No shared memory,
 // no atomics, no block-level synchronisation.
-#include "quant_math.cuh"
+#include "mixed_bundle.cuh"
 
 namespace actnn {
 namespace {
 
-constexpr int kBundle = 4;            // groups per warp task
 constexpr int kThreads = 256;
 
 struct BundleCoord {
@@ -171,7 +170,6 @@ pack_mixed_kernel(const T* __restrict__ data, const T* __restrict__ mn, const T*
 //     current one is quantized: a warp always has loads in flight.
 constexpr int kFlatGroups = 32;       // groups per task
 constexpr int kFlatBundle = 4;        // groups per bundle
-enum NoiseMode { kNoisePhilox = 0, kNoiseTensor = 1, kNoiseNone = 2 };
 #ifndef ACTNN_FLAT_BLOCKS
 #define ACTNN_FLAT_BLOCKS 2
 #endif
@@ -180,32 +178,6 @@ enum NoiseMode { kNoisePhilox = 0, kNoiseTensor = 1, kNoiseNone = 2 };
 #endif
 constexpr int kFlatUnpackBlocks = ACTNN_FLAT_UNPACK_BLOCKS;
 constexpr int kFlatBlocks16 = ACTNN_FLAT_BLOCKS;   // resident blocks per SM the flat kernels are compiled for (16-bit types)
-
-// (mn', scale) of the lane's own group in the form the quantizer consumes.
-template <typename T> struct LaneParams { uint32_t a, b; };
-template <typename T> ACTNN_DEV LaneParams<T> lane_params(const GroupParams& gp) {
-  LaneParams<T> p;
-  if constexpr (sizeof(T) == 4) {
-    p.a = __float_as_uint(gp.mn1);
-    p.b = __float_as_uint(gp.scale);
-  } else {
-    p.a = bits_of<T>(gp.mn1) * 0x00010001u;
-    p.b = bits_of<T>(gp.scale) * 0x00010001u;
-  }
-  return p;
-}
-template <typename T> ACTNN_DEV QP<T> fetch_lane_params(const LaneParams<T>& mine, int src_lane) {
-  const uint32_t a = __shfl_sync(kFull, mine.a, src_lane), b = __shfl_sync(kFull, mine.b, src_lane);
-  QP<T> q;
-  if constexpr (sizeof(T) == 4) {
-    q.mn1 = __uint_as_float(a);
-    q.scale = __uint_as_float(b);
-  } else {
-    q.mn2 = *reinterpret_cast<const decltype(q.mn2)*>(&a);
-    q.sc2 = *reinterpret_cast<const decltype(q.sc2)*>(&b);
-  }
-  return q;
-}
 
 template <typename T, int B, int MODE, bool CLAMP_LOW>
 ACTNN_DEV void pack_flat_bundle(const Oct<T> (&x)[kFlatBundle], const LaneParams<T>& mine, int first_lane,
@@ -362,148 +334,6 @@ pack_mixed_flat_kernel(const T* __restrict__ data, const T* __restrict__ mn, con
 // and the elements look theirs up: for 16-bit types and B <= 2 the table of a group fits
 // two registers and a byte-permute picks two elements per instruction; otherwise a warp
 // shuffle fetches the entry; from 6 bits on the division is done per element.
-template <int B> ACTNN_DEV uint32_t spread_codes_to_bytes(uint32_t r) {   // four B-bit codes -> one per byte
-  if constexpr (B == 2) {
-    uint32_t t = (r | (r << 12)) & 0x000f000fu;
-    return (t | (t << 6)) & 0x03030303u;
-  } else {
-    uint32_t t = (r | (r << 14)) & 0x00030003u;
-    return (t | (t << 7)) & 0x01010101u;
-  }
-}
-
-// `words[k]` is word 32k + lane of the bundle (zero past its end); lanes 0..count-1 hold the
-// statistics of their group in (stat_scale, stat_mn).  Both were loaded ahead of time.
-template <typename T, int B>
-ACTNN_DEV void unpack_bundle(const uint32_t (&words)[8], float stat_scale, float stat_mn, const BundleCoord& c,
-                             T* __restrict__ out, const TransposePlan& plan, int lane) {
-  constexpr int E = 1 << (B < 6 ? B : 5);              // table entries per group
-  constexpr int GPC = (32 / E) < kBundle ? (32 / E) : kBundle;   // groups served by one table computation
-  uint32_t S[B];
-#pragma unroll
-  for (int k = 0; k < B; ++k) S[k] = warp_transpose32(words[k], plan);
-  uint32_t entry = 0u, pairs = 0u;
-#pragma unroll
-  for (int gi = 0; gi < kBundle; ++gi) {
-    if constexpr (B < 6) {
-      if (gi % GPC == 0) {                               // (re)build the table for groups gi .. gi+GPC-1
-        const int g = (gi + lane / E) & (kBundle - 1);
-        const float sc = __shfl_sync(kFull, stat_scale, g), m = __shfl_sync(kFull, stat_mn, g);
-        entry = dequant_bits<T>((float)(lane % E), sc, m);
-        if constexpr (sizeof(T) == 2 && B <= 2)
-          pairs = entry | (__shfl_down_sync(kFull, entry, 1) << 16);
-      }
-    }
-    uint32_t lo = 0u, hi = 0u;                           // this group's row
-    if (gi == 0) { lo = get_bits<0 * 8 * B, (8 * B < 32 ? 8 * B : 32)>(S); if constexpr (8 * B > 32) hi = get_bits<0 * 8 * B + 32, 8 * B - 32>(S); }
-    if (gi == 1) { lo = get_bits<1 * 8 * B, (8 * B < 32 ? 8 * B : 32)>(S); if constexpr (8 * B > 32) hi = get_bits<1 * 8 * B + 32, 8 * B - 32>(S); }
-    if (gi == 2) { lo = get_bits<2 * 8 * B, (8 * B < 32 ? 8 * B : 32)>(S); if constexpr (8 * B > 32) hi = get_bits<2 * 8 * B + 32, 8 * B - 32>(S); }
-    if (gi == 3) { lo = get_bits<3 * 8 * B, (8 * B < 32 ? 8 * B : 32)>(S); if constexpr (8 * B > 32) hi = get_bits<3 * 8 * B + 32, 8 * B - 32>(S); }
-    Oct<T> o;
-    uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-    if constexpr (sizeof(T) == 2 && B <= 2) {
-      const int base = (gi % GPC) * E;
-      const uint32_t t01 = __shfl_sync(kFull, pairs, base);
-      const uint32_t t23 = B == 2 ? __shfl_sync(kFull, pairs, base + 2) : t01;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {                      // four elements per step
-        const uint32_t y = spread_codes_to_bytes<B>((lo >> (4 * B * h)) & ((1u << (4 * B)) - 1u));
-        const uint32_t sel = y * 0x22u + 0x10101010u;    // byte pair (2c, 2c+1) per element
-        ow[2 * h] = __byte_perm(t01, t23, sel);
-        ow[2 * h + 1] = __byte_perm(t01, t23, sel >> 16);
-      }
-    } else {
-      uint32_t v[8];
-      const uint32_t S2[2] = {lo, hi};
-      uint32_t code[8];
-      get_codes<B, 0>(S2, code);
-      if constexpr (B < 6) {
-        const int base = (gi % GPC) * E;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __shfl_sync(kFull, entry, base + (int)code[j]);
-      } else {
-        const float sc = __shfl_sync(kFull, stat_scale, gi), m = __shfl_sync(kFull, stat_mn, gi);
-        float y = 0.f;
-        if (sizeof(T) == 2 && group_reciprocal(sc, y)) {           // 16-bit statistics; warp-uniform
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = dequant_bits_recip<T>((float)code[j], sc, y, m);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = dequant_bits<T>((float)code[j], sc, m);
-        }
-      }
-      if constexpr (sizeof(T) == 4) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ow[j] = v[j];
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) ow[k] = v[2 * k] | (v[2 * k + 1] << 16);
-      }
-    }
-    if (gi < c.count) store_oct_streaming<T>(out + (c.q0 + gi) * kGroup + lane * kOct, o);
-  }
-}
-
-template <typename T, typename ST>
-__global__ void __launch_bounds__(kThreads, 4)
-unpack_mixed_kernel(const int32_t* __restrict__ packed, const int32_t* __restrict__ bits,
-                    const int64_t* __restrict__ word_offsets, const ST* __restrict__ scale,
-                    const ST* __restrict__ mn, T* __restrict__ out, int64_t N, int64_t G) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
-  const TransposePlan plan = make_transpose_plan(lane);
-
-  // A bundle's input is only b * 128 bytes per warp: issue the loads of DEPTH bundles before
-  // decoding the first, so that enough bytes are in flight to cover the memory latency.
-  constexpr int DEPTH = 2;
-  BundleWalker walk(warp, nwarps, N, G);
-  while (walk.valid()) {
-    BundleCoord t_c[DEPTH];
-    int t_b[DEPTH];
-    bool t_ok[DEPTH];
-    uint32_t t_w[DEPTH][8];
-    float t_sc[DEPTH], t_m[DEPTH];
-#pragma unroll
-    for (int d = 0; d < DEPTH; ++d) {
-      t_ok[d] = walk.valid();
-      t_b[d] = 0;
-      t_sc[d] = 1.f;
-      t_m[d] = 0.f;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) t_w[d][k] = 0u;
-      if (t_ok[d]) {
-        t_c[d] = walk.coord();
-        const BundleCoord& c = t_c[d];
-        const int b = __ldg(bits + c.n);
-        t_b[d] = b;
-        const int32_t* in = packed + (__ldg(word_offsets + c.n) + (int64_t)c.g0 * 8 * b);
-        const int words = c.count * 8 * b;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          if (k < b && k * 32 + lane < words) t_w[d][k] = (uint32_t)__ldg(in + k * 32 + lane);
-        if (lane < c.count) {
-          t_sc[d] = load_scalar<ST>(scale, c.q0 + lane);
-          t_m[d] = load_scalar<ST>(mn, c.q0 + lane);
-        }
-        walk.next();
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < DEPTH; ++d) {
-      if (!t_ok[d]) break;                                // warp-uniform
-#define ACTNN_CASE(B) \
-      case B: unpack_bundle<T, B>(t_w[d], t_sc[d], t_m[d], t_c[d], out, plan, lane); break;
-      switch (t_b[d]) {
-        ACTNN_CASE(1) ACTNN_CASE(2) ACTNN_CASE(3) ACTNN_CASE(4) ACTNN_CASE(5) ACTNN_CASE(6) ACTNN_CASE(7)
-        ACTNN_CASE(8)
-        default: break;
-      }
-#undef ACTNN_CASE
-    }
-  }
-}
-
 // How the flat unpack kernel deals out its tasks (32 consecutive groups each).  Block b owns tasks
 // b, b + gridDim.x, b + 2 gridDim.x, ... -- a sample is 20 to 30 consecutive tasks, so every block
 // meets every width in the proportion of the whole activation -- and its warps claim them one at
@@ -882,10 +712,7 @@ int launch_unpack(const int32_t* packed, const int32_t* bits, const int64_t* wor
         packed, bits, word_offsets, (const ST*)scale, (const ST*)mn, (T*)out, N * G, G);
     return check_launch();
   }
-  const int64_t tasks = N * ((G + kBundle - 1) / kBundle);
-  unpack_mixed_kernel<T, ST><<<persistent_grid(unpack_mixed_kernel<T, ST>, kThreads, tasks), kThreads, 0, stream>>>(
-      packed, bits, word_offsets, (const ST*)scale, (const ST*)mn, (T*)out, N, G);
-  return check_launch();
+  return column_unpack(packed, bits, word_offsets, scale, mn, out, N, G * kGroup, DType<T>::id, DType<ST>::id, stream);
 }
 
 int check_common(int64_t N, int64_t G, int64_t group_size, int dtype, int stat_dtype) {
@@ -925,6 +752,11 @@ int pack_mixed_impl(const void* data, const void* mn, const void* mx, const int3
                               stat_dtype, stochastic, noise, seed, offset, s);
   const size_t al = dtype == ACTNN_F32 ? 32 : 16;
   if (!aligned(data, al) || (noise && !aligned(noise, al)) || !aligned(packed, 4)) return ACTNN_ERR_ALIGN;
+  // the flat tasks need whole bundles and at most one sample boundary in 32 groups; other group counts
+  // take the column kernels, which the step-by-step entry (min not known to be exact) does not have
+  if (min_is_exact && mn_out && (G % kFlatBundle != 0 || G < kFlatGroups))
+    return column_pack(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, G * kGroup, dtype, stat_dtype,
+                       stochastic, noise, seed, offset, s);
   switch (dtype) {
     case ACTNN_F16:
       return launch_pack<__half, __half>(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, G,

@@ -257,6 +257,16 @@ int pack_mixed_impl(const void* data, const void* mn, const void* mx, const int3
                     int64_t group_size, int dtype, int stat_dtype, int stochastic, const void* noise, uint64_t seed,
                     uint64_t offset, bool min_is_exact, cudaStream_t stream);
 
+// codec_column.cu: min / max, pack and unpack of [N, F] activations, any F (groups of 256; elements past
+// the end of a sample count as zeros in its last group).  `mn` must be the true group minima.
+int column_minimax(const void* data, void* mn, void* mx, int64_t N, int64_t F, int dtype, unsigned* clear_word,
+                   cudaStream_t stream);
+int column_pack(const void* data, const void* mn, const void* mx, const int32_t* bits, const int64_t* word_offsets,
+                int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t F, int dtype, int stat_dtype,
+                int stochastic, const void* noise, uint64_t seed, uint64_t offset, cudaStream_t stream);
+int column_unpack(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets, const void* scale,
+                  const void* mn, void* out, int64_t N, int64_t F, int dtype, int stat_dtype, cudaStream_t stream);
+
 // stats.cu: actnn_minimax with two extras for the one-call compress: rows walked from the
 // last to the first (`reverse`), and a word zeroed by the kernel (`clear_word`, the ticket of
 // the next kernel).

@@ -58,6 +58,51 @@ extern "C" int actnn_compress_mixed(const void* data, int32_t* packed, void* sca
                          stat_dtype, stochastic, noise, seed, offset, true, (cudaStream_t)stream);
 }
 
+// The same compress of [N, F] samples that need not be whole groups: the last group of a sample is
+// completed with zeros that are neither read nor written (codec_column.cu).
+extern "C" int actnn_compress_mixed_samples(const void* data, int32_t* packed, void* scale, void* mn_out,
+                                            int32_t* bits_out, int64_t* word_offsets_out, float* C_out,
+                                            void* workspace, int64_t workspace_bytes, int64_t N, int64_t F, int dtype,
+                                            int stat_dtype, float range_factor, float coeff, const float* grad_scale,
+                                            int initial_bits, double target, int stochastic, const void* noise,
+                                            uint64_t seed, uint64_t offset, actnn_stream_t stream) {
+  if (N < 0 || F < 0) return ACTNN_ERR_SHAPE;
+  if (F % kGroup == 0 && aligned(data, dtype == ACTNN_F32 ? 32 : 16))
+    return actnn_compress_mixed(data, packed, scale, mn_out, bits_out, word_offsets_out, C_out, workspace,
+                                workspace_bytes, N, F / kGroup, kGroup, dtype, stat_dtype, range_factor, coeff,
+                                grad_scale, initial_bits, target, stochastic, noise, seed, offset, stream);
+  if (dtype < ACTNN_F32 || dtype > ACTNN_BF16) return ACTNN_ERR_DTYPE;
+  if (!(stat_dtype == dtype || (dtype == ACTNN_F32 && stat_dtype == ACTNN_BF16))) return ACTNN_ERR_DTYPE;
+  if (initial_bits < 1 || initial_bits > 8) return ACTNN_ERR_BITS;
+  if (N == 0) return ACTNN_OK;
+  if (!data || !packed || !scale || !mn_out || !bits_out || !word_offsets_out || !C_out || !workspace)
+    return ACTNN_ERR_NULL;
+  const int64_t G = (F + kGroup - 1) / kGroup;
+  const int64_t need = actnn_compress_mixed_workspace(N, G, dtype);
+  if (need < 0) return ACTNN_ERR_SHAPE;
+  if (workspace_bytes < need) return ACTNN_ERR_CAPACITY;
+  if (!aligned(workspace, 256) || !aligned(data, dtype_size(dtype)) || !aligned(packed, 4)) return ACTNN_ERR_ALIGN;
+  const int64_t one = (need - 256) / 2;
+  void* mn = workspace;
+  void* mx = (char*)workspace + one;
+  unsigned* ticket = (unsigned*)((char*)workspace + 2 * one);
+  cudaStream_t s = (cudaStream_t)stream;
+  const bool fused_alloc = range_greedy_supported(N, initial_bits);
+  if (int st = column_minimax(data, mn, mx, N, F, dtype, fused_alloc ? ticket : nullptr, s)) return st;
+  if (fused_alloc) {
+    if (int st = range_greedy_impl(mn, mx, N, G, dtype, range_factor, coeff, grad_scale, C_out, ticket, initial_bits,
+                                   target, bits_out, word_offsets_out, kGroup, s))
+      return st;
+  } else {
+    if (int st = actnn_range_sqr(mn, mx, N, G, dtype, range_factor, coeff, grad_scale, C_out, stream)) return st;
+    if (int st = actnn_calc_precision(C_out, nullptr, N, initial_bits, target, bits_out, word_offsets_out, G, kGroup,
+                                      nullptr, 0, stream))
+      return st;
+  }
+  return column_pack(data, mn, mx, bits_out, word_offsets_out, packed, scale, mn_out, N, F, dtype, stat_dtype,
+                     stochastic, noise, seed, offset, s);
+}
+
 // The same compress when the per-group min / max already exist (actnn_batch_norm_stats_minimax
 // produces them in the pass that computes the batch-norm statistics): sensitivities + greedy
 // allocation, then the pack.  `ticket_workspace`: 256 bytes, 256-byte aligned.

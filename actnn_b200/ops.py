@@ -168,15 +168,21 @@ def dequantize_activation(quantized, q_input_shape, dtype=None):
     q_input, q_bits, q_scale, q_min = quantized
     if dtype is None:
         dtype = torch.float32 if q_scale.dtype == torch.bfloat16 else q_scale.dtype
+    N = q_input_shape[0]
+    num_features = math.prod(q_input_shape[1:])
     if config.simulate:
         if dtype != q_scale.dtype:
             q_scale, q_min = q_scale.to(dtype), q_min.to(dtype)
         input = dequantize_and_unpack(q_input, q_input_shape, q_bits, q_scale, q_min)
+    elif config.group_size == 256 and N and num_features % 256 != 0 and not isinstance(q_bits, int):
+        # decoded into place: no padded intermediate to cut the samples out of
+        if config.swap:
+            q_input = swap_to_gpu(q_input)
+        return ext_quantization.unpack_mixed_samples(q_input, q_bits, q_scale, q_min, tuple(q_input_shape),
+                                                     out_dtype=dtype)
     else:
         input = dequantize_and_unpack(q_input, q_input_shape, q_bits, q_scale, q_min, out_dtype=dtype)
 
-    N = q_input_shape[0]
-    num_features = math.prod(q_input_shape[1:])
     input = input.view(N, -1)[:, :num_features]
     return input.reshape(*q_input_shape).contiguous()
 

@@ -2,8 +2,7 @@
 preceding conv / linear layer (mirror of actnn/actnn/qbnscheme.py:9-60)."""
 from .conf import config
 from .cpp_extension import calc_precision as ext_calc_precision
-from .cpp_extension import quantization as ext_quantization
-from .qscheme import QScheme, group_minimax, to_groups, total_bits_after_greedy
+from .qscheme import QScheme, compress_groups, group_minimax, total_bits_after_greedy
 
 
 class QBNScheme(QScheme):
@@ -37,8 +36,8 @@ class QBNScheme(QScheme):
         self.prev_linear = QScheme.prev_layer
         N, D = input.shape[0], input.shape[1]
         num_pixels = (input.numel() // N) // D
-        q_input, b, q_scale, q_min, _ = ext_quantization.compress_mixed_precision(
-            to_groups(input), int(self.bits * N), int(self.initial_bits), config.group_size / num_pixels,
+        q_input, b, q_scale, q_min, _ = compress_groups(
+            input, int(self.bits * N), int(self.initial_bits), config.group_size / num_pixels,
             1.0, None, config.stochastic, stat_dtype=stat_dtype, minmax=minmax)
         return q_input, b, q_scale, q_min
 

@@ -27,6 +27,18 @@ def to_groups(input: torch.Tensor) -> torch.Tensor:
     return flat.view(N, -1, gs)
 
 
+def compress_groups(input: torch.Tensor, *args, minmax=None, **kwargs):
+    """``ext_quantization.compress_mixed_precision`` of an activation's groups; samples that are not
+    whole groups of 256 are compressed where they are instead of from a padded copy."""
+    n = input.shape[0]
+    if config.group_size == 256 and n and (input.numel() // n) % 256 != 0 and input.is_cuda:
+        flat = input.view(n, -1)
+        if not flat.is_contiguous():                  # as the padded copy would have made it
+            flat = flat.contiguous()
+        return ext_quantization.compress_mixed_samples(flat, *args, **kwargs)
+    return ext_quantization.compress_mixed_precision(to_groups(input), *args, minmax=minmax, **kwargs)
+
+
 def group_minimax(input: torch.Tensor):
     """``(groups [N,G,gs], mn[N,G,1], mx[N,G,1])`` of an activation."""
     N = input.shape[0]
@@ -138,8 +150,8 @@ class QScheme(object):
             self.scales = grad
         if minmax is not None and (config.group_size != 256 or (input.numel() // N) % 256 != 0):
             minmax = None                                      # padded groups: not the producer's
-        q_input, b, q_scale, q_min, C = ext_quantization.compress_mixed_precision(
-            to_groups(input), int(self.bits * N), int(self.initial_bits), config.group_size / num_pixels,
+        q_input, b, q_scale, q_min, C = compress_groups(
+            input, int(self.bits * N), int(self.initial_bits), config.group_size / num_pixels,
             self.num_locations / 4 / self.depthwise_groups, grad.reshape(1), config.stochastic,
             stat_dtype=stat_dtype, minmax=minmax)
         self.C = C

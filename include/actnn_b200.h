@@ -192,6 +192,20 @@ int actnn_compress_mixed(const void* data, int32_t* packed, void* scale, void* m
                          int stochastic, const void* noise, uint64_t seed, uint64_t offset,
                          actnn_stream_t stream);
 
+/* actnn_compress_mixed and actnn_unpack_mixed on samples of any length: data / out are [N, F], contiguous,
+ * groups are 256 elements, G = ceil(F / 256), and the last group of a sample is completed with zeros, as the
+ * reference's padding does (actnn/actnn/qscheme.py:61-71, stripped again in ops.py:137-139), without a padded copy.
+ * data / out need the alignment of one element only.  `noise`, when given, is [N, G, 256]. */
+int actnn_compress_mixed_samples(const void* data, int32_t* packed, void* scale, void* mn_out,
+                                 int32_t* bits_out, int64_t* word_offsets_out, float* C_out,
+                                 void* workspace, int64_t workspace_bytes, int64_t N, int64_t F, int dtype,
+                                 int stat_dtype, float range_factor, float coeff, const float* grad_scale,
+                                 int initial_bits, double target, int stochastic, const void* noise,
+                                 uint64_t seed, uint64_t offset, actnn_stream_t stream);
+int actnn_unpack_mixed_samples(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets,
+                               const void* scale, const void* mn, void* out, int64_t N, int64_t F, int dtype,
+                               int stat_dtype, actnn_stream_t stream);
+
 /* actnn_compress_mixed for callers that cannot hand over scratch memory.  (This entry point
  * has no counterpart in the reference.)
  * Who needs it: code that only works with pointers it was given -- a plug-in of a host
