@@ -25,6 +25,8 @@ SIGNATURES = {
     "actnn_compress_mixed_prestat_kept": ['P'] * 10 + ['L', 'L', 'L', 'I', 'I', 'F', 'F', 'P', 'I', 'D', 'I', 'P', 'U', 'U',
                                           'P'],
     "actnn_batch_norm_stats_minimax": ['P'] * 9 + ['L', 'L', 'L', 'D', 'D', 'I', 'P', 'L', 'P'],
+    "actnn_batch_norm_codes_workspace": ['L', 'L', 'L', 'I', 'P'],
+    "actnn_batch_norm_codes_backward": ['P'] * 12 + ['L', 'L', 'L', 'I', 'I', 'P', 'L', 'P'],
     "actnn_range_sqr": ['P', 'P', 'L', 'L', 'I', 'F', 'F', 'P', 'P', 'P'],
     "actnn_sample_sumsq": ['P', 'P', 'L', 'L', 'I', 'P'],
     "actnn_calc_precision": ['P', 'P', 'L', 'I', 'D', 'P', 'P', 'L', 'L', 'P', 'L', 'P'],

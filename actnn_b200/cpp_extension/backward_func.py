@@ -12,9 +12,13 @@ channel over many blocks instead of cuDNN's one block per channel.  ``batch_norm
 ``batch_norm_elemt``, ``batch_norm_backward_reduce`` and ``batch_norm_backward_elemt`` are
 the same kernels under the names of the ATen operators the reference's synchronised batch
 norm calls (ops.py:515-603)."""
+import ctypes
+import functools
+
 import torch
 
 from .. import _lib
+from . import quantization
 
 aten = torch.ops.aten
 
@@ -123,6 +127,55 @@ def cudnn_batch_norm_backward(input, grad_output, weight, running_mean, running_
     _lib.call("actnn_batch_norm_backward", x, _lib.ptr(x), _lib.ptr(dy), _lib.ptr(w32), _lib.ptr(save_mean),
               _lib.ptr(save_var), _lib.ptr(dx), _lib.ptr(dweight), _lib.ptr(dbias), N, C, HW,
               _lib.dtype_id(x.dtype), _lib.ptr(ws), nbytes, _lib.stream_of(x))
+    if weight is not None and weight.dtype != torch.float32:
+        dweight, dbias = dweight.to(weight.dtype), dbias.to(weight.dtype)
+    return dx, dweight, dbias
+
+
+@functools.lru_cache(maxsize=4096)
+def _codes_workspace(N, C, HW, dtype_id, device_index):
+    """Scratch bytes of ``actnn_batch_norm_codes_backward``; ``None``: a geometry it does not cover."""
+    nbytes = ctypes.c_int64(0)
+    with torch.cuda.device(device_index):
+        status = _lib.load().actnn_batch_norm_codes_workspace(N, C, HW, dtype_id, ctypes.addressof(nbytes))
+    return None if status else nbytes.value
+
+
+def batch_norm_codes_backward(quantized, shape, dtype, grad_output, weight, save_mean, save_invstd):
+    """Backward of a training-mode batch norm from the compressed input: what ``dequantize_activation``
+    followed by ``cudnn_batch_norm_backward`` computes (ops.py:470-493), with the decoded input in
+    registers only.  ``quantized``: ``(packed, bits, scale, min)`` of the mixed stream, on the device.
+    Returns ``(grad_input, grad_weight, grad_bias)``, or ``None`` when the geometry is not covered."""
+    packed, bits, scale, mn = quantized
+    if len(shape) < 2 or not packed.is_cuda or dtype not in (torch.float16, torch.bfloat16, torch.float32) \
+            or scale.dtype != (torch.bfloat16 if dtype == torch.float32 else dtype):
+        return None
+    N, C = shape[0], shape[1]
+    F = 1
+    for d in shape[1:]:
+        F *= d
+    if N * F == 0 or tuple(scale.shape) != (N, (F + 255) // 256, 1) or bits.numel() != N:
+        return None
+    HW = F // C
+    dt = _lib.dtype_id(dtype)
+    nbytes = _codes_workspace(N, C, HW, dt, packed.device.index)
+    if nbytes is None:
+        return None
+    dy = grad_output.contiguous()
+    if dy.dtype != dtype:
+        dy = dy.to(dtype)
+    word_offsets = getattr(packed, "word_offsets", None)
+    if word_offsets is None:
+        word_offsets = quantization.bits_prefix(bits, scale.shape[1], 256)
+    w32 = _as_f32(weight)
+    dx = torch.empty(shape, dtype=dtype, device=packed.device)
+    dweight = torch.empty(C, dtype=torch.float32, device=packed.device)
+    dbias = torch.empty(C, dtype=torch.float32, device=packed.device)
+    ws = _lib.scratch(packed.device, nbytes)
+    _lib.call("actnn_batch_norm_codes_backward", packed, packed.data_ptr(), bits.data_ptr(), word_offsets.data_ptr(),
+              scale.data_ptr(), mn.data_ptr(), dy.data_ptr(), _lib.ptr(w32), save_mean.data_ptr(),
+              save_invstd.data_ptr(), dx.data_ptr(), dweight.data_ptr(), dbias.data_ptr(), N, C, HW, dt,
+              _lib.dtype_id(scale.dtype), ws.data_ptr(), nbytes, _lib.stream_of(packed))
     if weight is not None and weight.dtype != torch.float32:
         dweight, dbias = dweight.to(weight.dtype), dbias.to(weight.dtype)
     return dx, dweight, dbias

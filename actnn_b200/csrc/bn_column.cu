@@ -1,0 +1,386 @@
+// Batch-norm passes that work on the compressed activation, on the column mapping (column.cuh).
+//
+// Backward: both passes decode the saved codes in registers, so the decoded activation is never
+// written to memory (the reference decodes it, ops.py:470-476, and cuDNN reads it back, ops.py:490-493):
+//   reduce  reads the codes and dy; sum(dy) and sum(dy * (x - mean)) of the lane's octets stay in
+//           registers across the samples of the split, because an octet position has one channel;
+//   finish  one warp per channel adds the columns' and splits' sums in a fixed order;
+//   apply   reads the codes and dy again and writes dx, walking the samples backwards so that it
+//           starts with what the reduce left in the L2.
+// Per element of a 16-bit activation that is 2 + b/8 bytes for the reduce and 4 + b/8 for the apply,
+// against 2 (decode) + 4 + 6.  What bounds it now is instruction issue (about 430 instructions a
+// bundle of 1024 elements, some 200 of them decoding), not memory: bringing dy and the words through a
+// ring of bulk copies in shared memory measured the same or slower (42.0 / 40.6 us with 3 stages).
+// float16, 256 x 64 x 56 x 56: decode 24.9 + reduce 40.9 + apply 40.5 us -> 37.2 + 3.2 + 40.1.
+#include "column.cuh"
+
+namespace actnn {
+namespace {
+
+// Elements 8t .. 8t+7 touch one channel (SUB = 8: HW % 8 == 0), one channel per half (SUB = 4: HW % 4 == 0) or change
+// channel at any element (SUB = 1).  HW >= 8, so there are at most two.
+template <int SUB> struct Slots { static constexpr int N = SUB == 8 ? 1 : 2; };
+
+struct BnColumns { int C, HW, kmax; };       // kmax: channels a column can touch
+
+// Channels of the lane's octets; a channel number >= C marks elements past the end of the sample.
+template <int SUB> struct ColumnChannels {
+  static constexpr int NS = Slots<SUB>::N;
+  int ch[kBundle][NS];
+  int first_of_next[SUB == 1 ? kBundle : 1];      // SUB = 1: first element of slot 1
+  int c_lo, nch;                                  // channels of the whole column
+  ACTNN_DEV ColumnChannels(const ColumnShape& sh, const BnColumns& bn, const ColumnTask& t, int lane) {
+    const uint32_t hw = (uint32_t)bn.HW;
+    const uint32_t e0 = (uint32_t)t.p * (kBundle * kGroup);
+    const uint32_t last = (uint32_t)min((int64_t)e0 + kBundle * kGroup, sh.F) - 1u;
+    c_lo = (int)(e0 / hw);
+    nch = (int)(last / hw) - c_lo + 1;
+#pragma unroll
+    for (int gi = 0; gi < kBundle; ++gi) {
+      const uint32_t e = e0 + gi * kGroup + lane * kOct;
+      ch[gi][0] = (int)(e / hw);
+      if constexpr (SUB == 4) ch[gi][1] = (int)((e + 4) / hw);
+      if constexpr (SUB == 1) {
+        ch[gi][1] = ch[gi][0] + 1;
+        first_of_next[gi] = (int)min(8u, (uint32_t)ch[gi][1] * hw - e);
+      }
+    }
+  }
+  ACTNN_DEV bool second(int gi, int j) const {     // element j of octet gi belongs to slot 1
+    if constexpr (SUB == 8) return false;
+    else if constexpr (SUB == 4) return j >= 4;
+    else return j >= first_of_next[gi];
+  }
+};
+
+// Two float32 operations per instruction (sm_100).
+ACTNN_DEV float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.f32x2 c, a, b;\n\t"
+      "mov.b64 {%0, %1}, c;\n\t}" : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+ACTNN_DEV float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+ACTNN_DEV float2 both(float v) { return make_float2(v, v); }
+
+// Elements 2k, 2k+1 of an octet.
+template <typename T> ACTNN_DEV float2 octet_pair(const Oct<T>& o, int k) {
+  if constexpr (sizeof(T) == 4) return make_float2(o.f[2 * k], o.f[2 * k + 1]);
+  else if constexpr (DType<T>::id == ACTNN_F16) return __half22float2(*reinterpret_cast<const __half2*>(&o.r[k]));
+  else return make_float2(__uint_as_float(o.r[k] << 16), __uint_as_float(o.r[k] & 0xffff0000u));
+}
+// Elements 2k, 2k+1 plus (a, b): for the 16-bit types the mixed-precision add of sm_100, no conversion.
+template <typename T> ACTNN_DEV float2 octet_pair_plus(const Oct<T>& o, int k, float a, float b) {
+  if constexpr (sizeof(T) == 4) {
+    return add2(make_float2(o.f[2 * k], o.f[2 * k + 1]), make_float2(a, b));
+  } else {
+    float2 r;
+    const uint16_t lo = (uint16_t)o.r[k], hi = (uint16_t)(o.r[k] >> 16);
+    if constexpr (DType<T>::id == ACTNN_F16) {
+      asm("add.rn.f32.f16 %0, %1, %2;" : "=f"(r.x) : "h"(lo), "f"(a));
+      asm("add.rn.f32.f16 %0, %1, %2;" : "=f"(r.y) : "h"(hi), "f"(b));
+    } else {
+      asm("add.rn.f32.bf16 %0, %1, %2;" : "=f"(r.x) : "h"(lo), "f"(a));
+      asm("add.rn.f32.bf16 %0, %1, %2;" : "=f"(r.y) : "h"(hi), "f"(b));
+    }
+    return r;
+  }
+}
+template <typename T> ACTNN_DEV void set_octet_pair(Oct<T>& o, int k, float2 v) {
+  if constexpr (sizeof(T) == 4) {
+    o.f[2 * k] = v.x;
+    o.f[2 * k + 1] = v.y;
+  } else if constexpr (DType<T>::id == ACTNN_F16) {
+    const __half2 h = __floats2half2_rn(v.x, v.y);
+    o.r[k] = *reinterpret_cast<const uint32_t*>(&h);
+  } else {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+    o.r[k] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+
+// Sums of two quantities per channel of the column, from per-lane sums per octet and slot; partial sum k
+// of the column is channel c_lo + k's.
+template <int SUB>
+ACTNN_DEV void write_partials(const ColumnChannels<SUB>& cc, const float2 (&a)[kBundle][Slots<SUB>::N],
+                              const float2 (&b)[kBundle][Slots<SUB>::N], float2* __restrict__ dst, int lane) {
+  for (int k = 0; k < cc.nch; ++k) {
+    float sa = 0.f, sb = 0.f;
+#pragma unroll
+    for (int gi = 0; gi < kBundle; ++gi) {
+#pragma unroll
+      for (int s = 0; s < Slots<SUB>::N; ++s) {
+        if (cc.ch[gi][s] == cc.c_lo + k) { sa += a[gi][s].x + a[gi][s].y; sb += b[gi][s].x + b[gi][s].y; }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sa += __shfl_xor_sync(kFull, sa, o);
+      sb += __shfl_xor_sync(kFull, sb, o);
+    }
+    if (lane == 0) dst[k] = make_float2(sa, sb);
+  }
+}
+
+// Channel c's sums over all columns and splits, in a fixed order; one warp, the result in every lane.
+ACTNN_DEV float2 collect_partials(const ColumnShape& sh, const BnColumns& bn, const float2* __restrict__ partial, int c,
+                                  int lane) {
+  const uint32_t span = kBundle * kGroup;
+  const uint32_t first = (uint32_t)c * (uint32_t)bn.HW, last = first + (uint32_t)bn.HW - 1u;
+  const int p_lo = (int)(first / span), np = (int)(last / span) - p_lo + 1;
+  float a = 0.f, b = 0.f;
+  for (int i = lane; i < np * sh.S; i += 32) {
+    const int s = i / np, p = p_lo + (i - s * np);
+    const int k = c - (int)((uint32_t)p * span / (uint32_t)bn.HW);
+    const float2 v = __ldg(partial + ((int64_t)s * sh.P + p) * bn.kmax + k);
+    a += v.x;
+    b += v.y;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(kFull, a, o);
+    b += __shfl_xor_sync(kFull, b, o);
+  }
+  return make_float2(a, b);
+}
+
+// ------------------------------------------------------------------ backward
+constexpr int kBnBlocks = 2;     // resident blocks per SM: 128 registers and no spills beat 3 blocks with them (40.1 against 41.3 us, apply)
+
+// EDGE: samples that are not whole groups, or octets off their natural alignment.
+template <typename T, typename ST, int SUB, bool EDGE>
+__global__ void __launch_bounds__(kColThreads, kBnBlocks)
+bn_codes_reduce_kernel(const int32_t* __restrict__ packed, const int32_t* __restrict__ bits,
+                       const int64_t* __restrict__ word_offsets, const ST* __restrict__ scale,
+                       const ST* __restrict__ mn, const T* __restrict__ dy, ColumnShape sh, BnColumns bn,
+                       const float* __restrict__ save_mean, float2* __restrict__ partial) {
+  constexpr int NS = Slots<SUB>::N;
+  const int lane = threadIdx.x & 31;
+  const ColumnTask t = column_task(sh);
+  if (!t.valid) return;
+  const ColumnChannels<SUB> cc(sh, bn, t, lane);
+  const TransposePlan plan = make_transpose_plan(lane);
+  float neg_mean[kBundle][NS];
+  float2 sg[kBundle][NS], sgx[kBundle][NS];
+#pragma unroll
+  for (int gi = 0; gi < kBundle; ++gi) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      neg_mean[gi][s] = cc.ch[gi][s] < bn.C ? -__ldg(save_mean + cc.ch[gi][s]) : 0.f;
+      sg[gi][s] = sgx[gi][s] = both(0.f);
+    }
+  }
+  auto add = [&](int gi, const Oct<T>& x, const Oct<T>& g) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 vg = octet_pair<T>(g, k);
+      if constexpr (SUB != 1) {
+        const int s = SUB == 8 ? 0 : k / 2;
+        sg[gi][s] = add2(sg[gi][s], vg);
+        sgx[gi][s] = fma2(vg, octet_pair_plus<T>(x, k, neg_mean[gi][s], neg_mean[gi][s]), sgx[gi][s]);
+      } else {
+        const bool s0 = cc.second(gi, 2 * k), s1 = cc.second(gi, 2 * k + 1);
+        const float2 d = octet_pair_plus<T>(x, k, neg_mean[gi][s0 ? 1 : 0], neg_mean[gi][s1 ? 1 : 0]);
+        const float p0 = vg.x * d.x, p1 = vg.y * d.y;
+        sg[gi][0].x += s0 ? 0.f : vg.x; sg[gi][0].y += s1 ? 0.f : vg.y;
+        sg[gi][1].x += s0 ? vg.x : 0.f; sg[gi][1].y += s1 ? vg.y : 0.f;
+        sgx[gi][0].x += s0 ? 0.f : p0; sgx[gi][0].y += s1 ? 0.f : p1;
+        sgx[gi][1].x += s0 ? p0 : 0.f; sgx[gi][1].y += s1 ? p1 : 0.f;
+      }
+    }
+  };
+  const ColumnOctets<EDGE> oct(sh, t, lane);
+  for (int nb = t.n0; nb < t.n1; nb += 32) {
+    const int nl = min(32, t.n1 - nb);
+    ColumnStream st;
+    st.open(t, nb + lane, lane < nl, bits, word_offsets);
+    BundleWords next = st.fetch<ST>(t, sh.G, nb, 0, packed, scale, mn, lane);
+    for (int i = 0; i < nl; ++i) {
+      const BundleWords cur = next;
+      Oct<T> g[kBundle];
+      oct.template load<T>(dy + (int64_t)(nb + i) * sh.F, g);
+      if (i + 1 < nl) next = st.fetch<ST>(t, sh.G, nb + i + 1, i + 1, packed, scale, mn, lane);
+      decode_column<T>(cur, t.count, plan, lane, [&](int gi, const Oct<T>& x) { add(gi, x, g[gi]); });
+    }
+  }
+  const int split = t.n0 / sh.spp;
+  write_partials<SUB>(cc, sg, sgx, partial + ((int64_t)split * sh.P + t.p) * bn.kmax, lane);
+}
+
+// coef[c]: (mean, weight * invstd, sum_dy / M, sum_dy_xmu * invstd^2 / M); one warp per channel.
+__global__ void __launch_bounds__(kColThreads)
+bn_codes_finish_kernel(const float2* __restrict__ partial, ColumnShape sh, BnColumns bn,
+                       const float* __restrict__ weight, const float* __restrict__ save_mean,
+                       const float* __restrict__ save_invstd, float* __restrict__ dweight, float* __restrict__ dbias,
+                       float4* __restrict__ coef) {
+  const int lane = threadIdx.x & 31;
+  const int c = (int)(blockIdx.x * (kColThreads / 32) + (threadIdx.x >> 5));
+  if (c >= bn.C) return;
+  const float2 tot = collect_partials(sh, bn, partial, c, lane);
+  if (lane != 0) return;
+  const float M = (float)sh.N * (float)bn.HW, invstd = save_invstd[c];
+  if (dbias) dbias[c] = tot.x;
+  if (dweight) dweight[c] = tot.y * invstd;
+  coef[c] = make_float4(save_mean[c], (weight ? weight[c] : 1.f) * invstd, tot.x / M, tot.y * invstd * invstd / M);
+}
+
+template <typename T, typename ST, int SUB, bool EDGE>
+__global__ void __launch_bounds__(kColThreads, kBnBlocks)
+bn_codes_apply_kernel(const int32_t* __restrict__ packed, const int32_t* __restrict__ bits,
+                      const int64_t* __restrict__ word_offsets, const ST* __restrict__ scale,
+                      const ST* __restrict__ mn, const T* __restrict__ dy, T* __restrict__ dx, ColumnShape sh,
+                      BnColumns bn, const float4* __restrict__ coef) {
+  constexpr int NS = Slots<SUB>::N;
+  const int lane = threadIdx.x & 31;
+  const ColumnTask t = column_task(sh);
+  if (!t.valid) return;
+  const ColumnOctets<EDGE> oct(sh, t, lane);
+  const ColumnChannels<SUB> cc(sh, bn, t, lane);
+  const TransposePlan plan = make_transpose_plan(lane);
+  float4 kf[kBundle][NS];                              // (-mean, weight * invstd, -mean_dy, -q)
+#pragma unroll
+  for (int gi = 0; gi < kBundle; ++gi) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const float4 k = cc.ch[gi][s] < bn.C ? __ldg(coef + cc.ch[gi][s]) : make_float4(0.f, 0.f, 0.f, 0.f);
+      kf[gi][s] = make_float4(-k.x, k.y, -k.z, -k.w);
+    }
+  }
+  auto gradient = [&](int gi, const Oct<T>& x, const Oct<T>& g) {
+    Oct<T> r;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if constexpr (SUB != 1) {
+        const float4 c = kf[gi][SUB == 8 ? 0 : k / 2];
+        const float2 d = fma2(octet_pair_plus<T>(x, k, c.x, c.x), both(c.w), octet_pair_plus<T>(g, k, c.z, c.z));
+        set_octet_pair<T>(r, k, make_float2(c.y * d.x, c.y * d.y));
+      } else {
+        const float4 c0 = cc.second(gi, 2 * k) ? kf[gi][1] : kf[gi][0];
+        const float4 c1 = cc.second(gi, 2 * k + 1) ? kf[gi][1] : kf[gi][0];
+        const float2 vx = octet_pair_plus<T>(x, k, c0.x, c1.x), vg = octet_pair_plus<T>(g, k, c0.z, c1.z);
+        set_octet_pair<T>(r, k, make_float2(c0.y * fmaf(vx.x, c0.w, vg.x), c1.y * fmaf(vx.y, c1.w, vg.y)));
+      }
+    }
+    return r;
+  };
+  // the samples from the last to the first: what the reduce read last is still in the L2
+  const int total = t.n1 - t.n0;
+  for (int kb = 0; kb < total; kb += 32) {
+    const int nl = min(32, total - kb);
+    const int top = t.n1 - 1 - kb;
+    ColumnStream st;
+    st.open(t, top - lane, lane < nl, bits, word_offsets);
+    BundleWords next = st.fetch<ST>(t, sh.G, top, 0, packed, scale, mn, lane);
+    for (int i = 0; i < nl; ++i) {
+      const BundleWords cur = next;
+      Oct<T> g[kBundle];
+      oct.template load<T>(dy + (int64_t)(top - i) * sh.F, g);
+      if (i + 1 < nl) next = st.fetch<ST>(t, sh.G, top - i - 1, i + 1, packed, scale, mn, lane);
+      T* sample = dx + (int64_t)(top - i) * sh.F;
+      decode_column<T>(cur, t.count, plan, lane,
+                       [&](int gi, const Oct<T>& x) { oct.template store<T>(sample, gi, gradient(gi, x, g[gi])); });
+    }
+  }
+}
+
+// ------------------------------------------------------------------ host side
+bool bn_columns_supported(int64_t N, int64_t C, int64_t HW) {
+  if (N <= 0 || C <= 0 || HW < kOct || C > 0x7fffffff || HW > 0x7fffffff) return false;
+  return C * HW < ((int64_t)1 << 31) - kBundle * kGroup && column_supported(N, C * HW);
+}
+BnColumns bn_columns(int64_t C, int64_t HW) {
+  BnColumns bn;
+  bn.C = (int)C;
+  bn.HW = (int)HW;
+  bn.kmax = (int)((kBundle * kGroup - 1) / HW + 2);
+  return bn;
+}
+constexpr int kBnWarps = kBnBlocks * kColThreads / 32;       // resident warps per SM
+int64_t bn_partial_bytes(const ColumnShape& sh, const BnColumns& bn) {
+  return ((int64_t)sh.P * sh.S * bn.kmax * (int64_t)sizeof(float2) + 255) / 256 * 256;
+}
+int64_t bn_coef_bytes(int64_t C) { return (C * (int64_t)sizeof(float4) + 255) / 256 * 256; }
+
+template <typename T, typename ST, int SUB, bool EDGE>
+int launch_backward(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets, const void* scale,
+                    const void* mn, const void* dy, const float* weight, const float* save_mean,
+                    const float* save_invstd, void* dx, float* dweight, float* dbias, const ColumnShape& sh,
+                    const BnColumns& bn, void* workspace, cudaStream_t s) {
+  float4* coef = (float4*)workspace;
+  float2* partial = (float2*)((char*)workspace + bn_coef_bytes(bn.C));
+  bn_codes_reduce_kernel<T, ST, SUB, EDGE><<<column_grid(sh), kColThreads, 0, s>>>(
+      packed, bits, word_offsets, (const ST*)scale, (const ST*)mn, (const T*)dy, sh, bn, save_mean, partial);
+  if (int st = check_launch()) return st;
+  bn_codes_finish_kernel<<<(bn.C + kColThreads / 32 - 1) / (kColThreads / 32), kColThreads, 0, s>>>(
+      partial, sh, bn, weight, save_mean, save_invstd, dweight, dbias, coef);
+  if (int st = check_launch()) return st;
+  bn_codes_apply_kernel<T, ST, SUB, EDGE><<<column_grid(sh), kColThreads, 0, s>>>(
+      packed, bits, word_offsets, (const ST*)scale, (const ST*)mn, (const T*)dy, (T*)dx, sh, bn, coef);
+  return check_launch();
+}
+
+}  // namespace
+}  // namespace actnn
+
+using namespace actnn;
+
+extern "C" int actnn_batch_norm_codes_workspace(int64_t N, int64_t C, int64_t HW, int dtype, int64_t* bytes) {
+  if (!bytes) return ACTNN_ERR_NULL;
+  if (dtype < ACTNN_F32 || dtype > ACTNN_BF16) return ACTNN_ERR_DTYPE;
+  if (!bn_columns_supported(N, C, HW)) return ACTNN_ERR_SHAPE;
+  const ColumnShape sh = column_shape(N, C * HW, kOct, kBnWarps);
+  *bytes = bn_coef_bytes(C) + bn_partial_bytes(sh, bn_columns(C, HW));
+  return ACTNN_OK;
+}
+
+extern "C" int actnn_batch_norm_codes_backward(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets,
+                                               const void* scale, const void* mn, const void* grad_out,
+                                               const float* weight, const float* save_mean, const float* save_invstd,
+                                               void* grad_in, float* grad_weight, float* grad_bias, int64_t N,
+                                               int64_t C, int64_t HW, int dtype, int stat_dtype, void* workspace,
+                                               int64_t workspace_bytes, actnn_stream_t stream) {
+  if (dtype < ACTNN_F32 || dtype > ACTNN_BF16) return ACTNN_ERR_DTYPE;
+  if (stat_dtype != (dtype == ACTNN_F32 ? ACTNN_BF16 : dtype)) return ACTNN_ERR_DTYPE;
+  if (!bn_columns_supported(N, C, HW)) return ACTNN_ERR_SHAPE;
+  if (!packed || !bits || !word_offsets || !scale || !mn || !grad_out || !save_mean || !save_invstd || !grad_in ||
+      !workspace)
+    return ACTNN_ERR_NULL;
+  const int es = dtype_size(dtype);
+  const int64_t F = C * HW;
+  const int al = min(octet_alignment(grad_out, F, es), octet_alignment(grad_in, F, es));
+  if (!aligned(grad_out, es) || !aligned(grad_in, es) || !aligned(packed, 4) || !aligned(workspace, 16))
+    return ACTNN_ERR_ALIGN;
+  const ColumnShape sh = column_shape(N, F, al, kBnWarps);
+  const BnColumns bn = bn_columns(C, HW);
+  if (workspace_bytes < bn_coef_bytes(C) + bn_partial_bytes(sh, bn)) return ACTNN_ERR_CAPACITY;
+  cudaStream_t s = (cudaStream_t)stream;
+  const bool edge = al != kOct || F % kGroup != 0;
+#define ACTNN_BWD(T, ST, SUB, EDGE)                                                                                 \
+  return launch_backward<T, ST, SUB, EDGE>(packed, bits, word_offsets, scale, mn, grad_out, weight, save_mean,      \
+                                           save_invstd, grad_in, grad_weight, grad_bias, sh, bn, workspace, s)
+#define ACTNN_BWD_T(T, ST)                                  \
+  {                                                         \
+    if (HW % 8 == 0) {                                      \
+      if (edge) ACTNN_BWD(T, ST, 8, true);                  \
+      ACTNN_BWD(T, ST, 8, false);                           \
+    }                                                       \
+    if (HW % 4 == 0) {                                      \
+      if (edge) ACTNN_BWD(T, ST, 4, true);                  \
+      ACTNN_BWD(T, ST, 4, false);                           \
+    }                                                       \
+    ACTNN_BWD(T, ST, 1, true);                              \
+  }
+  switch (dtype) {
+    case ACTNN_F16: ACTNN_BWD_T(__half, __half)
+    case ACTNN_BF16: ACTNN_BWD_T(__nv_bfloat16, __nv_bfloat16)
+    default: ACTNN_BWD_T(float, __nv_bfloat16)
+  }
+#undef ACTNN_BWD_T
+#undef ACTNN_BWD
+}

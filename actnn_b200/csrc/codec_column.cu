@@ -116,21 +116,14 @@ column_unpack_kernel(const int32_t* __restrict__ packed, const int32_t* __restri
   for (int nb = t.n0; nb < t.n1; nb += 32) {
     const int nl = min(32, t.n1 - nb);
     ColumnStream st;
-    st.open(t, nb, nl, bits, word_offsets, lane);
-    uint32_t wn[8];
-    float scn, mn_n;
-    int bn = st.fetch<ST>(t, sh.G, nb, 0, packed, scale, mn, lane, wn, scn, mn_n);
+    st.open(t, nb + lane, lane < nl, bits, word_offsets);
+    BundleWords next = st.fetch<ST>(t, sh.G, nb, 0, packed, scale, mn, lane);
     for (int i = 0; i < nl; ++i) {
-      uint32_t w[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) w[k] = wn[k];
-      const int b = bn;
-      const float sc = scn, m = mn_n;
-      if (i + 1 < nl) bn = st.fetch<ST>(t, sh.G, nb, i + 1, packed, scale, mn, lane, wn, scn, mn_n);
-      if (b == 0) continue;                              // the pack wrote nothing for this sample either
-      Oct<T> x[kBundle];
-      decode_column<T>(b, w, sc, m, plan, lane, x);
-      oct.template store<T>(out + (int64_t)(nb + i) * sh.F, x);
+      const BundleWords cur = next;
+      if (i + 1 < nl) next = st.fetch<ST>(t, sh.G, nb + i + 1, i + 1, packed, scale, mn, lane);
+      T* sample = out + (int64_t)(nb + i) * sh.F;
+      decode_column<T>(cur, t.count, plan, lane,
+                       [&](int gi, const Oct<T>& x) { oct.template store<T>(sample, gi, x); });
     }
   }
 }

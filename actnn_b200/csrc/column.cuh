@@ -154,12 +154,9 @@ template <bool EDGE> struct ColumnOctets {
       else x[gi] = gi < count ? load_oct<T>(sample + first + gi * kGroup) : zero_oct<T>();
     }
   }
-  template <typename T> ACTNN_DEV void store(T* sample, const Oct<T> (&x)[kBundle]) const {
-#pragma unroll
-    for (int gi = 0; gi < kBundle; ++gi) {
-      if constexpr (EDGE) store_octet<T, true>(sample + first + gi * kGroup, x[gi], valid[gi], align);
-      else if (gi < count) store_oct_streaming<T>(sample + first + gi * kGroup, x[gi]);
-    }
+  template <typename T> ACTNN_DEV void store(T* sample, int gi, const Oct<T>& x) const {
+    if constexpr (EDGE) store_octet<T, true>(sample + first + gi * kGroup, x, valid[gi], align);
+    else if (gi < count) store_oct_streaming<T>(sample + first + gi * kGroup, x);
   }
 };
 
@@ -228,55 +225,72 @@ ACTNN_DEV void pack_column_bundle(const Oct<T> (&x)[kBundle], const Oct<T> (&nz)
 }
 
 // ------------------------------------------------------------------ the stream of a column, read ahead
-// Lane l of a block of 32 samples knows sample nb + l's width and stream position; the words and the
-// statistics (lane gi < 4: group gi) of one bundle are requested a sample ahead of their use.
+// Of a block of 32 samples, lane l knows the width and the stream position of the l-th; the first words
+// and the statistics (lane gi < 4: group gi) of one bundle are requested a sample ahead of their use.
+// Four words a lane are a bundle of up to 4 bits, nearly all there is at an average of 2; wider
+// bundles load the rest when they are decoded, which keeps four registers free in the common case.
+constexpr int kAhead = 4;
+struct BundleWords {
+  uint32_t w[kAhead];
+  float sc, m;                // statistics of group `lane`
+  const int32_t* in;          // the lane's first word
+  int b;                      // 0: not a width, nothing was written
+};
 struct ColumnStream {
-  int b_l;                    // width of sample nb + lane; 0: not a width, nothing was written
+  int b_l;                    // width of the lane's sample
   int64_t off_l;              // first word of that sample's bundle
-  ACTNN_DEV void open(const ColumnTask& t, int nb, int nl, const int32_t* __restrict__ bits,
-                      const int64_t* __restrict__ word_offsets, int lane) {
+  ACTNN_DEV void open(const ColumnTask& t, int n_l, bool active, const int32_t* __restrict__ bits,
+                      const int64_t* __restrict__ word_offsets) {
     b_l = 0;
     off_l = 0;
-    if (lane < nl) {
-      b_l = __ldg(bits + nb + lane);
+    if (active) {
+      b_l = __ldg(bits + n_l);
       if (b_l < 1 || b_l > 8) b_l = 0;
-      off_l = __ldg(word_offsets + nb + lane) + (int64_t)t.g0 * 8 * b_l;
+      off_l = __ldg(word_offsets + n_l) + (int64_t)t.g0 * 8 * b_l;
     }
   }
-  // sample nb + i (i < 32)
+  // sample n, which is lane i's
   template <typename ST>
-  ACTNN_DEV int fetch(const ColumnTask& t, int G, int nb, int i, const int32_t* __restrict__ packed,
-                      const ST* __restrict__ scale, const ST* __restrict__ mn, int lane, uint32_t (&w)[8], float& sc,
-                      float& m) const {
-    const int b = __shfl_sync(kFull, b_l, i);
+  ACTNN_DEV BundleWords fetch(const ColumnTask& t, int G, int n, int i, const int32_t* __restrict__ packed,
+                              const ST* __restrict__ scale, const ST* __restrict__ mn, int lane) const {
+    BundleWords r;
+    r.b = __shfl_sync(kFull, b_l, i);
     const uint32_t olo = __shfl_sync(kFull, (uint32_t)off_l, i);
     const uint32_t ohi = __shfl_sync(kFull, (uint32_t)((uint64_t)off_l >> 32), i);
-    const int32_t* in = packed + (int64_t)(((uint64_t)ohi << 32) | olo);
-    const int words = t.count * 8 * b;
+    r.in = packed + (int64_t)(((uint64_t)ohi << 32) | olo) + lane;
+    const int left = t.count * 8 * r.b - lane;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) w[k] = k * 32 + lane < words ? (uint32_t)__ldg(in + k * 32 + lane) : 0u;
-    sc = 1.f;
-    m = 0.f;
+    for (int k = 0; k < kAhead; ++k) r.w[k] = k * 32 < left ? (uint32_t)__ldg(r.in + k * 32) : 0u;
+    r.sc = 1.f;
+    r.m = 0.f;
     if (lane < t.count) {
-      const int64_t q = (int64_t)(nb + i) * G + t.g0 + lane;
-      sc = load_scalar<ST>(scale, q);
-      m = load_scalar<ST>(mn, q);
+      const int64_t q = (int64_t)n * G + t.g0 + lane;
+      r.sc = load_scalar<ST>(scale, q);
+      r.m = load_scalar<ST>(mn, q);
     }
-    return b;
+    return r;
   }
 };
-template <typename T>
-ACTNN_DEV void decode_column(int b, const uint32_t (&w)[8], float sc, float m, const TransposePlan& plan, int lane,
-                             Oct<T> (&x)[kBundle]) {
-  switch (b) {
-    case 1: decode_bundle<T, 1>(w, sc, m, plan, lane, x); break;
-    case 2: decode_bundle<T, 2>(w, sc, m, plan, lane, x); break;
-    case 3: decode_bundle<T, 3>(w, sc, m, plan, lane, x); break;
-    case 4: decode_bundle<T, 4>(w, sc, m, plan, lane, x); break;
-    case 5: decode_bundle<T, 5>(w, sc, m, plan, lane, x); break;
-    case 6: decode_bundle<T, 6>(w, sc, m, plan, lane, x); break;
-    case 7: decode_bundle<T, 7>(w, sc, m, plan, lane, x); break;
-    default: decode_bundle<T, 8>(w, sc, m, plan, lane, x); break;
+template <typename T, int B, typename Use>
+ACTNN_DEV void decode_words(const BundleWords& r, int count, const TransposePlan& plan, int lane, Use use) {
+  uint32_t w[B];
+#pragma unroll
+  for (int k = 0; k < B; ++k)
+    w[k] = k < kAhead ? r.w[k < kAhead ? k : 0] : k * 32 + lane < count * 8 * B ? (uint32_t)__ldg(r.in + k * 32) : 0u;
+  decode_bundle<T, B>(w, r.sc, r.m, plan, lane, use);
+}
+template <typename T, typename Use>
+ACTNN_DEV void decode_column(const BundleWords& r, int count, const TransposePlan& plan, int lane, Use use) {
+  switch (r.b) {
+    case 1: decode_words<T, 1>(r, count, plan, lane, use); break;
+    case 2: decode_words<T, 2>(r, count, plan, lane, use); break;
+    case 3: decode_words<T, 3>(r, count, plan, lane, use); break;
+    case 4: decode_words<T, 4>(r, count, plan, lane, use); break;
+    case 5: decode_words<T, 5>(r, count, plan, lane, use); break;
+    case 6: decode_words<T, 6>(r, count, plan, lane, use); break;
+    case 7: decode_words<T, 7>(r, count, plan, lane, use); break;
+    case 8: decode_words<T, 8>(r, count, plan, lane, use); break;
+    default: break;
   }
 }
 

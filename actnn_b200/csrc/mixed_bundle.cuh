@@ -47,11 +47,12 @@ template <int B> ACTNN_DEV uint32_t spread_codes_to_bytes(uint32_t r) {   // fou
   }
 }
 
-// Decodes the four groups of a bundle of width B.  `words[k]` is word 32k + lane of the bundle (zero
-// past its end); lane g < 4 holds the statistics of group g in (stat_scale, stat_mn).
-template <typename T, int B>
-ACTNN_DEV void decode_bundle(const uint32_t (&words)[8], float stat_scale, float stat_mn, const TransposePlan& plan,
-                             int lane, Oct<T> (&x)[kBundle]) {
+// Decodes the four groups of a bundle of width B and hands them on one by one, use(group, octet): only
+// one decoded octet per lane is live.  `words[k]` is word 32k + lane of the bundle (zero past its end);
+// lane g < 4 holds the statistics of group g in (stat_scale, stat_mn).
+template <typename T, int B, typename Use>
+ACTNN_DEV void decode_bundle(const uint32_t (&words)[B], float stat_scale, float stat_mn, const TransposePlan& plan,
+                             int lane, Use use) {
   constexpr int E = 1 << (B < 6 ? B : 5);              // table entries per group
   constexpr int GPC = (32 / E) < kBundle ? (32 / E) : kBundle;   // groups served by one table computation
   uint32_t S[B];
@@ -74,7 +75,8 @@ ACTNN_DEV void decode_bundle(const uint32_t (&words)[8], float stat_scale, float
     if (gi == 1) { lo = get_bits<1 * 8 * B, (8 * B < 32 ? 8 * B : 32)>(S); if constexpr (8 * B > 32) hi = get_bits<1 * 8 * B + 32, 8 * B - 32>(S); }
     if (gi == 2) { lo = get_bits<2 * 8 * B, (8 * B < 32 ? 8 * B : 32)>(S); if constexpr (8 * B > 32) hi = get_bits<2 * 8 * B + 32, 8 * B - 32>(S); }
     if (gi == 3) { lo = get_bits<3 * 8 * B, (8 * B < 32 ? 8 * B : 32)>(S); if constexpr (8 * B > 32) hi = get_bits<3 * 8 * B + 32, 8 * B - 32>(S); }
-    uint32_t* ow = reinterpret_cast<uint32_t*>(&x[gi]);
+    Oct<T> x;
+    uint32_t* ow = reinterpret_cast<uint32_t*>(&x);
     if constexpr (sizeof(T) == 2 && B <= 2) {
       const int base = (gi % GPC) * E;
       const uint32_t t01 = __shfl_sync(kFull, pairs, base);
@@ -114,6 +116,7 @@ ACTNN_DEV void decode_bundle(const uint32_t (&words)[8], float stat_scale, float
         for (int k = 0; k < 4; ++k) ow[k] = v[2 * k] | (v[2 * k + 1] << 16);
       }
     }
+    use(gi, x);
   }
 }
 

@@ -409,6 +409,12 @@ def _fused_bn_statistics(input, scheme, weight, bias, running_mean, running_var,
                                                       out=out)
 
 
+def _holds_codes(quantized):
+    """Whether a saved activation is the mixed stream over groups of 256 that the kernels decode."""
+    return (config.compress_activation and not config.simulate and config.group_size == 256
+            and isinstance(quantized[1], torch.Tensor))
+
+
 class batch_norm(Function):
     @staticmethod
     def forward(ctx, input, running_mean, running_var, weight, bias, training, exponential_average_factor, eps,
@@ -453,7 +459,16 @@ class batch_norm(Function):
     def backward(ctx, grad_output):
         quantized, weight, running_mean, running_var, save_mean, save_var, training, eps, reserve = ctx.saved
         q_input_shape, in_dtype = ctx.other_args
-        input = dequantize_activation(quantized, q_input_shape, in_dtype)
+        grads = None
+        if training and _holds_codes(quantized):
+            # both backward passes decode the codes themselves: the input is never written out
+            packed = swap_to_gpu(quantized[0]) if config.swap else quantized[0]
+            quantized = (packed,) + tuple(quantized[1:])
+            grads = ext_backward_func.batch_norm_codes_backward(quantized, tuple(q_input_shape), in_dtype, grad_output,
+                                                                weight, save_mean, save_var)
+        input = None
+        if grads is None:
+            input = dequantize_activation(quantized, q_input_shape, in_dtype)
         del quantized, ctx.saved
         empty_cache(config.empty_cache_threshold)
         if config.debug_memory_op_backward:
@@ -462,7 +477,9 @@ class batch_norm(Function):
             get_memory_usage(True)
             bn_layer_ct += 1
 
-        if training:
+        if grads is not None:
+            grad_input, grad_weight, grad_bias = grads
+        elif training:
             grad_input, grad_weight, grad_bias = ext_backward_func.cudnn_batch_norm_backward(
                 input.contiguous(), grad_output.contiguous(), weight, running_mean, running_var, save_mean,
                 save_var, eps, reserve)

@@ -253,6 +253,19 @@ int actnn_batch_norm_stats_minimax(const void* x, void* mn, void* mx, const floa
                                    int64_t N, int64_t C, int64_t HW, double momentum, double eps, int dtype,
                                    void* workspace, int64_t workspace_bytes, actnn_stream_t stream);
 
+/* The backward half of a training-mode batch norm straight from the compressed activation (mixed stream, groups of 256
+ * over samples of C * HW elements, as actnn_compress_mixed / actnn_compress_mixed_samples write them).  Replaces
+ * unpack + batch-norm backward, actnn/actnn/ops.py:470-493: the decoded activation only exists in registers.
+ * Arguments as in actnn_unpack_mixed and actnn_batch_norm_backward; stat_dtype is `dtype`, or bfloat16 for float32.
+ * Any C, HW >= 8.  grad_out / grad_in need the alignment of one element.  Scratch: *bytes of the first call (a host
+ * pointer; ACTNN_ERR_SHAPE: not covered), 16-byte aligned, for the current device. */
+int actnn_batch_norm_codes_workspace(int64_t N, int64_t C, int64_t HW, int dtype, int64_t* bytes);
+int actnn_batch_norm_codes_backward(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets,
+                                    const void* scale, const void* mn, const void* grad_out, const float* weight,
+                                    const float* save_mean, const float* save_invstd, void* grad_in,
+                                    float* grad_weight, float* grad_bias, int64_t N, int64_t C, int64_t HW, int dtype,
+                                    int stat_dtype, void* workspace, int64_t workspace_bytes, actnn_stream_t stream);
+
 /* ------------------------------------------------------------------------------------
  * actnn_compress_mixed for an activation whose per-group min / max are already known (from
  * actnn_batch_norm_stats_minimax or actnn_minimax): sensitivities, greedy allocation and pack,

@@ -1,0 +1,74 @@
+"""Batch-norm passes that work on the compressed activation, against decode + 64-bit arithmetic."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# (N, C, HW): one channel per octet, per half octet, changes inside octets; a channel over several columns and many
+# channels in a column; samples that are not whole groups; one sample; more samples than a block of 32
+SHAPES = [(2, 64, 3136), (70, 24, 784), (5, 3, 40), (37, 32, 196), (3, 20, 12), (40, 7, 49), (33, 5, 225), (1, 130, 9),
+          (6, 33, 8), (9, 2, 1600), (4, 3, 1029)]
+EPS = {torch.float16: 2 ** -11, torch.bfloat16: 2 ** -8, torch.float32: 2 ** -24}
+
+
+def compressed(n, c, hw, dtype, seed=0):
+    from actnn_b200.cpp_extension import quantization as q
+    torch.manual_seed(seed)
+    x = (torch.randn(n, c, hw, device="cuda") * 1.5 + torch.linspace(-1, 1, c, device="cuda").view(1, c, 1)).to(dtype)
+    stat = torch.bfloat16 if dtype == torch.float32 else dtype
+    f = c * hw
+    if f % 256:
+        out = q.compress_mixed_samples(x.view(n, f), 2 * n, 8, 0.5, philox=(1, 4), stat_dtype=stat)
+        x_hat = q.unpack_mixed_samples(out[0], out[1], out[2], out[3], (n, c, hw), out_dtype=dtype)
+    else:
+        out = q.compress_mixed_precision(x.view(n, f // 256, 256), 2 * n, 8, 0.5, philox=(1, 4), stat_dtype=stat)
+        x_hat = q.unpack_mixed_precision(*out[:4], n, f // 256, 256, out_dtype=dtype).view(n, c, hw)
+    return x, out[:4], x_hat
+
+
+def backward64(x_hat, dy, weight, mean, invstd):
+    x, g = x_hat.double(), dy.double()
+    m, i, w = (t.double().view(1, -1, 1) for t in (mean, invstd, weight))
+    cnt = x.shape[0] * x.shape[2]
+    sdy, sdyx = g.sum((0, 2)), (g * (x - m)).sum((0, 2))
+    dx = w * i * (g - sdy.view(1, -1, 1) / cnt - (x - m) * i * i * sdyx.view(1, -1, 1) / cnt)
+    return dx, sdyx * i.view(-1), sdy
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("offset", [0, 1])
+def test_backward_from_codes(shape, dtype, offset):
+    from actnn_b200.cpp_extension import backward_func as bf
+    n, c, hw = shape
+    x, quantized, x_hat = compressed(n, c, hw, dtype)
+    base = torch.randn(n * c * hw + offset, device="cuda").to(dtype)
+    dy = base[offset:].view(n, c, hw)
+    weight = torch.rand(c, device="cuda") + 0.5
+    mean = x.float().mean((0, 2))
+    invstd = 1 / torch.sqrt(x.float().var((0, 2), unbiased=False) + 1e-5)
+    dx, dw, db = bf.batch_norm_codes_backward(quantized, shape, dtype, dy, weight, mean, invstd)
+    rx, rw, rb = backward64(x_hat, dy, weight, mean, invstd)
+    # sums of N * HW float32 terms of order one in chains and trees: well under 64 roundings of the sum of magnitudes
+    mags = (dy.double().abs()).sum((0, 2)), (dy.double() * (x_hat.double() - mean.double().view(1, -1, 1))).abs().sum((0, 2))
+    assert ((db.double() - rb).abs() <= 64 * 2 ** -24 * mags[0] + 1e-6).all()
+    assert ((dw.double() - rw).abs() <= 64 * 2 ** -24 * mags[1] * invstd.double() + 1e-6).all()
+    # dx: a few float32 operations on values of order |w i| * max|dy|, then one rounding to the type
+    big = (weight * invstd).double().view(1, -1, 1) * (dy.double().abs().max() + (x_hat.double() - mean.double().view(1, -1, 1)).abs() * invstd.double().view(1, -1, 1))
+    assert ((dx.double() - rx).abs() <= (EPS[dtype] * 1.01 + 64 * 2 ** -24) * big + 1e-7).all()
+
+
+def test_layer_backward_takes_the_codes_and_agrees_with_the_decoded_path(monkeypatch):
+    import actnn_b200 as actnn
+    from actnn_b200.cpp_extension import backward_func as bf
+    layer = actnn.QBatchNorm2d(48).cuda()
+    x = torch.randn(20, 48, 14, 14, device="cuda", dtype=torch.float16).requires_grad_()
+    gy = torch.randn_like(x)
+    results = []
+    for use in (True, False):
+        if not use:
+            monkeypatch.setattr(bf, "batch_norm_codes_backward", lambda *a: None)
+        torch.manual_seed(5)
+        results.append(torch.autograd.grad(layer(x), [x, layer.weight, layer.bias], gy))
+    for a, b in zip(*results):
+        assert torch.allclose(a.float(), b.float(), rtol=2e-3, atol=2e-3 * b.float().abs().max().item())
