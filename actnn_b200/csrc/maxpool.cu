@@ -230,6 +230,151 @@ max_pool_forward_row_kernel(const T* __restrict__ x, T* __restrict__ y, int8_t* 
   }
 }
 
+// Forward for 16-bit types, the same geometries with equal row and column padding P: a thread walks down
+// `rows` output rows of a segment of eight output columns.  Everything stays in packed pairs, two output columns
+// per register: pair k of tap kw holds the inputs that outputs 2k and 2k + 1 see through that tap.  An input
+// row is loaded and regrouped once, although two windows of height 3 share every other row.  The maximum
+// comes first (packed max), the arg-max by comparing the taps with it from the last to the first, so that
+// the first of equals wins; a window without any value above -infinity keeps code 0.
+// Bound by HBM: 205 MB in, 77 MB out for float16 128 x 64 x 112 x 112, 3 x 3 / 2.  The version that compared
+// in float32, one output at a time and every row three times, took 69.9 us; this one 57.9 (4.9 TB/s).
+template <typename T> struct Packed;
+template <> struct Packed<__half> {
+  using V = __half2;
+  static constexpr uint32_t kLowest = 0xFC00FC00u;               // -infinity
+};
+template <> struct Packed<__nv_bfloat16> {
+  using V = __nv_bfloat162;
+  static constexpr uint32_t kLowest = 0xFF80FF80u;
+};
+template <typename T> ACTNN_DEV uint32_t packed_max(uint32_t a, uint32_t b) {
+  using V = typename Packed<T>::V;
+  const V r = __hmax2(*reinterpret_cast<const V*>(&a), *reinterpret_cast<const V*>(&b));     // NaN loses
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+template <typename T> ACTNN_DEV uint32_t packed_equal(uint32_t a, uint32_t b) {               // 0xffff per equal half
+  using V = typename Packed<T>::V;
+  return __heq2_mask(*reinterpret_cast<const V*>(&a), *reinterpret_cast<const V*>(&b));
+}
+
+// Sixteen columns from c0 of an input row and one beside them, as loaded.  Ordinary cached loads: the side column is
+// in a neighbouring thread's sector.  `wide`: one 32-byte load.
+template <typename T, int K, int P> struct RawRow {
+  uint32_t c[8], side;                                           // side: column left (P = 1) or right (K - P = 3) of the sixteen
+  ACTNN_DEV void load(const T* r, int c0, int W, bool wide) {
+    constexpr uint32_t low = Packed<T>::kLowest;
+    side = low;
+    if (wide && r != nullptr && c0 + 16 <= W) {
+      asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]), "=r"(c[4]), "=r"(c[5]), "=r"(c[6]), "=r"(c[7])
+                   : "l"(r + c0));
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {                              // W % 8 == 0: an octet is whole or absent (c0 == W: the last
+        uint4 v = make_uint4(low, low, low, low);                // window of K = 2, P = 1 sees column W - 1 only)
+        if (r != nullptr && c0 + 8 * h + 8 <= W) v = __ldg(reinterpret_cast<const uint4*>(r + c0 + 8 * h));
+        c[4 * h] = v.x; c[4 * h + 1] = v.y; c[4 * h + 2] = v.z; c[4 * h + 3] = v.w;
+      }
+    }
+    if constexpr (P == 1) { if (r != nullptr && c0 >= 1) side = __ldg(reinterpret_cast<const uint16_t*>(r + c0 - 1)); }
+    if constexpr (K - P == 3) { if (r != nullptr && c0 + 16 < W) side = __ldg(reinterpret_cast<const uint16_t*>(r + c0 + 16)); }
+  }
+};
+template <typename T, int K, int P> struct PoolRow {
+  uint32_t tap[K][4];
+  ACTNN_DEV void regroup(const RawRow<T, K, P>& raw) {
+    uint32_t even[4], odd[4];                                    // columns 2i resp. 2i + 1 of outputs i = 2k, 2k + 1
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      even[k] = __byte_perm(raw.c[2 * k], raw.c[2 * k + 1], 0x5410);
+      odd[k] = __byte_perm(raw.c[2 * k], raw.c[2 * k + 1], 0x7632);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      tap[P][k] = even[k];
+      if constexpr (P + 1 < K) tap[P + 1][k] = odd[k];
+      if constexpr (P == 1) tap[0][k] = k ? __byte_perm(odd[k ? k - 1 : 0], odd[k], 0x5432) : __byte_perm(raw.side, odd[0], 0x5410);
+      if constexpr (K - P == 3) tap[2][k] = k < 3 ? __byte_perm(even[k], even[k < 3 ? k + 1 : 3], 0x5432) : __byte_perm(even[3], raw.side, 0x5432);
+    }
+  }
+};
+
+template <typename T, int K, int P>
+__global__ void __launch_bounds__(256)
+max_pool_forward_packed_kernel(const T* __restrict__ x, T* __restrict__ y, int8_t* __restrict__ idx, uint32_t total,
+                               int segs, int chunks, int rows, PoolGeom g, int vector_store, int wide_rows) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  const bool wide = wide_rows != 0;
+  const uint32_t strip = t / (uint32_t)segs;
+  const int seg = (int)(t - strip * (uint32_t)segs);
+  const uint32_t nc = strip / (uint32_t)chunks;
+  const int ho0 = (int)(strip - nc * (uint32_t)chunks) * rows, ho1 = min(g.Ho, ho0 + rows);
+  const int wo0 = seg * 8, c0 = 2 * wo0;
+  const T* plane = x + (int64_t)nc * g.H * g.W;
+  auto row = [&](int h) { return h >= 0 && h < g.H ? plane + (int64_t)h * g.W : (const T*)nullptr; };
+  PoolRow<T, K, P> r[K];
+  RawRow<T, K, P> n0, n1;                                        // the two rows the next window adds, requested a window ahead
+  if constexpr (K == 3) {
+    n0.load(row(2 * ho0 - P), c0, g.W, wide);
+    r[2].regroup(n0);
+  }
+  n0.load(row(2 * ho0 - P + K - 2), c0, g.W, wide);
+  n1.load(row(2 * ho0 - P + K - 1), c0, g.W, wide);
+  for (int ho = ho0; ho < ho1; ++ho) {
+    if constexpr (K == 3) r[0] = r[2];                           // the last row of the window above is the first of this one
+    r[K - 2].regroup(n0);
+    r[K - 1].regroup(n1);
+    if (ho + 1 < ho1) {
+      n0.load(row(2 * ho - P + K), c0, g.W, wide);
+      n1.load(row(2 * ho - P + K + 1), c0, g.W, wide);
+    }
+    uint32_t best[4], arg[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      uint32_t m = Packed<T>::kLowest;
+#pragma unroll
+      for (int kh = 0; kh < K; ++kh)
+#pragma unroll
+        for (int kw = 0; kw < K; ++kw) m = packed_max<T>(m, r[kh].tap[kw][k]);
+      uint32_t a = 0u;
+#pragma unroll
+      for (int c = K * K - 1; c >= 1; --c) {
+        const uint32_t eq = packed_equal<T>(m, r[c / K].tap[c % K][k]);
+        a = (eq & ((uint32_t)c * 0x00010001u)) | (~eq & a);
+      }
+      a &= ~(packed_equal<T>(m, r[0].tap[0][k]) | packed_equal<T>(m, Packed<T>::kLowest));
+      best[k] = m;
+      arg[k] = a;
+    }
+    const int64_t o = ((int64_t)nc * g.Ho + ho) * g.Wo + wo0;
+    if (vector_store) {                                          // Wo % 8 == 0, aligned outputs
+      Oct<T> out;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) out.r[k] = best[k];
+      store_oct<T>(y + o, out);
+      *reinterpret_cast<uint2*>(idx + o) =
+          make_uint2(__byte_perm(arg[0], arg[1], 0x6420), __byte_perm(arg[2], arg[3], 0x6420));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (wo0 + i < g.Wo) {
+          reinterpret_cast<uint16_t*>(y)[o + i] = (uint16_t)(best[i / 2] >> (16 * (i & 1)));
+          idx[o + i] = (int8_t)(arg[i / 2] >> (16 * (i & 1)));
+        }
+      }
+    }
+  }
+}
+
+// Rows a thread of the strip kernels walks: eight (an input row is regrouped once, the shared one at the head
+// of a strip twice), fewer where that would leave the chip short of threads.
+int strip_rows(int64_t planes, int segs, int row_count) {
+  int rows = 8;
+  while (rows > 1 && planes * segs * ((row_count + rows - 1) / rows) < (int64_t)device_info().sm_count * 2048) rows >>= 1;
+  return rows;
+}
+
 template <typename T>
 int launch_forward(const void* x, void* y, int8_t* idx, int64_t planes, const PoolGeom& g, cudaStream_t s) {
   const int out_elems = g.Ho * g.Wo;
@@ -239,6 +384,23 @@ int launch_forward(const void* x, void* y, int8_t* idx, int64_t planes, const Po
   if (unit && (g.KH == 2 || g.KH == 3) && g.SW == 2 && g.PW <= 1 && g.W % 8 == 0 && aligned(x, sizeof(T) * 8) &&
       total_segments < ((int64_t)1 << 31)) {
     const int vec = g.Wo % 8 == 0 && aligned(y, sizeof(T) * 8) && aligned(idx, 8);
+    if constexpr (sizeof(T) == 2) {
+      if (g.PH == g.PW && g.SH == 2) {
+        const int rows = strip_rows(planes, segs, g.Ho), chunks = (g.Ho + rows - 1) / rows;
+        const int64_t total = planes * segs * chunks;            // <= total_segments
+        const int pgrid = (int)((total + 255) / 256);
+        const int wide = g.W % 16 == 0 && aligned(x, 32);
+#define ACTNN_PACKED(K, P)                                                                                     \
+        max_pool_forward_packed_kernel<T, K, P><<<pgrid, 256, 0, s>>>((const T*)x, (T*)y, idx, (uint32_t)total, segs, \
+                                                                      chunks, rows, g, vec, wide)
+        if (g.KH == 3 && g.PW == 1) ACTNN_PACKED(3, 1);
+        else if (g.KH == 3) ACTNN_PACKED(3, 0);
+        else if (g.PW == 1) ACTNN_PACKED(2, 1);
+        else ACTNN_PACKED(2, 0);
+#undef ACTNN_PACKED
+        return check_launch();
+      }
+    }
     const int64_t blocks = (total_segments + 255) / 256;
     const int rgrid = (int)max((int64_t)1, min(blocks, (int64_t)device_info().sm_count * 16));
 #define ACTNN_ROW(K, P)                                                                                       \
@@ -520,6 +682,126 @@ max_pool_backward_s2_kernel(const T* __restrict__ gy, const int8_t* __restrict__
   }
 }
 
+// Backward by strips, the geometries above with equal row and column padding: a thread walks down `rows` pairs
+// of input rows of a segment of eight columns.  Pair r is the rows 2r - P and 2r + 1 - P: windows of height 3
+// reach the first through their last row (window row r - 1) and their first (r), the second through their middle
+// row (r) only, so every window row is loaded once per strip, kept for the next pair, and only the
+// 9 / 4 candidates a position has on average are compared (the segment kernel compares 2 rows of 5 for every row).
+// The order of additions is that of the general kernel.  float16 128 x 64 x 112 x 112, 3 x 3 / 2 (282 MB): segment
+// kernel 128.0 us, bound by instruction issue; strips 71.7, with the next window row requested ahead 63.8.
+template <typename T, int K, int P> struct PoolWindows {
+  static constexpr int BLO = (K == 3 && P == 0) ? -1 : 0, BHI = P == 1 ? 4 : 3, NB = BHI - BLO + 1;
+  static constexpr bool kSide = NB == 5;                         // a fifth window column, left (BLO) or right (BHI) of the four
+  // as loaded: codes and gradients of window columns b0 .. b0 + 3 of a window row, and the fifth
+  struct Raw {
+    uint32_t codes, side_code;
+    T grads[4], side_grad;
+  };
+  // Window row ho; windows that do not exist get code 0xff.
+  static ACTNN_DEV void request(Raw& raw, const T* gy_p, const int8_t* idx_p, int ho, int b0, const PoolGeom& g, int vector_load) {
+    raw.codes = 0xffffffffu;
+    raw.side_code = 0xffu;
+    if (ho < 0 || ho >= g.Ho) return;                            // their gradients are never looked at
+    const int base = ho * g.Wo + b0;
+    if (vector_load && b0 + 4 <= g.Wo) {
+      raw.codes = __ldg(reinterpret_cast<const uint32_t*>(idx_p + base));
+      if constexpr (sizeof(T) == 4) *reinterpret_cast<float4*>(raw.grads) = __ldg(reinterpret_cast<const float4*>(gy_p + base));
+      else *reinterpret_cast<uint2*>(raw.grads) = __ldg(reinterpret_cast<const uint2*>(gy_p + base));
+    } else {
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        if (b0 + b < g.Wo) {
+          raw.codes = (raw.codes & ~(0xffu << (8 * b))) | ((uint32_t)(uint8_t)idx_p[base + b] << (8 * b));
+          raw.grads[b] = gy_p[base + b];
+        }
+      }
+    }
+    if constexpr (kSide) {
+      const int b = BLO < 0 ? -1 : 4;
+      if (b0 + b >= 0 && b0 + b < g.Wo) {
+        raw.side_code = (uint8_t)idx_p[base + b];
+        raw.side_grad = gy_p[base + b];
+      }
+    }
+  }
+  int code[NB];
+  float grad[NB];
+  ACTNN_DEV void set(const Raw& raw) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      code[b - BLO] = (int)((raw.codes >> (8 * b)) & 0xffu);
+      grad[b - BLO] = (float)raw.grads[b];
+    }
+    if constexpr (kSide) {
+      code[BLO < 0 ? 0 : NB - 1] = (int)raw.side_code;
+      grad[BLO < 0 ? 0 : NB - 1] = (float)raw.side_grad;
+    }
+  }
+  // adds what the windows give to the input row they reach through tap row kh
+  template <int KH> ACTNN_DEV void add(float (&acc)[8]) const {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int q = j + P, b_hi = q >> 1, kw_hi = q & 1;         // compile-time after unrolling
+      if (K == 3 && kw_hi == 0 && b_hi - 1 >= BLO) {
+        if (code[b_hi - 1 - BLO] == KH * K + 2) acc[j] += grad[b_hi - 1 - BLO];
+      }
+      if (b_hi <= BHI) {
+        if (code[b_hi - BLO] == KH * K + kw_hi) acc[j] += grad[b_hi - BLO];
+      }
+    }
+  }
+};
+
+template <typename T, int K, int P>
+__global__ void __launch_bounds__(256)
+max_pool_backward_strip_kernel(const T* __restrict__ gy, const int8_t* __restrict__ idx, T* __restrict__ gx,
+                               uint32_t total, int segs, int chunks, int rows, PoolGeom g, int vector_load) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  const uint32_t strip = t / (uint32_t)segs;
+  const int seg = (int)(t - strip * (uint32_t)segs);
+  const uint32_t nc = strip / (uint32_t)chunks;
+  const int pairs = (g.H - 1 + P) / 2 + 1;
+  const int r0 = (int)(strip - nc * (uint32_t)chunks) * rows, r1 = min(pairs, r0 + rows);
+  const T* gy_p = gy + (int64_t)nc * g.Ho * g.Wo;
+  const int8_t* idx_p = idx + (int64_t)nc * g.Ho * g.Wo;
+  T* out = gx + (int64_t)nc * g.H * g.W + seg * 8;
+  auto store = [&](int h, const float (&acc)[8]) {
+    if (h < 0 || h >= g.H) return;
+    Oct<T> o;
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o.f[j] = acc[j];
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        o.r[k] = bits_of<T>(round_to<T>(acc[2 * k])) | (bits_of<T>(round_to<T>(acc[2 * k + 1])) << 16);
+    }
+    store_oct<T>(out + (int64_t)h * g.W, o);
+  };
+  using Windows = PoolWindows<T, K, P>;
+  Windows above, here;
+  typename Windows::Raw next;                                    // requested a pair ahead
+  if constexpr (K == 3) {
+    Windows::request(next, gy_p, idx_p, r0 - 1, seg * 4, g, vector_load);
+    here.set(next);
+  }
+  Windows::request(next, gy_p, idx_p, r0, seg * 4, g, vector_load);
+  for (int r = r0; r < r1; ++r) {
+    if constexpr (K == 3) above = here;
+    here.set(next);
+    if (r + 1 < r1) Windows::request(next, gy_p, idx_p, r + 1, seg * 4, g, vector_load);
+    float first[8], second[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) first[j] = second[j] = 0.f;
+    if constexpr (K == 3) above.template add<2>(first);
+    here.template add<0>(first);
+    here.template add<1>(second);
+    store(2 * r - P, first);
+    store(2 * r + 1 - P, second);
+  }
+}
+
 template <typename T>
 int launch_backward(const void* gy, const int8_t* idx, void* gx, int64_t planes, const PoolGeom& g, cudaStream_t s) {
   const int plane_elems = g.H * g.W;
@@ -533,6 +815,21 @@ int launch_backward(const void* gy, const int8_t* idx, void* gx, int64_t planes,
   if (unit && g.KH == g.KW && (g.KH == 2 || g.KH == 3) && g.SH == 2 && g.SW == 2 && g.PW <= 1 && g.W % 8 == 0 &&
       aligned(gx, sizeof(T) * 8) && total_segments < ((int64_t)1 << 31)) {
     const int vec = g.Wo % 4 == 0 && aligned(gy, sizeof(T) * 4) && aligned(idx, 4);
+    if (g.PH == g.PW) {
+      const int pairs = (g.H - 1 + g.PH) / 2 + 1;
+      const int rows = strip_rows(planes, segs, pairs), chunks = (pairs + rows - 1) / rows;
+      const int64_t total = planes * segs * chunks;              // <= total_segments + planes * segs
+      const int sgrid = (int)((total + 255) / 256);
+#define ACTNN_STRIP(K, P)                                                                                          \
+      max_pool_backward_strip_kernel<T, K, P><<<sgrid, 256, 0, s>>>((const T*)gy, idx, (T*)gx, (uint32_t)total, segs, \
+                                                                    chunks, rows, g, vec)
+      if (g.KH == 3 && g.PW == 1) ACTNN_STRIP(3, 1);
+      else if (g.KH == 3) ACTNN_STRIP(3, 0);
+      else if (g.PW == 1) ACTNN_STRIP(2, 1);
+      else ACTNN_STRIP(2, 0);
+#undef ACTNN_STRIP
+      return check_launch();
+    }
     const int64_t blocks = (total_segments + 255) / 256;
     const int grid = (int)max((int64_t)1, min(blocks, (int64_t)device_info().sm_count * 16));
 #define ACTNN_S2(K, P)                                                                                      \
