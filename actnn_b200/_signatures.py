@@ -30,6 +30,7 @@ SIGNATURES = {
     "actnn_range_sqr": ['P', 'P', 'L', 'L', 'I', 'F', 'F', 'P', 'P', 'P'],
     "actnn_sample_sumsq": ['P', 'P', 'L', 'L', 'I', 'P'],
     "actnn_calc_precision": ['P', 'P', 'L', 'I', 'D', 'P', 'P', 'L', 'L', 'P', 'L', 'P'],
+    "actnn_allocate_layers": ['P', 'P', 'I', 'L', 'I', 'D', 'P', 'P'],
     "actnn_relu_forward": ['P', 'P', 'P', 'L', 'I', 'P'],
     "actnn_relu_forward_minimax": ['P', 'P', 'P', 'P', 'P', 'L', 'I', 'P'],
     "actnn_relu_backward": ['P', 'P', 'P', 'L', 'I', 'P'],

@@ -6,6 +6,8 @@ CPU tensors; here the same result comes from one CUDA kernel.  CPU tensors are a
 (copied to the current device and back, as a drop-in must); CUDA tensors are processed in
 place without any host synchronisation.  ``allocate_bits`` is the sync-free entry the
 schemes use: it also returns the word offsets of the mixed-precision stream."""
+import array
+
 import torch
 
 from .. import _lib
@@ -36,6 +38,28 @@ def allocate_bits(C: torch.Tensor, initial_bits: int, target: float, w: torch.Te
               bits.data_ptr(), _lib.ptr(offsets), int(num_groups), int(group_size), _lib.ptr(ws),
               0 if ws is None else 256, _lib.stream_of(C))
     return bits, offsets
+
+
+MAX_LAYERS, MAX_LAYER_SAMPLES = 256, 32768            # of actnn_allocate_layers
+
+
+def allocate_layers(Cs, dims, initial_bits: int, target: float):
+    """``allocate_bits`` over the concatenation of the layers' sensitivities ``Cs`` (float32 CUDA ``[N]`` each) with
+    weight ``dims[l]`` for layer ``l``, reduced to the sum of each layer's widths: int32 CUDA ``[L]`` from one launch.
+    ``None`` when the problem does not fit that kernel."""
+    first = Cs[0]
+    n, dev = first.numel(), first.device
+    if not 1 <= initial_bits <= 8 or len(Cs) > MAX_LAYERS or n * len(Cs) > MAX_LAYER_SAMPLES or not first.is_cuda:
+        return None
+    for C, d in zip(Cs, dims):
+        if C.numel() != n or C.dtype != torch.float32 or C.device != dev or not C.is_contiguous() \
+                or not 0 < d < 2 ** 31:
+            return None
+    sums = torch.empty(len(Cs), dtype=torch.int32, device=dev)
+    ptrs, weights = array.array("Q", [C.data_ptr() for C in Cs]), array.array("i", dims)
+    _lib.call("actnn_allocate_layers", first, ptrs.buffer_info()[0], weights.buffer_info()[0], len(Cs), n,
+              int(initial_bits), float(target), sums.data_ptr(), _lib.stream_of(first))
+    return sums
 
 
 def sensitivity(mn: torch.Tensor, mx: torch.Tensor, n: int, range_factor: float, coeff: float = 1.0,

@@ -180,10 +180,17 @@ class QScheme(object):
             else:
                 # joint allocation over layers x samples, then the per-layer average
                 N = layers[0].C.shape[0]
+                total = float(sum(layer.dim for layer in layers) * N * group_bits)
+                sums = ext_calc_precision.allocate_layers([layer.C for layer in layers], [layer.dim for layer in layers],
+                                                          config.initial_bits, total)
+                if sums is not None:
+                    means = sums.cpu().float() / N                 # the one host read per step, see below
+                    for i, layer in enumerate(layers):
+                        layer.bits = means[i]
+                    continue
                 C = torch.cat([layer.C for layer in layers], 0).contiguous()
                 w = torch.tensor([layer.dim for layer in layers], dtype=torch.int32,
                                  device=device).repeat_interleave(N).contiguous()
-                total = float(sum(layer.dim for layer in layers) * N * group_bits)
                 b, _ = ext_calc_precision.allocate_bits(C, config.initial_bits, total, w)
                 # the one host read per step.  Integer sums are exact on any device; the division
                 # is done on the host in float32 like the reference's ``bs.float().mean()``

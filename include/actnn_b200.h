@@ -171,6 +171,14 @@ int actnn_calc_precision(const float* C, const int32_t* w, int64_t N, int initia
                          int64_t G, int64_t group_size, void* workspace, int64_t workspace_bytes,
                          actnn_stream_t stream);
 
+/* The joint allocation over layers x samples that a step ends with (QScheme.allocate_perlayer,
+ * actnn/actnn/qscheme.py:96-128): actnn_calc_precision over the concatenation of L sensitivity vectors C[l][N] with
+ * the weight dims[l] > 0 for layer l's samples, and the sum of the widths of each layer's samples, sums[L].  C and dims
+ * are host arrays (of device pointers / values), read before the call returns.  One launch.  initial_bits 1..8;
+ * ACTNN_ERR_CAPACITY for L > 256 or N * L > 32768 (take actnn_calc_precision then). */
+int actnn_allocate_layers(const float* const* C, const int32_t* dims, int L, int64_t N, int initial_bits,
+                          double target, int32_t* sums, actnn_stream_t stream);
+
 /* The adaptive compress of one activation as one call: per-group min/max, sensitivities,
  * greedy allocation at `target` total bits, scale + stochastic rounding + mixed-precision
  * pack.  Replaces the sequence QScheme.compute_quantization_bits -> quantize_and_pack,
