@@ -25,6 +25,7 @@ SIGNATURES = {
     "actnn_compress_mixed_prestat_kept": ['P'] * 10 + ['L', 'L', 'L', 'I', 'I', 'F', 'F', 'P', 'I', 'D', 'I', 'P', 'U', 'U',
                                           'P'],
     "actnn_batch_norm_stats_minimax": ['P'] * 9 + ['L', 'L', 'L', 'D', 'D', 'I', 'P', 'L', 'P'],
+    "actnn_transpose16": ['P', 'P', 'L', 'L', 'L', 'P'],
     "actnn_batch_norm_codes_workspace": ['L', 'L', 'L', 'I', 'P'],
     "actnn_batch_norm_codes_backward": ['P'] * 12 + ['L', 'L', 'L', 'I', 'I', 'P', 'L', 'P'],
     "actnn_range_sqr": ['P', 'P', 'L', 'L', 'I', 'F', 'F', 'P', 'P', 'P'],

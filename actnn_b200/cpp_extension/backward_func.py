@@ -62,6 +62,44 @@ def cudnn_convolution_transpose_backward(input, grad_output, weight, padding, ou
     return gi, gw
 
 
+# ---------------------------------------------------------------------------------------
+# channels-last around the convolution library
+# ---------------------------------------------------------------------------------------
+def channels_last_pays(input, weight, groups) -> bool:
+    """Whether a 2-D convolution of contiguous NCHW tensors is computed on channels-last copies.
+
+    cuDNN has only NHWC kernels for 16-bit convolutions with more than one tap on this GPU, so for
+    NCHW operands it converts each of them in every call (in a backward pass the gradient twice).  Measured on a
+    B200, float16, forward + backward: 3x3, 256 x 64 x 56 x 56: 742 us on NCHW, 230 on NHWC operands, 31
+    per converted tensor; 256 x 256 x 28 x 28: 920 against 509.  1x1 convolutions are matrix products in
+    either layout (188 against 157, less than the conversions cost) and stay; so do channel counts that
+    NHWC kernels cannot read in 16-byte vectors, grouped convolutions and float32, whose NCHW path
+    does not go through the same kernels."""
+    return (input.dim() == 4 and input.is_cuda and input.dtype in (torch.float16, torch.bfloat16)
+            and weight.dtype == input.dtype and groups == 1 and weight.shape[2] * weight.shape[3] > 1
+            and weight.shape[0] % 8 == 0 and weight.shape[1] % 8 == 0 and input.shape[1] == weight.shape[1]
+            and input.shape[2] * input.shape[3] > 1 and input.is_contiguous() and weight.is_contiguous()
+            and torch.backends.cudnn.enabled)
+
+
+def to_channels_last(x):
+    """A channels-last copy of a contiguous 16-bit NCHW tensor."""
+    n, c, h, w = x.shape
+    out = torch.empty(x.shape, dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
+    _lib.call("actnn_transpose16", x, x.data_ptr(), out.data_ptr(), n, c, h * w, _lib.stream_of(x))
+    return out
+
+
+def to_planes(x):
+    """The contiguous NCHW form of a 16-bit tensor that came back channels-last."""
+    if x.is_contiguous() or not x.is_contiguous(memory_format=torch.channels_last):
+        return x.contiguous()
+    n, c, h, w = x.shape
+    out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    _lib.call("actnn_transpose16", x, x.data_ptr(), out.data_ptr(), n, h * w, c, _lib.stream_of(x))
+    return out
+
+
 def _as_f32(t):
     return None if t is None else (t if t.dtype == torch.float32 else t.float()).contiguous()
 

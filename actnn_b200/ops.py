@@ -240,6 +240,10 @@ class convnd(Function):
             empty_cache(config.empty_cache_threshold)
             if config.debug_memory_op_forward:
                 _debug_forward("conv%dd" % n, quantized)
+            if n == 2 and ext_backward_func.channels_last_pays(input, weight, groups):
+                return ext_backward_func.to_planes(forward_op(
+                    ext_backward_func.to_channels_last(input), ext_backward_func.to_channels_last(weight), bias,
+                    stride, padding, dilation, groups))
             return forward_op(input, weight, bias, stride, padding, dilation, groups)
 
     @staticmethod
@@ -267,6 +271,11 @@ class convnd(Function):
         if use_pipeline:
             grad_input, grad_weight = _chunked_conv_backward(
                 ext_backward_func.cudnn_convolution_backward, input, grad_output, weight, args, needs)
+        elif n == 2 and ext_backward_func.channels_last_pays(input, weight, groups):
+            grad_input, grad_weight = (g if g is None else ext_backward_func.to_planes(g) for g in
+                                       ext_backward_func.cudnn_convolution_backward(
+                ext_backward_func.to_channels_last(input), ext_backward_func.to_channels_last(grad_output.contiguous()),
+                ext_backward_func.to_channels_last(weight), *args, config.cudnn_benchmark_conv2d, False, False, needs))
         else:
             grad_input, grad_weight = ext_backward_func.cudnn_convolution_backward(
                 input, grad_output, weight, *args, config.cudnn_benchmark_conv2d, False, False, needs)

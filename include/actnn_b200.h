@@ -261,6 +261,10 @@ int actnn_batch_norm_stats_minimax(const void* x, void* mn, void* mx, const floa
                                    int64_t N, int64_t C, int64_t HW, double momentum, double eps, int dtype,
                                    void* workspace, int64_t workspace_bytes, actnn_stream_t stream);
 
+/* [batch, rows, cols] -> [batch, cols, rows] for 16-bit elements: NCHW <-> NHWC around the convolution
+ * library (reference call sites: actnn/actnn/ops.py:163-220).  in and out must not overlap. */
+int actnn_transpose16(const void* in, void* out, int64_t batch, int64_t rows, int64_t cols, actnn_stream_t stream);
+
 /* The backward half of a training-mode batch norm straight from the compressed activation (mixed stream, groups of 256
  * over samples of C * HW elements, as actnn_compress_mixed / actnn_compress_mixed_samples write them).  Replaces
  * unpack + batch-norm backward, actnn/actnn/ops.py:470-493: the decoded activation only exists in registers.
