@@ -27,6 +27,7 @@ SIGNATURES = {
     "actnn_batch_norm_stats_minimax": ['P'] * 9 + ['L', 'L', 'L', 'D', 'D', 'I', 'P', 'L', 'P'],
     "actnn_transpose16": ['P', 'P', 'L', 'L', 'L', 'P'],
     "actnn_batch_norm_codes_workspace": ['L', 'L', 'L', 'I', 'P'],
+    "actnn_batch_norm_codes_forward": ['P'] * 16 + ['L', 'L', 'L', 'D', 'D', 'I', 'I', 'F', 'I', 'D', 'I', 'U', 'U', 'P', 'P', 'L', 'P'],
     "actnn_batch_norm_codes_backward": ['P'] * 12 + ['L', 'L', 'L', 'I', 'I', 'P', 'L', 'P'],
     "actnn_range_sqr": ['P', 'P', 'L', 'L', 'I', 'F', 'F', 'P', 'P', 'P'],
     "actnn_sample_sumsq": ['P', 'P', 'L', 'L', 'I', 'P'],

@@ -179,6 +179,53 @@ def _codes_workspace(N, C, HW, dtype_id, device_index):
     return None if status else nbytes.value
 
 
+def batch_norm_codes_forward(x, weight, bias, running_mean, running_var, momentum, eps, target_bits, initial_bits,
+                             range_factor, stochastic, stats=None):
+    """Training-mode batch norm of a contiguous ``x`` and its compressed copy in one native call:
+    ``(y, (packed, bits, scale, min), mean, invstd)``, or ``None`` when the geometry is not covered (nothing
+    has been drawn or written then).  ``stats``: what ``batch_norm_stats_minimax`` returned for ``x``, when it was
+    called (and has updated the running statistics).  The same codes as ``compress_mixed_precision`` with the next Philox offset."""
+    if x.dim() < 2 or x.dtype not in (torch.float16, torch.bfloat16, torch.float32) or x.numel() == 0:
+        return None
+    for t in (running_mean, running_var):
+        if t is not None and (t.dtype != torch.float32 or not t.is_contiguous()):
+            return None
+    N, C, HW = _bn_dims(x)
+    dev, dt = x.device, _lib.dtype_id(x.dtype)
+    nbytes = _codes_workspace(N, C, HW, dt, dev.index)
+    if nbytes is None:
+        return None
+    stat = torch.bfloat16 if x.dtype == torch.float32 else x.dtype
+    G = (C * HW + 255) // 256
+    total = min(initial_bits * N, max(int(target_bits), N))        # what the greedy ends with
+    w32, b32 = _as_f32(weight), _as_f32(bias)
+    y = torch.empty_like(x)
+    packed = torch.empty(total * G * 8, dtype=torch.int32, device=dev)
+    scale = torch.empty((N, G, 1), dtype=stat, device=dev)
+    mn = torch.empty((N, G, 1), dtype=stat, device=dev)
+    bits = torch.empty(N, dtype=torch.int32, device=dev)
+    offsets = torch.empty(N + 1, dtype=torch.int64, device=dev)
+    if stats is None:
+        floats = torch.empty(2 * C + N, dtype=torch.float32, device=dev)      # mean, invstd, sensitivities
+        gmn = gmx = None
+        mean, invstd, sens = floats[:C], floats[C:2 * C], floats.data_ptr() + 8 * C
+    else:
+        gmn, gmx, mean, invstd = stats
+        floats = torch.empty(N, dtype=torch.float32, device=dev)
+        sens = floats.data_ptr()
+    seed, offset = _lib.next_philox(dev) if stochastic else (0, 0)
+    ws = _lib.scratch(dev, nbytes)
+    _lib.call("actnn_batch_norm_codes_forward", x, x.data_ptr(), _lib.ptr(gmn), _lib.ptr(gmx), _lib.ptr(w32),
+              _lib.ptr(b32), _lib.ptr(running_mean), _lib.ptr(running_var), y.data_ptr(), mean.data_ptr(),
+              invstd.data_ptr(), packed.data_ptr(), scale.data_ptr(), mn.data_ptr(), bits.data_ptr(),
+              offsets.data_ptr(), sens, N, C, HW, float(momentum), float(eps), dt,
+              _lib.dtype_id(stat), float(range_factor), int(initial_bits), float(target_bits), int(bool(stochastic)),
+              seed, offset, _lib.ticket(dev).data_ptr(), ws.data_ptr(), nbytes, _lib.stream_of(x))
+    packed.word_offsets = bits.word_offsets = offsets
+    bits.total_bits = total
+    return y, (packed, bits, scale, mn), mean, invstd
+
+
 def batch_norm_codes_backward(quantized, shape, dtype, grad_output, weight, save_mean, save_invstd):
     """Backward of a training-mode batch norm from the compressed input: what ``dequantize_activation``
     followed by ``cudnn_batch_norm_backward`` computes (ops.py:470-493), with the decoded input in

@@ -1,4 +1,15 @@
-// Batch-norm passes that work on the compressed activation, on the column mapping (column.cuh).
+// Batch-norm passes fused with the compression of their input, on the column mapping (column.cuh).
+//
+// Forward: one read of x gives the statistics and the group ranges, the second packs AND normalises:
+//   stats   min / max of the bundle's groups, sums of (x - shift) and its square per octet in registers;
+//   finish  one warp per channel: mean, inverse deviation, running statistics, coefficients;
+//   (allocation of the widths, stats.cu)
+//   pack    codes and y from the same registers.
+// (Statistics and ranges of maps of 256 and more whole groups come from bn_stats_minimax_kernel in batch_norm.cu
+// instead, which the synchronised batch norm shares; see the binding.)
+// 4 + b/8 + 2 bytes an element for 16-bit types; statistics, pack and normalisation as passes of their own read x
+// three times.  float16 256 x 64 x 56 x 56: pack 28.1 + coefficients 1.6 + normalise 32.4 us -> 41.6 us (6.1 TB/s would be
+// 36, the rest is instruction issue); 128 x 256 x 14 x 14, seven launches 34 us -> four 24.6 us.
 //
 // Backward: both passes decode the saved codes in registers, so the decoded activation is never
 // written to memory (the reference decodes it, ops.py:470-476, and cuDNN reads it back, ops.py:490-493):
@@ -150,9 +161,147 @@ ACTNN_DEV float2 collect_partials(const ColumnShape& sh, const BnColumns& bn, co
   return make_float2(a, b);
 }
 
-// ------------------------------------------------------------------ backward
 constexpr int kBnBlocks = 2;     // resident blocks per SM: 128 registers and no spills beat 3 blocks with them (40.1 against 41.3 us, apply)
 
+constexpr int bn_stats_blocks(int elem_size, int sub) { return elem_size == 2 && sub == 8 ? 3 : 2; }
+
+// ------------------------------------------------------------------ forward
+template <typename T, int SUB, bool EDGE>
+__global__ void __launch_bounds__(kColThreads, bn_stats_blocks(sizeof(T), SUB))
+bn_column_stats_kernel(const T* __restrict__ x, ColumnShape sh, BnColumns bn, T* __restrict__ mn, T* __restrict__ mx,
+                       float2* __restrict__ partial) {
+  constexpr int NS = Slots<SUB>::N;
+  const int lane = threadIdx.x & 31;
+  const ColumnTask t = column_task(sh);
+  if (!t.valid) return;
+  const ColumnOctets<EDGE> oct(sh, t, lane);
+  const ColumnChannels<SUB> cc(sh, bn, t, lane);
+  float neg_shift[kBundle][NS];                        // shift: the channel's first element
+  float2 sum[kBundle][NS], sq[kBundle][NS];
+#pragma unroll
+  for (int gi = 0; gi < kBundle; ++gi) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      neg_shift[gi][s] = cc.ch[gi][s] < bn.C ? -load_scalar<T>(x, (int64_t)cc.ch[gi][s] * bn.HW) : 0.f;
+      sum[gi][s] = sq[gi][s] = both(0.f);
+    }
+  }
+  // the samples from the last to the first: the pack starts with what is read here last
+  Oct<T> next[kBundle];
+  oct.template load<T>(x + (int64_t)(t.n1 - 1) * sh.F, next);
+  for (int n = t.n1 - 1; n >= t.n0; --n) {
+    Oct<T> v[kBundle];
+#pragma unroll
+    for (int gi = 0; gi < kBundle; ++gi) v[gi] = next[gi];
+    if (n > t.n0) oct.template load<T>(x + (int64_t)(n - 1) * sh.F, next);
+    float lo = 0.f, hi = 0.f;
+    bundle_minmax<T>(v, lane, lo, hi);
+    if (lane < t.count) {
+      const int64_t q = (int64_t)n * sh.G + t.g0 + lane;
+      store_scalar<T>(mn, q, lo);
+      store_scalar<T>(mx, q, hi);
+    }
+#pragma unroll
+    for (int gi = 0; gi < kBundle; ++gi) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if constexpr (SUB != 1) {
+          const int s = SUB == 8 ? 0 : k / 2;
+          const float2 d = octet_pair_plus<T>(v[gi], k, neg_shift[gi][s], neg_shift[gi][s]);
+          sum[gi][s] = add2(sum[gi][s], d);
+          sq[gi][s] = fma2(d, d, sq[gi][s]);
+        } else {
+          const bool s0 = cc.second(gi, 2 * k), s1 = cc.second(gi, 2 * k + 1);
+          const float2 d = octet_pair_plus<T>(v[gi], k, neg_shift[gi][s0 ? 1 : 0], neg_shift[gi][s1 ? 1 : 0]);
+          sum[gi][0].x += s0 ? 0.f : d.x; sum[gi][0].y += s1 ? 0.f : d.y;
+          sum[gi][1].x += s0 ? d.x : 0.f; sum[gi][1].y += s1 ? d.y : 0.f;
+          sq[gi][0].x += s0 ? 0.f : d.x * d.x; sq[gi][0].y += s1 ? 0.f : d.y * d.y;
+          sq[gi][1].x += s0 ? d.x * d.x : 0.f; sq[gi][1].y += s1 ? d.y * d.y : 0.f;
+        }
+      }
+    }
+  }
+  const int split = t.n0 / sh.spp;
+  write_partials<SUB>(cc, sum, sq, partial + ((int64_t)split * sh.P + t.p) * bn.kmax, lane);
+}
+
+// One warp per channel.
+template <typename T>
+__global__ void __launch_bounds__(kColThreads)
+bn_column_stats_finish_kernel(const float2* __restrict__ partial, ColumnShape sh, BnColumns bn, const T* __restrict__ x,
+                              float* __restrict__ running_mean, float* __restrict__ running_var,
+                              float* __restrict__ save_mean, float* __restrict__ save_invstd, float momentum,
+                              float eps) {
+  const int lane = threadIdx.x & 31;
+  const int c = (int)(blockIdx.x * (kColThreads / 32) + (threadIdx.x >> 5));
+  if (c >= bn.C) return;
+  const float2 tot = collect_partials(sh, bn, partial, c, lane);
+  if (lane != 0) return;
+  const float M = (float)sh.N * (float)bn.HW;
+  const float m_s = tot.x / M;
+  const float var = fmaxf(tot.y / M - m_s * m_s, 0.f);
+  const float mean = load_scalar<T>(x, (int64_t)c * bn.HW) + m_s;
+  const float invstd = 1.0f / sqrtf(var + eps);
+  save_mean[c] = mean;
+  save_invstd[c] = invstd;
+  if (running_mean) running_mean[c] = (1.f - momentum) * running_mean[c] + momentum * mean;
+  if (running_var) {
+    const float unbiased = M > 1.f ? var * (M / (M - 1.f)) : var;
+    running_var[c] = (1.f - momentum) * running_var[c] + momentum * unbiased;
+  }
+}
+
+template <typename T, typename ST, int SUB, bool PHILOX, bool EDGE>
+__global__ void __launch_bounds__(kColThreads, kBnBlocks)
+bn_column_pack_kernel(const T* __restrict__ x, ColumnShape sh, BnColumns bn, const T* __restrict__ mn,
+                      const T* __restrict__ mx, const int32_t* __restrict__ bits,
+                      const int64_t* __restrict__ word_offsets, int32_t* __restrict__ packed, ST* __restrict__ scale,
+                      ST* __restrict__ mn_out, const NoiseKey key, const float* __restrict__ mean,
+                      const float* __restrict__ invstd, const float* __restrict__ weight,
+                      const float* __restrict__ bias, T* __restrict__ y) {
+  constexpr int NS = Slots<SUB>::N;
+  const int lane = threadIdx.x & 31;
+  const ColumnTask t = column_task(sh);
+  if (!t.valid) return;
+  const ColumnOctets<EDGE> oct(sh, t, lane);
+  const ColumnChannels<SUB> cc(sh, bn, t, lane);
+  float neg_mean[kBundle][NS], slope[kBundle][NS], shift[kBundle][NS];
+#pragma unroll
+  for (int gi = 0; gi < kBundle; ++gi) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const int c = min(cc.ch[gi][s], bn.C - 1);       // elements past the sample are never stored
+      neg_mean[gi][s] = -__ldg(mean + c);
+      slope[gi][s] = __ldg(invstd + c) * (weight ? __ldg(weight + c) : 1.f);
+      shift[gi][s] = bias ? __ldg(bias + c) : 0.f;
+    }
+  }
+  pack_column<T, ST, PHILOX>(
+      x, sh, t, oct, mn, mx, bits, word_offsets, packed, scale, mn_out, (const T*)nullptr, key, lane,
+      [&](int n, const Oct<T> (&v)[kBundle]) {
+        T* sample = y + (int64_t)n * sh.F;
+#pragma unroll
+        for (int gi = 0; gi < kBundle; ++gi) {
+          Oct<T> r;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if constexpr (SUB != 1) {
+              const int s = SUB == 8 ? 0 : k / 2;
+              const float2 d = octet_pair_plus<T>(v[gi], k, neg_mean[gi][s], neg_mean[gi][s]);
+              set_octet_pair<T>(r, k, fma2(d, both(slope[gi][s]), both(shift[gi][s])));
+            } else {
+              const int a = cc.second(gi, 2 * k) ? 1 : 0, b = cc.second(gi, 2 * k + 1) ? 1 : 0;
+              const float2 d = octet_pair_plus<T>(v[gi], k, a ? neg_mean[gi][1] : neg_mean[gi][0], b ? neg_mean[gi][1] : neg_mean[gi][0]);
+              set_octet_pair<T>(r, k, make_float2(fmaf(d.x, a ? slope[gi][1] : slope[gi][0], a ? shift[gi][1] : shift[gi][0]),
+                                                  fmaf(d.y, b ? slope[gi][1] : slope[gi][0], b ? shift[gi][1] : shift[gi][0])));
+            }
+          }
+          oct.template store<T>(sample, gi, r);
+        }
+      });
+}
+
+// ------------------------------------------------------------------ backward
 // EDGE: samples that are not whole groups, or octets off their natural alignment.
 template <typename T, typename ST, int SUB, bool EDGE>
 __global__ void __launch_bounds__(kColThreads, kBnBlocks)
@@ -307,6 +456,61 @@ int64_t bn_partial_bytes(const ColumnShape& sh, const BnColumns& bn) {
 }
 int64_t bn_coef_bytes(int64_t C) { return (C * (int64_t)sizeof(float4) + 255) / 256 * 256; }
 
+ColumnShape bn_stats_shape(int64_t N, int64_t C, int64_t HW, int align, int elem_size) {
+  return column_shape(N, C * HW, align, bn_stats_blocks(elem_size, HW % 8 == 0 ? 8 : 4) * kColThreads / 32);
+}
+struct BnForward {
+  const void *group_mn, *group_mx;
+  unsigned* ticket;
+  const float *weight, *bias;
+  float *running_mean, *running_var, *save_mean, *save_invstd;
+  int32_t *packed, *bits;
+  void *scale, *mn_out;
+  int64_t* word_offsets;
+  float* C;
+  float momentum, eps, range_factor;
+  int initial_bits, stochastic;
+  double target;
+  uint64_t seed, offset;
+};
+int64_t bn_range_bytes(int64_t N, int64_t F, int elem_size) {
+  return (N * ((F + kGroup - 1) / kGroup) * elem_size + 255) / 256 * 256;
+}
+
+template <typename T, typename ST, int SUB, bool EDGE>
+int launch_forward(const void* x, void* y, const BnForward& f, const ColumnShape& stats, const ColumnShape& sh,
+                   const BnColumns& bn, void* workspace, cudaStream_t s) {
+  const T *mn = (const T*)f.group_mn, *mx = (const T*)f.group_mx;
+  if (!mn) {                                           // else ranges and statistics come from a pass before this call
+    float2* partial = (float2*)workspace;
+    T* own_mn = (T*)((char*)partial + bn_partial_bytes(stats, bn));
+    T* own_mx = (T*)((char*)own_mn + bn_range_bytes(sh.N, sh.F, sizeof(T)));
+    bn_column_stats_kernel<T, SUB, EDGE><<<column_grid(stats), kColThreads, 0, s>>>((const T*)x, stats, bn, own_mn, own_mx,
+                                                                                   partial);
+    if (int st = check_launch()) return st;
+    bn_column_stats_finish_kernel<T><<<(bn.C + kColThreads / 32 - 1) / (kColThreads / 32), kColThreads, 0, s>>>(
+        partial, stats, bn, (const T*)x, f.running_mean, f.running_var, f.save_mean, f.save_invstd, f.momentum, f.eps);
+    if (int st = check_launch()) return st;
+    mn = own_mn;
+    mx = own_mx;
+  }
+  if (range_greedy_supported(sh.N, f.initial_bits)) {
+    if (int st = range_greedy_impl(mn, mx, sh.N, sh.G, DType<T>::id, f.range_factor, 1.f, nullptr, f.C, f.ticket,
+                                   f.initial_bits, f.target, f.bits, f.word_offsets, kGroup, s))
+      return st;
+  } else {
+    if (int st = actnn_range_sqr(mn, mx, sh.N, sh.G, DType<T>::id, f.range_factor, 1.f, nullptr, f.C, s)) return st;
+    if (int st = actnn_calc_precision(f.C, nullptr, sh.N, f.initial_bits, f.target, f.bits, f.word_offsets, sh.G, kGroup,
+                                      nullptr, 0, s))
+      return st;
+  }
+  auto pack = f.stochastic ? bn_column_pack_kernel<T, ST, SUB, true, EDGE> : bn_column_pack_kernel<T, ST, SUB, false, EDGE>;
+  pack<<<column_grid(sh), kColThreads, 0, s>>>((const T*)x, sh, bn, mn, mx, f.bits, f.word_offsets, f.packed,
+                                               (ST*)f.scale, (ST*)f.mn_out, make_noise_key(f.seed, f.offset), f.save_mean,
+                                               f.save_invstd, f.weight, f.bias, (T*)y);
+  return check_launch();
+}
+
 template <typename T, typename ST, int SUB, bool EDGE>
 int launch_backward(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets, const void* scale,
                     const void* mn, const void* dy, const float* weight, const float* save_mean,
@@ -335,8 +539,66 @@ extern "C" int actnn_batch_norm_codes_workspace(int64_t N, int64_t C, int64_t HW
   if (dtype < ACTNN_F32 || dtype > ACTNN_BF16) return ACTNN_ERR_DTYPE;
   if (!bn_columns_supported(N, C, HW)) return ACTNN_ERR_SHAPE;
   const ColumnShape sh = column_shape(N, C * HW, kOct, kBnWarps);
-  *bytes = bn_coef_bytes(C) + bn_partial_bytes(sh, bn_columns(C, HW));
+  const BnColumns bn = bn_columns(C, HW);
+  const ColumnShape stats = bn_stats_shape(N, C, HW, kOct, dtype_size(dtype));
+  *bytes = bn_coef_bytes(C) + max(bn_partial_bytes(sh, bn), bn_partial_bytes(stats, bn)) +
+           2 * bn_range_bytes(N, C * HW, dtype_size(dtype));                       // ranges: forward only
   return ACTNN_OK;
+}
+
+extern "C" int actnn_batch_norm_codes_forward(const void* x, const void* group_mn, const void* group_mx,
+                                              const float* weight, const float* bias, float* running_mean, float* running_var,
+                                              void* y, float* save_mean,
+                                              float* save_invstd, int32_t* packed, void* scale, void* mn_out,
+                                              int32_t* bits_out, int64_t* word_offsets_out, float* C_out, int64_t N,
+                                              int64_t C, int64_t HW, double momentum, double eps, int dtype,
+                                              int stat_dtype, float range_factor, int initial_bits, double target,
+                                              int stochastic, uint64_t seed, uint64_t offset, void* ticket,
+                                              void* workspace, int64_t workspace_bytes, actnn_stream_t stream) {
+  if (dtype < ACTNN_F32 || dtype > ACTNN_BF16) return ACTNN_ERR_DTYPE;
+  if (stat_dtype != (dtype == ACTNN_F32 ? ACTNN_BF16 : dtype)) return ACTNN_ERR_DTYPE;
+  if (initial_bits < 1 || initial_bits > 8) return ACTNN_ERR_BITS;
+  if (!(target == target)) return ACTNN_ERR_ARG;
+  if (!bn_columns_supported(N, C, HW)) return ACTNN_ERR_SHAPE;
+  if (!x || !y || !save_mean || !save_invstd || !packed || !scale || !mn_out || !bits_out || !word_offsets_out ||
+      !C_out || !ticket || !workspace || (!group_mn != !group_mx))
+    return ACTNN_ERR_NULL;
+  const int es = dtype_size(dtype);
+  const int64_t F = C * HW;
+  // whole groups want vector alignment, as in the codec's own entries
+  if (!aligned(x, F % kGroup == 0 ? es * kOct : es) || !aligned(y, es) || !aligned(packed, 4) || !aligned(workspace, 256))
+    return ACTNN_ERR_ALIGN;
+  const int al = min(octet_alignment(x, F, es), octet_alignment(y, F, es));
+  const ColumnShape sh = column_shape(N, F, al, kBnWarps);
+  const BnColumns bn = bn_columns(C, HW);
+  const ColumnShape stats = bn_stats_shape(N, C, HW, al, es);
+  if (!group_mn && workspace_bytes < bn_partial_bytes(stats, bn) + 2 * bn_range_bytes(N, F, es))
+    return ACTNN_ERR_CAPACITY;
+  const BnForward f{group_mn, group_mx, (unsigned*)ticket, weight, bias, running_mean, running_var, save_mean, save_invstd, packed, bits_out, scale, mn_out,
+                    word_offsets_out, C_out, (float)momentum, (float)eps, range_factor, initial_bits, stochastic,
+                    target, seed, offset};
+  cudaStream_t s = (cudaStream_t)stream;
+  const bool edge = al != kOct || F % kGroup != 0;
+#define ACTNN_FWD(T, ST, SUB, EDGE) return launch_forward<T, ST, SUB, EDGE>(x, y, f, stats, sh, bn, workspace, s)
+#define ACTNN_FWD_T(T, ST)                                  \
+  {                                                         \
+    if (HW % 8 == 0) {                                      \
+      if (edge) ACTNN_FWD(T, ST, 8, true);                  \
+      ACTNN_FWD(T, ST, 8, false);                           \
+    }                                                       \
+    if (HW % 4 == 0) {                                      \
+      if (edge) ACTNN_FWD(T, ST, 4, true);                  \
+      ACTNN_FWD(T, ST, 4, false);                           \
+    }                                                       \
+    ACTNN_FWD(T, ST, 1, true);                              \
+  }
+  switch (dtype) {
+    case ACTNN_F16: ACTNN_FWD_T(__half, __half)
+    case ACTNN_BF16: ACTNN_FWD_T(__nv_bfloat16, __nv_bfloat16)
+    default: ACTNN_FWD_T(float, __nv_bfloat16)
+  }
+#undef ACTNN_FWD_T
+#undef ACTNN_FWD
 }
 
 extern "C" int actnn_batch_norm_codes_backward(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets,

@@ -224,6 +224,66 @@ ACTNN_DEV void pack_column_bundle(const Oct<T> (&x)[kBundle], const Oct<T> (&nz)
   }
 }
 
+// Scale, stochastic rounding and pack of a column; each(n, octets) sees every sample's octets on the way.  Eight samples at a time: lane 4i + g prepares group g of
+// the i-th of them (one division per lane for eight bundles).  The noise octets are formed before
+// the dispatch on the width, so the eight width variants stay short.
+template <typename T, typename ST, bool PHILOX, bool EDGE, typename Each>
+ACTNN_DEV void pack_column(const T* __restrict__ data, const ColumnShape& sh, const ColumnTask& t,
+                           const ColumnOctets<EDGE>& oct, const T* __restrict__ mn, const T* __restrict__ mx,
+                           const int32_t* __restrict__ bits, const int64_t* __restrict__ word_offsets,
+                           int32_t* __restrict__ packed, ST* __restrict__ scale, ST* __restrict__ mn_out,
+                           const T* __restrict__ noise, const NoiseKey& key, int lane, Each each) {
+  const TransposePlan plan = make_transpose_plan(lane);
+  Oct<T> next[kBundle];
+  oct.template load<T>(data + (int64_t)t.n0 * sh.F, next);
+  for (int nb = t.n0; nb < t.n1; nb += 8) {
+    const int n_l = nb + (lane >> 2), g_l = lane & 3;
+    int b_l = 0;
+    int64_t off_l = 0;
+    LaneParams<T> mine = {0u, 0u};
+    if (n_l < t.n1 && g_l < t.count) {
+      b_l = __ldg(bits + n_l);
+      if (b_l < 1 || b_l > 8) b_l = 0;                   // not a width: nothing written
+      off_l = __ldg(word_offsets + n_l) + (int64_t)t.g0 * 8 * b_l;
+      const int64_t q = (int64_t)n_l * sh.G + t.g0 + g_l;
+      const float gmn = load_scalar<T>(mn, q), gmx = load_scalar<T>(mx, q);
+      const GroupParams gp = prepare_group<T>(gmn, gmx, b_l);
+      store_scalar<ST>(scale, q, gp.scale);
+      store_scalar<ST>(mn_out, q, gmn);
+      mine = lane_params<T>(gp);
+    }
+    const int cnt = min(8, t.n1 - nb);
+    for (int i = 0; i < cnt; ++i) {
+      const int n = nb + i;
+      Oct<T> x[kBundle], nz[kBundle];
+#pragma unroll
+      for (int gi = 0; gi < kBundle; ++gi) x[gi] = next[gi];
+      if (n + 1 < t.n1) oct.template load<T>(data + (int64_t)(n + 1) * sh.F, next);
+      const int64_t q0 = (int64_t)n * sh.G + t.g0;
+      if constexpr (PHILOX) {
+        noise_bundle<T>(key, q0, lane, nz);
+      } else {                                           // an injected tensor shaped [N, G, 256], or none
+#pragma unroll
+        for (int gi = 0; gi < kBundle; ++gi)
+          nz[gi] = noise && gi < t.count ? load_oct<T>(noise + (q0 + gi) * kGroup + lane * kOct) : zero_oct<T>();
+      }
+      each(n, x);
+      const int b = __shfl_sync(kFull, b_l, 4 * i);
+      const uint32_t olo = __shfl_sync(kFull, (uint32_t)off_l, 4 * i);
+      const uint32_t ohi = __shfl_sync(kFull, (uint32_t)((uint64_t)off_l >> 32), 4 * i);
+      int32_t* out = packed + (int64_t)(((uint64_t)ohi << 32) | olo);
+#define ACTNN_CASE(B) \
+      case B: pack_column_bundle<T, B>(x, nz, mine, 4 * i, t.count, out, plan, lane); break;
+      switch (b) {
+        ACTNN_CASE(1) ACTNN_CASE(2) ACTNN_CASE(3) ACTNN_CASE(4) ACTNN_CASE(5) ACTNN_CASE(6) ACTNN_CASE(7)
+        ACTNN_CASE(8)
+        default: break;
+      }
+#undef ACTNN_CASE
+    }
+  }
+}
+
 // ------------------------------------------------------------------ the stream of a column, read ahead
 // Of a block of 32 samples, lane l knows the width and the stream position of the l-th; the first words
 // and the statistics (lane gi < 4: group gi) of one bundle are requested a sample ahead of their use.

@@ -28,6 +28,7 @@ from .conf import config
 from .cpp_extension import backward_func as ext_backward_func
 from .cpp_extension import minimax as ext_minimax  # noqa: F401  (kept under the name the reference imports)
 from .cpp_extension import quantization as ext_quantization
+from .qbnscheme import QBNScheme
 from .qscheme import group_minimax, to_groups
 from .utils import compute_tensor_bytes, empty_cache, get_memory_usage, swap_to_cpu, swap_to_gpu
 
@@ -428,12 +429,21 @@ class batch_norm(Function):
     @staticmethod
     def forward(ctx, input, running_mean, running_var, weight, bias, training, exponential_average_factor, eps,
                 scheme):
-        fused = None
+        fused = whole = None
         if training and input.is_cuda:
             input = input.contiguous()
             fused = _fused_bn_statistics(input, scheme, weight, bias, running_mean, running_var,
                                          exponential_average_factor, eps)
-        if fused is not None:
+            if config.compress_activation and config.pergroup and not config.simulate and config.group_size == 256 \
+                    and getattr(type(scheme), "compress", None) is QBNScheme.compress:
+                # codes and output from one read of the input (and the statistics from another, if not there yet)
+                whole = scheme.batch_norm(input, weight, bias, running_mean, running_var, exponential_average_factor,
+                                          eps, fused)
+        if whole is not None:
+            output, quantized, save_mean, save_var = whole
+            if config.swap:
+                quantized = (swap_to_cpu(quantized[0]),) + tuple(quantized[1:])
+        elif fused is not None:
             # one read of the input gave the statistics and the group ranges; the second read
             # packs, the third normalises (the reference reads it four times)
             mn, mx, save_mean, save_var = fused
@@ -449,7 +459,9 @@ class batch_norm(Function):
             total_act_mem += compute_tensor_bytes([t for t in quantized if isinstance(t, torch.Tensor)])
             print("Act mem: %.2f MB" % (total_act_mem / 1024 ** 2))
 
-        if fused is not None:
+        if whole is not None:
+            reserve = None
+        elif fused is not None:
             output = ext_backward_func.batch_norm_elemt(input, weight, bias, save_mean, save_var, eps)
             reserve = torch.empty(0, dtype=torch.uint8, device=input.device)
         elif training:

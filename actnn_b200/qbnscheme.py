@@ -1,6 +1,7 @@
 """Quantization scheme for batch-norm inputs: sensitivity = range only, bits follow the
 preceding conv / linear layer (mirror of actnn/actnn/qbnscheme.py:9-60)."""
 from .conf import config
+from .cpp_extension import backward_func as ext_backward_func
 from .cpp_extension import calc_precision as ext_calc_precision
 from .qscheme import QScheme, compress_groups, group_minimax, total_bits_after_greedy
 
@@ -40,6 +41,20 @@ class QBNScheme(QScheme):
             input, int(self.bits * N), int(self.initial_bits), config.group_size / num_pixels,
             1.0, None, config.stochastic, stat_dtype=stat_dtype, minmax=minmax)
         return q_input, b, q_scale, q_min
+
+    def batch_norm(self, input, weight, bias, running_mean, running_var, momentum, eps, stats=None):
+        """Normalise ``input`` and compress it as ``compress`` does, from two reads of it; ``None`` when
+        that does not apply (see ``backward_func.batch_norm_codes_forward``)."""
+        N, D = input.shape[0], input.shape[1]
+        num_pixels = (input.numel() // max(N, 1)) // max(D, 1)
+        if num_pixels == 0:
+            return None
+        out = ext_backward_func.batch_norm_codes_forward(
+            input, weight, bias, running_mean, running_var, momentum, eps, int(self.bits * N), int(self.initial_bits),
+            config.group_size / num_pixels, config.stochastic, stats)
+        if out is not None:
+            self.prev_linear = QScheme.prev_layer
+        return out
 
     @staticmethod
     def allocate_perlayer():

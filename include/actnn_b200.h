@@ -272,6 +272,19 @@ int actnn_transpose16(const void* in, void* out, int64_t batch, int64_t rows, in
  * Any C, HW >= 8.  grad_out / grad_in need the alignment of one element.  Scratch: *bytes of the first call (a host
  * pointer; ACTNN_ERR_SHAPE: not covered), 16-byte aligned, for the current device. */
 int actnn_batch_norm_codes_workspace(int64_t N, int64_t C, int64_t HW, int dtype, int64_t* bytes);
+/* The forward half: statistics, widths, codes and y = normalised x from two reads of x.  Replaces the compress of the
+ * input followed by the batch norm, actnn/actnn/ops.py:446-458 and qbnscheme.py:28-52.  Outputs as in
+ * actnn_compress_mixed_samples (coeff 1, no grad_scale, no injected noise) and actnn_batch_norm_forward; same
+ * geometry and scratch as the backward half, the scratch 256-byte aligned.  With group_mn / group_mx (what
+ * actnn_batch_norm_stats_minimax wrote; else both NULL) save_mean and save_invstd are inputs, too, and the running
+ * statistics are left alone.  `ticket`: as in actnn_compress_mixed_prestat_kept. */
+int actnn_batch_norm_codes_forward(const void* x, const void* group_mn, const void* group_mx, const float* weight,
+                                   const float* bias, float* running_mean, float* running_var, void* y, float* save_mean, float* save_invstd, int32_t* packed,
+                                   void* scale, void* mn_out, int32_t* bits_out, int64_t* word_offsets_out,
+                                   float* C_out, int64_t N, int64_t C, int64_t HW, double momentum, double eps,
+                                   int dtype, int stat_dtype, float range_factor, int initial_bits, double target,
+                                   int stochastic, uint64_t seed, uint64_t offset, void* ticket, void* workspace,
+                                   int64_t workspace_bytes, actnn_stream_t stream);
 int actnn_batch_norm_codes_backward(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets,
                                     const void* scale, const void* mn, const void* grad_out, const float* weight,
                                     const float* save_mean, const float* save_invstd, void* grad_in,

@@ -58,6 +58,45 @@ def test_backward_from_codes(shape, dtype, offset):
     assert ((dx.double() - rx).abs() <= (EPS[dtype] * 1.01 + 64 * 2 ** -24) * big + 1e-7).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", SHAPES + [(1030, 8, 16)])
+@pytest.mark.parametrize("stochastic", [True, False])
+def test_forward(shape, dtype, stochastic, monkeypatch):
+    from actnn_b200 import _lib
+    from actnn_b200.cpp_extension import backward_func as bf
+    from actnn_b200.cpp_extension import quantization as q
+    n, c, hw = shape
+    torch.manual_seed(1)
+    x = (torch.randn(n, c, hw, device="cuda") * 1.5 + torch.linspace(-8, 8, c, device="cuda").view(1, c, 1)).to(dtype)
+    weight, bias = torch.rand(c, device="cuda") + 0.5, torch.randn(c, device="cuda")
+    rm, rv = torch.randn(c, device="cuda"), torch.rand(c, device="cuda")
+    rm0, rv0 = rm.double(), rv.double()
+    monkeypatch.setattr(_lib, "next_philox", lambda dev: (9, 4))
+    y, quantized, mean, invstd = bf.batch_norm_codes_forward(x, weight, bias, rm, rv, 0.1, 1e-5, 2 * n, 8, 0.5, stochastic)
+    f = c * hw
+    stat = torch.bfloat16 if dtype == torch.float32 else dtype
+    kw = dict(philox=(9, 4), stat_dtype=stat) if stochastic else dict(stochastic=False, stat_dtype=stat)
+    if f % 256:
+        ref = q.compress_mixed_samples(x.view(n, f), 2 * n, 8, 0.5, **kw)
+    else:
+        ref = q.compress_mixed_precision(x.view(n, f // 256, 256), 2 * n, 8, 0.5, **kw)
+    assert all(torch.equal(a, b) for a, b in zip(quantized, ref))          # the codec to the bit
+    xd = x.double()
+    m, v = xd.mean((0, 2)), xd.var((0, 2), unbiased=False)
+    i = 1 / torch.sqrt(v + 1e-5)
+    # shifted float32 sums: 64 roundings of sums of |x - shift| and its square, shift within 4 deviations of the mean
+    dev = torch.sqrt(v) + 1e-3
+    assert ((mean.double() - m).abs() <= 64 * 2 ** -24 * (5 * dev + m.abs())).all()
+    assert ((invstd.double() / i - 1).abs() <= 64 * 2 ** -24 * 25).all()
+    cnt = n * hw
+    assert torch.allclose(rm.double(), 0.9 * rm0 + 0.1 * m, rtol=1e-5, atol=1e-5)
+    assert torch.allclose(rv.double(), 0.9 * rv0 + 0.1 * v * (cnt / (cnt - 1)), rtol=1e-4, atol=1e-6)
+    ry = (xd - m.view(1, -1, 1)) * (i * weight.double()).view(1, -1, 1) + bias.double().view(1, -1, 1)
+    big = ry.abs() + (xd - m.view(1, -1, 1)).abs() * (i * weight.double()).view(1, -1, 1) + bias.double().abs().view(1, -1, 1) \
+        + (m.abs() * i * weight.double()).view(1, -1, 1)
+    assert ((y.double() - ry).abs() <= (EPS[dtype] * 1.01 + 2048 * 2 ** -24) * big).all()
+
+
 def test_layer_backward_takes_the_codes_and_agrees_with_the_decoded_path(monkeypatch):
     import actnn_b200 as actnn
     from actnn_b200.cpp_extension import backward_func as bf
