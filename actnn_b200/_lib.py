@@ -147,6 +147,29 @@ def _fast_module():
     return _fast
 
 
+_native = None
+NATIVE_PATH = os.path.join(_HERE, "csrc", "_actnn_native.so")
+
+
+def native():
+    """The C++ half of the binding (csrc/native.cpp); ``False`` when another build of the library was
+    requested, to which it is not linked (the Python functions then make the calls one by one)."""
+    global _native
+    if _native is None:
+        if os.environ.get("ACTNN_B200_LIB"):
+            _native = False
+        else:
+            import importlib.util
+            load()
+            if not os.path.exists(NATIVE_PATH):
+                raise RuntimeError("actnn_b200: %s is missing. Build it with `python -m actnn_b200.csrc.build`." % NATIVE_PATH)
+            spec = importlib.util.spec_from_file_location("_actnn_native", NATIVE_PATH)
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            _native = mod
+    return _native
+
+
 def call(name: str, tensor_for_device: torch.Tensor, *args) -> None:
     """Invoke ``name`` with the tensor's device current and check the status."""
     fn = _fns.get(name)

@@ -84,6 +84,9 @@ def channels_last_pays(input, weight, groups) -> bool:
 
 def to_channels_last(x):
     """A channels-last copy of a contiguous 16-bit NCHW tensor."""
+    nat = _lib.native()
+    if nat:
+        return nat.transpose16(x, True)
     n, c, h, w = x.shape
     out = torch.empty(x.shape, dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
     _lib.call("actnn_transpose16", x, x.data_ptr(), out.data_ptr(), n, c, h * w, _lib.stream_of(x))
@@ -94,6 +97,9 @@ def to_planes(x):
     """The contiguous NCHW form of a 16-bit tensor that came back channels-last."""
     if x.is_contiguous() or not x.is_contiguous(memory_format=torch.channels_last):
         return x.contiguous()
+    nat = _lib.native()
+    if nat:
+        return nat.transpose16(x, False)
     n, c, h, w = x.shape
     out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
     _lib.call("actnn_transpose16", x, x.data_ptr(), out.data_ptr(), n, h * w, c, _lib.stream_of(x))
@@ -190,6 +196,17 @@ def batch_norm_codes_forward(x, weight, bias, running_mean, running_var, momentu
     for t in (running_mean, running_var):
         if t is not None and (t.dtype != torch.float32 or not t.is_contiguous()):
             return None
+    nat = _lib.native()
+    if nat:
+        out = nat.batch_norm_forward(x, weight, bias, running_mean, running_var, momentum, eps, int(target_bits),
+                                     initial_bits, range_factor, bool(stochastic), *(stats or (None,) * 4),
+                                     _lib.ticket(x.device))
+        if out is None:
+            return None
+        y, packed, bits, scale, mn, mean, invstd, offsets = out
+        packed.word_offsets = bits.word_offsets = offsets
+        bits.total_bits = min(initial_bits * x.shape[0], max(int(target_bits), x.shape[0]))
+        return y, (packed, bits, scale, mn), mean, invstd
     N, C, HW = _bn_dims(x)
     dev, dt = x.device, _lib.dtype_id(x.dtype)
     nbytes = _codes_workspace(N, C, HW, dt, dev.index)
@@ -242,6 +259,16 @@ def batch_norm_codes_backward(quantized, shape, dtype, grad_output, weight, save
     if N * F == 0 or tuple(scale.shape) != (N, (F + 255) // 256, 1) or bits.numel() != N:
         return None
     HW = F // C
+    word_offsets = getattr(packed, "word_offsets", None)
+    if word_offsets is None:
+        word_offsets = quantization.bits_prefix(bits, scale.shape[1], 256)
+    nat = _lib.native()
+    if nat:
+        out = nat.batch_norm_backward(packed, bits, word_offsets, scale, mn, shape, grad_output,
+                                      dtype == torch.float32, weight, save_mean, save_invstd)
+        if out is not None and weight is not None and weight.dtype != torch.float32:
+            out = out[0], out[1].to(weight.dtype), out[2].to(weight.dtype)
+        return out
     dt = _lib.dtype_id(dtype)
     nbytes = _codes_workspace(N, C, HW, dt, packed.device.index)
     if nbytes is None:
@@ -249,9 +276,6 @@ def batch_norm_codes_backward(quantized, shape, dtype, grad_output, weight, save
     dy = grad_output.contiguous()
     if dy.dtype != dtype:
         dy = dy.to(dtype)
-    word_offsets = getattr(packed, "word_offsets", None)
-    if word_offsets is None:
-        word_offsets = quantization.bits_prefix(bits, scale.shape[1], 256)
     w32 = _as_f32(weight)
     dx = torch.empty(shape, dtype=dtype, device=packed.device)
     dweight = torch.empty(C, dtype=torch.float32, device=packed.device)

@@ -81,6 +81,9 @@ def sample_sumsq(grad: torch.Tensor) -> torch.Tensor:
     read of ``grad``: float32 ``[N]``."""
     if not grad.is_cuda or grad.dtype not in (torch.float32, torch.float16, torch.bfloat16):
         raise RuntimeError("grad must be a floating-point CUDA tensor!")
+    nat = _lib.native()
+    if nat:
+        return nat.sample_sumsq(grad)
     grad = grad.contiguous()
     n = grad.shape[0]
     out = torch.empty(n, dtype=torch.float32, device=grad.device)

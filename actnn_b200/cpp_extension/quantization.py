@@ -138,26 +138,35 @@ def _compress_mixed(data, n, g, gs, features, target_bits, initial_bits, range_f
     sdt = _stat_dtype(data.dtype, stat_dtype)
     total = min(initial_bits * n, max(int(target_bits), n))        # what the greedy ends with
     dev = data.device
+    gmn, gmx = minmax if minmax is not None else (None, None)
+    if minmax is not None:
+        check_cuda_tensor(gmn, "min", dtype=data.dtype)
+        check_cuda_tensor(gmx, "max", dtype=data.dtype)
+        if gmn.numel() != n * g or gmx.numel() != n * g:
+            raise RuntimeError("min / max must have one element per group!")
+    if grad_scale is not None and (grad_scale.dtype != torch.float32 or not grad_scale.is_cuda
+                                   or grad_scale.numel() != 1):
+        raise RuntimeError("grad_scale must be a float32 CUDA tensor with one element!")
+    nat = _lib.native() if noise is None and philox is None else None
+    if nat:
+        packed, bits, scale, mn, C, offsets = nat.compress_mixed(
+            data, n, g, gs, -1 if features is None else features, target_bits, initial_bits, range_factor, coeff,
+            grad_scale, bool(stochastic), sdt != data.dtype, gmn, gmx, None if minmax is None else _lib.ticket(dev))
+        packed.word_offsets = bits.word_offsets = offsets
+        bits.total_bits = total
+        return packed, bits, scale, mn, C
     packed = torch.empty((total * g * gs + 31) // 32, dtype=torch.int32, device=dev)
     scale = torch.empty((n, g, 1), dtype=sdt, device=dev)
     mn = torch.empty((n, g, 1), dtype=sdt, device=dev)
     bits = torch.empty(n, dtype=torch.int32, device=dev)
     offsets = torch.empty(n + 1, dtype=torch.int64, device=dev)
     C = torch.empty(n, dtype=torch.float32, device=dev)
-    if grad_scale is not None and (grad_scale.dtype != torch.float32 or not grad_scale.is_cuda
-                                   or grad_scale.numel() != 1):
-        raise RuntimeError("grad_scale must be a float32 CUDA tensor with one element!")
     if features is not None and noise is not None and stochastic:
         check_cuda_tensor(noise, "noise", dtype=data.dtype)
         nz, seed, offset = noise.data_ptr(), 0, 0
     else:
         nz, seed, offset = _noise_args(data, stochastic, noise, philox)
     if minmax is not None:
-        gmn, gmx = minmax
-        check_cuda_tensor(gmn, "min", dtype=data.dtype)
-        check_cuda_tensor(gmx, "max", dtype=data.dtype)
-        if gmn.numel() != n * g or gmx.numel() != n * g:
-            raise RuntimeError("min / max must have one element per group!")
         workspace = _lib.ticket(dev)
         _lib.call("actnn_compress_mixed_prestat_kept", data, data.data_ptr(), gmn.data_ptr(), gmx.data_ptr(),
                   packed.data_ptr(), scale.data_ptr(), mn.data_ptr(), bits.data_ptr(), offsets.data_ptr(),
@@ -198,6 +207,10 @@ def unpack_mixed_precision(data, bits, scale, min, N, num_groups, group_size, *,
         word_offsets = getattr(data, "word_offsets", None)
     if word_offsets is None:
         word_offsets = bits_prefix(bits, num_groups, group_size)
+    nat = _lib.native()
+    if nat:
+        return nat.unpack_mixed(data, bits, word_offsets, scale, min, (N, num_groups, group_size), N, num_groups,
+                                group_size, -1, scale, out_dtype == torch.float32)
     out = torch.empty((N, num_groups, group_size), dtype=out_dtype, device=data.device)
     _lib.call("actnn_unpack_mixed", data, data.data_ptr(), bits.data_ptr(), word_offsets.data_ptr(),
               scale.data_ptr(), min.data_ptr(), out.data_ptr(), N, num_groups, group_size,
@@ -218,11 +231,18 @@ def unpack_mixed_samples(data, bits, scale, min, shape, *, out_dtype=None):
     word_offsets = getattr(data, "word_offsets", None)
     if word_offsets is None:
         word_offsets = bits_prefix(bits, g, 256)
-    out = torch.empty(shape, dtype=out_dtype, device=data.device)
-    if out.shape[0] != n or bits.numel() != n or (out.numel() // n + 255) // 256 != g:
+    features = 1
+    for d in shape[1:]:
+        features *= d
+    if shape[0] != n or bits.numel() != n or (features + 255) // 256 != g:
         raise RuntimeError("unpack_mixed_samples: the statistics do not belong to a tensor of this shape")
+    nat = _lib.native()
+    if nat:
+        return nat.unpack_mixed(data, bits, word_offsets, scale, min, shape, n, g, 256, features, scale,
+                                out_dtype == torch.float32)
+    out = torch.empty(shape, dtype=out_dtype, device=data.device)
     _lib.call("actnn_unpack_mixed_samples", data, data.data_ptr(), bits.data_ptr(), word_offsets.data_ptr(),
-              scale.data_ptr(), min.data_ptr(), out.data_ptr(), n, out.numel() // n, _lib.dtype_id(out_dtype),
+              scale.data_ptr(), min.data_ptr(), out.data_ptr(), n, features, _lib.dtype_id(out_dtype),
               _lib.dtype_id(scale.dtype), _lib.stream_of(data))
     return out
 
@@ -272,6 +292,11 @@ def compress_single_precision(data, bits, stochastic=True, *, noise=None, philox
     n, g, gs = data.shape
     _check_group_size(gs)
     sdt = _stat_dtype(data.dtype, stat_dtype)
+    nat = _lib.native() if noise is None and philox is None and not return_max else None
+    if nat:
+        out = nat.compress_single(data, bits, bool(stochastic), sdt != data.dtype, single_precision_bytes(bits, n, g, gs))
+        _lib.check_staged_pack(data, "actnn_compress_single")
+        return out
     packed = torch.empty(single_precision_bytes(bits, n, g, gs), dtype=torch.int8, device=data.device)
     scale = torch.empty((n, g, 1), dtype=sdt, device=data.device)
     mn = torch.empty((n, g, 1), dtype=sdt, device=data.device)
@@ -367,7 +392,8 @@ class _ActQuantizedReLUMinmax(torch.autograd.Function):
 
 def act_quantized_relu(input: torch.Tensor) -> torch.Tensor:
     check_cuda_tensor(input, "input")
-    return _ActQuantizedReLU.apply(input)
+    nat = _lib.native()
+    return nat.relu(input) if nat else _ActQuantizedReLU.apply(input)
 
 
 def act_quantized_relu_with_minmax(input: torch.Tensor, group_size: int = 256):
@@ -378,8 +404,9 @@ def act_quantized_relu_with_minmax(input: torch.Tensor, group_size: int = 256):
     check_cuda_tensor(input, "input")
     n = input.shape[0] if input.dim() > 1 else 1
     if group_size != 256 or n == 0 or (input.numel() // n) % 256 != 0 or not input.is_contiguous():
-        return _ActQuantizedReLU.apply(input)
-    y, mn, mx = _ActQuantizedReLUMinmax.apply(input)
+        return act_quantized_relu(input)
+    nat = _lib.native()
+    y, mn, mx = nat.relu_minmax(input) if nat else _ActQuantizedReLUMinmax.apply(input)
     y.actnn_minmax = (mn, mx, y._version)
     return y
 
@@ -429,7 +456,8 @@ class _ActQuantizedDropout(torch.autograd.Function):
 
 def act_quantized_dropout(input: torch.Tensor, dropout_p: float) -> torch.Tensor:
     check_cuda_tensor(input, "input")
-    return _ActQuantizedDropout.apply(input, float(dropout_p))
+    nat = _lib.native()
+    return nat.dropout(input, float(dropout_p)) if nat else _ActQuantizedDropout.apply(input, float(dropout_p))
 
 
 # ------------------------------------------------------------------------------- max-pool
@@ -491,5 +519,13 @@ def act_quantized_max_pool2d(input: torch.Tensor, kernel_size: Sequence[int], st
         raise RuntimeError("Do not support ceil_mode")
     if return_indices:
         raise RuntimeError("Do not support return_indices")
+    nat = _lib.native()
+    if nat:
+        geom = _pool_args(kernel_size, stride, padding, dilation)
+        if geom[0] * geom[1] >= 16:
+            raise RuntimeError("Expected kernel_size[0] * kernel_size[1] < 16 to be true, but got false.")
+        if input.dim() != 4:
+            raise RuntimeError("The dimension of input is not correct!")
+        return nat.max_pool2d(input, geom)
     return _ActQuantizedMaxPool2d.apply(input, tuple(kernel_size), tuple(stride), tuple(padding),
                                         tuple(dilation))

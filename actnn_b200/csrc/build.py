@@ -2,8 +2,8 @@
 
     python -m actnn_b200.csrc.build          (or: python actnn_b200/csrc/build.py)
 
-No torch headers are involved: the library is plain CUDA behind a C ABI
-(``include/actnn_b200.h``).  Objects are compiled in parallel and cached by mtime.
+The library is plain CUDA behind a C ABI (``include/actnn_b200.h``), no torch headers involved; the
+binding's C++ half (``native.cpp``) is built beside it.  Objects are compiled in parallel and cached by mtime.
 """
 from __future__ import annotations
 
@@ -56,6 +56,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         run([NVCC, "-shared", "-o", LIB] + objs + ["-gencode", "arch=compute_100a,code=sm_100a",
                                                    "-cudart", "shared"])
     build_fastcall(force)
+    build_native(force)
     return LIB
 
 
@@ -119,6 +120,36 @@ def build_fastcall(force: bool = False) -> str:
         if r.returncode != 0:
             raise RuntimeError("gcc failed: %s\n%s\n%s" % (" ".join(cmd), r.stdout, r.stderr))
     return FAST_LIB
+
+
+# ---------------------------------------------------------------------------------------
+# The host side of the hot entry points (native.cpp): the only source that needs torch's headers.
+# ---------------------------------------------------------------------------------------
+NATIVE_SRC = os.path.join(HERE, "native.cpp")
+NATIVE_LIB = os.path.join(HERE, "_actnn_native.so")
+
+
+def build_native(force: bool = False) -> str:
+    if not force and not _stale(NATIVE_LIB, [NATIVE_SRC, os.path.join(HERE, HEADERS[-1]), os.path.abspath(__file__)]):
+        return NATIVE_LIB
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as ext
+    # the system compiler, whatever CXX says: the module must share libstdc++.so.6 with torch, and a compiler that
+    # links its own copy statically makes a module that crashes when a number is formatted
+    cmd = ["/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++", "-O2", "-std=c++17", "-shared", "-fPIC", NATIVE_SRC, "-o", NATIVE_LIB,
+           "-DTORCH_EXTENSION_NAME=_actnn_native", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           "-I" + sysconfig.get_paths()["include"], "-I/usr/local/cuda/include"]
+    cmd += ["-isystem" + d for d in ext.include_paths()]
+    libdir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd += ["-L" + libdir, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+            "-L" + HERE, "-lactnn_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed: %s\n%s\n%s" % (" ".join(cmd), r.stdout, r.stderr))
+    return NATIVE_LIB
 
 
 if __name__ == "__main__":

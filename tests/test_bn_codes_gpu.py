@@ -61,8 +61,7 @@ def test_backward_from_codes(shape, dtype, offset):
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("shape", SHAPES + [(1030, 8, 16)])
 @pytest.mark.parametrize("stochastic", [True, False])
-def test_forward(shape, dtype, stochastic, monkeypatch):
-    from actnn_b200 import _lib
+def test_forward(shape, dtype, stochastic):
     from actnn_b200.cpp_extension import backward_func as bf
     from actnn_b200.cpp_extension import quantization as q
     n, c, hw = shape
@@ -71,7 +70,9 @@ def test_forward(shape, dtype, stochastic, monkeypatch):
     weight, bias = torch.rand(c, device="cuda") + 0.5, torch.randn(c, device="cuda")
     rm, rv = torch.randn(c, device="cuda"), torch.rand(c, device="cuda")
     rm0, rv0 = rm.double(), rv.double()
-    monkeypatch.setattr(_lib, "next_philox", lambda dev: (9, 4))
+    gen = torch.cuda.default_generators[torch.cuda.current_device()]
+    gen.manual_seed(9)
+    gen.set_offset(4)
     y, quantized, mean, invstd = bf.batch_norm_codes_forward(x, weight, bias, rm, rv, 0.1, 1e-5, 2 * n, 8, 0.5, stochastic)
     f = c * hw
     stat = torch.bfloat16 if dtype == torch.float32 else dtype
