@@ -249,10 +249,15 @@ pack_single_kernel(const T* __restrict__ data, const T* __restrict__ mn, const T
   }
 }
 
-// Unpack: a warp owns (sample block, group).  Lane t reads its eight bytes once; the table
-// of all wpt samples x 2^BITS codes is computed by the first wpt * 2^BITS lanes together
-// (one IEEE division per lane), and for 16-bit outputs with BITS <= 2 a byte-permute
-// selects two decoded elements per instruction.
+// Unpack: a warp owns (sample block, four neighbouring groups; two for float32).  Lane t reads its eight bytes of each group
+// once; the table of all wpt samples x 2^BITS codes of a group is computed by the first wpt * 2^BITS lanes
+// together (one IEEE division per lane), and for 16-bit outputs with BITS <= 2 a byte-permute selects two
+// decoded elements per instruction.
+// Bound by instruction issue: with one group per task, two tasks requested ahead, a lane spent 107 instructions on an
+// octet, most of them not on its elements (4 bits, 256 x 256 x 28 x 28 float16: 28.1 us).  Four groups share the
+// task's index arithmetic and addresses and are requested together: 21.7 us (two groups: 23.7). float32, whose octets
+// are twice as large, 2 bits, 64 x 64 x 56 x 56: one group 9.9, two 9.6, four 10.4 us.
+template <typename T> constexpr int unpack_groups() { return sizeof(T) == 2 ? 4 : 2; }
 template <typename T, typename ST, int BITS>
 __global__ void __launch_bounds__(kThreads, 4)
 unpack_single_kernel(const int8_t* __restrict__ packed, const ST* __restrict__ scale,
@@ -260,54 +265,38 @@ unpack_single_kernel(const int8_t* __restrict__ packed, const ST* __restrict__ s
   constexpr int WPT = 8 / BITS;
   constexpr int E = 1 << BITS;
   constexpr bool TABLE = BITS <= 4;                        // BITS == 8: divide per element
+  constexpr int kGroups = unpack_groups<T>();
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
   const int64_t nblocks = (N + WPT - 1) / WPT;
-
-  // The packed stream is an eighth of the output or less, so a task's loads are small; to
-  // keep enough bytes in flight each warp issues the loads of DEPTH tasks before it decodes
-  // the first of them.
-  constexpr int DEPTH = 2;
   const int my_s = TABLE ? lane / E : lane;                // lane l serves sample no*wpt + my_s
-  PairWalker walk(warp, nwarps, nblocks, G);
-  while (walk.valid()) {
-    int64_t t_no[DEPTH], t_g[DEPTH];
-    uint2 t_w[DEPTH];
-    float t_sc[DEPTH], t_m[DEPTH];
-    bool t_ok[DEPTH];
+  for (PairWalker walk(warp, nwarps, nblocks, (G + kGroups - 1) / kGroups); walk.valid(); walk.next()) {
+    const int64_t g0 = (int64_t)walk.r * kGroups, n0 = walk.no * WPT;
+    const int cnt = (int)min((int64_t)kGroups, G - g0);
+    const int8_t* in = packed + ((walk.no * G + g0) * kGroup + lane * kOct);
+    const bool mine = my_s < WPT && n0 + my_s < N;
+    const int64_t q = (n0 + my_s) * G + g0;
+    uint2 w[kGroups];
+    float sc[kGroups], m[kGroups];
 #pragma unroll
-    for (int d = 0; d < DEPTH; ++d) {
-      t_ok[d] = walk.valid();
-      t_no[d] = walk.no;
-      t_g[d] = walk.r;
-      t_w[d] = make_uint2(0u, 0u);
-      t_sc[d] = 1.f;
-      t_m[d] = 0.f;
-      if (t_ok[d]) {
-        t_w[d] = __ldg(reinterpret_cast<const uint2*>(packed + ((t_no[d] * G + t_g[d]) * kGroup + lane * kOct)));
-        const int64_t my_n = t_no[d] * WPT + my_s;
-        if (my_s < WPT && my_n < N) {
-          t_sc[d] = load_scalar<ST>(scale, my_n * G + t_g[d]);
-          t_m[d] = load_scalar<ST>(mn, my_n * G + t_g[d]);
-        }
-        walk.next();
-      }
+    for (int gi = 0; gi < kGroups; ++gi) {
+      const bool ok = gi < cnt;
+      w[gi] = ok ? __ldg(reinterpret_cast<const uint2*>(in + gi * kGroup)) : make_uint2(0u, 0u);
+      sc[gi] = ok && mine ? load_scalar<ST>(scale, q + gi) : 1.f;
+      m[gi] = ok && mine ? load_scalar<ST>(mn, q + gi) : 0.f;
     }
+    T* dst = out + (n0 * G + g0) * kGroup + lane * kOct;
 #pragma unroll
-    for (int d = 0; d < DEPTH; ++d) {
-      if (!t_ok[d]) break;                                 // warp-uniform
-      const int64_t no = t_no[d], g = t_g[d];
-      const uint2 w = t_w[d];
-      const float sc = t_sc[d], m = t_m[d];
+    for (int gi = 0; gi < kGroups; ++gi) {
+      if (gi >= cnt) break;                                // warp-uniform
       uint32_t entry = 0u, pairs = 0u;
       if constexpr (TABLE) {
-        entry = dequant_bits<T>((float)(lane % E), sc, m);
+        entry = dequant_bits<T>((float)(lane % E), sc[gi], m[gi]);
         if constexpr (sizeof(T) == 2 && BITS <= 2) pairs = entry | (__shfl_down_sync(kFull, entry, 1) << 16);
       }
 #pragma unroll
       for (int ni = 0; ni < WPT; ++ni) {
-        const int64_t n = no * WPT + ni;
         Oct<T> o;
         uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
         if constexpr (sizeof(T) == 2 && BITS <= 2) {
@@ -315,20 +304,20 @@ unpack_single_kernel(const int8_t* __restrict__ packed, const ST* __restrict__ s
           const uint32_t t23 = BITS == 2 ? __shfl_sync(kFull, pairs, ni * E + 2) : t01;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const uint32_t y = ((h ? w.y : w.x) >> (ni * BITS)) & (0x01010101u * (uint32_t)(E - 1));
+            const uint32_t y = ((h ? w[gi].y : w[gi].x) >> (ni * BITS)) & (0x01010101u * (uint32_t)(E - 1));
             const uint32_t sel = y * 0x22u + 0x10101010u;
             ow[2 * h] = __byte_perm(t01, t23, sel);
             ow[2 * h + 1] = __byte_perm(t01, t23, sel >> 16);
           }
         } else {
           uint32_t v[8];
-          const float sc_n = TABLE ? 0.f : __shfl_sync(kFull, sc, ni), m_n = TABLE ? 0.f : __shfl_sync(kFull, m, ni);
+          const float sc_n = TABLE ? 0.f : __shfl_sync(kFull, sc[gi], ni), m_n = TABLE ? 0.f : __shfl_sync(kFull, m[gi], ni);
           float y_n = 0.f;                                       // 16-bit statistics: one reciprocal per group
           const bool recip = !TABLE && sizeof(ST) == 2 && group_reciprocal(sc_n, y_n);   // warp-uniform
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const uint32_t code = ((((j < 4) ? w.x : w.y) >> (8 * (j & 3))) >> (ni * BITS)) & (uint32_t)(E - 1);
-            if constexpr (TABLE) v[j] = __shfl_sync(kFull, entry, ni * E + (int)code);
+            const uint32_t code = (((j < 4) ? w[gi].x : w[gi].y) >> (8 * (j & 3) + ni * BITS)) & (uint32_t)(E - 1);
+            if constexpr (TABLE) v[j] = __shfl_sync(kFull, entry, (int)((uint32_t)(ni * E) | code));
             else v[j] = recip ? dequant_bits_recip<T>((float)code, sc_n, y_n, m_n) : dequant_bits<T>((float)code, sc_n, m_n);
           }
           if constexpr (sizeof(T) == 4) {
@@ -339,7 +328,7 @@ unpack_single_kernel(const int8_t* __restrict__ packed, const ST* __restrict__ s
             for (int k = 0; k < 4; ++k) ow[k] = v[2 * k] | (v[2 * k + 1] << 16);
           }
         }
-        if (n < N) store_oct_streaming<T>(out + (n * G + g) * kGroup + lane * kOct, o);
+        if (n0 + ni < N) store_oct_streaming<T>(dst + (ni * G + gi) * kGroup, o);
       }
     }
   }
@@ -416,7 +405,7 @@ template <typename T, typename ST>
 int launch_unpack(int bits, const int8_t* packed, const void* scale, const void* mn, void* out, int64_t N,
                   int64_t G, cudaStream_t s) {
   const int wpt = 8 / bits;
-  const int64_t tasks = ((N + wpt - 1) / wpt) * G;
+  const int64_t tasks = ((N + wpt - 1) / wpt) * ((G + unpack_groups<T>() - 1) / unpack_groups<T>());
 #define ACTNN_LAUNCH(BITS)                                                                        \
   unpack_single_kernel<T, ST, BITS><<<persistent_grid(unpack_single_kernel<T, ST, BITS>, kThreads, tasks), \
                                       kThreads, 0, s>>>(packed, (const ST*)scale, (const ST*)mn, (T*)out, N, G)
