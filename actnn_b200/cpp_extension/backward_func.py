@@ -65,6 +65,9 @@ def cudnn_convolution_transpose_backward(input, grad_output, weight, padding, ou
 # ---------------------------------------------------------------------------------------
 # channels-last around the convolution library
 # ---------------------------------------------------------------------------------------
+CHANNELS_LAST_ELEMENTS = 1 << 24          # smallest input that is converted, see channels_last_pays
+
+
 def channels_last_pays(input, weight, groups) -> bool:
     """Whether a 2-D convolution of contiguous NCHW tensors is computed on channels-last copies.
 
@@ -74,11 +77,15 @@ def channels_last_pays(input, weight, groups) -> bool:
     per converted tensor; 256 x 256 x 28 x 28: 920 against 509.  1x1 convolutions are matrix products in
     either layout (188 against 157, less than the conversions cost) and stay; so do channel counts that
     NHWC kernels cannot read in 16-byte vectors, grouped convolutions and float32, whose NCHW path
-    does not go through the same kernels."""
+    does not go through the same kernels.  Small layers are paced by the host, to which the library's own
+    conversions are cheaper than seven calls: convolution + ReLU, forward + backward, 128 x 64 x 28 x 28 (6.4 M elements)
+    265 us on NCHW against 288, 12.8 M elements 277 against 285; from 25 M elements on the conversions are GPU time
+    (bottleneck block at batch 256: 253 us of cuDNN's against 93)."""
     return (input.dim() == 4 and input.is_cuda and input.dtype in (torch.float16, torch.bfloat16)
             and weight.dtype == input.dtype and groups == 1 and weight.shape[2] * weight.shape[3] > 1
             and weight.shape[0] % 8 == 0 and weight.shape[1] % 8 == 0 and input.shape[1] == weight.shape[1]
-            and input.shape[2] * input.shape[3] > 1 and input.is_contiguous() and weight.is_contiguous()
+            and input.numel() >= CHANNELS_LAST_ELEMENTS and input.shape[2] * input.shape[3] > 1
+            and input.is_contiguous() and weight.is_contiguous()
             and torch.backends.cudnn.enabled)
 
 

@@ -24,8 +24,10 @@ def test_transpose(batch, rows, cols, offset):
 @pytest.mark.parametrize("c,k,h,ks,stride,pad,dil,bias", [(16, 24, 14, 3, 1, 1, 1, True), (8, 8, 7, 3, 2, 1, 1, False),
                                                           (64, 32, 9, (1, 3), 1, (0, 1), 1, False), (24, 40, 21, 5, 1, 2, 1, True),
                                                           (32, 32, 16, 3, 1, 2, 2, False)])
-def test_convolution_against_64_bit(c, k, h, ks, stride, pad, dil, bias, dtype):
+def test_convolution_against_64_bit(c, k, h, ks, stride, pad, dil, bias, dtype, monkeypatch):
     import actnn_b200 as actnn
+    from actnn_b200.cpp_extension import backward_func as bf
+    monkeypatch.setattr(bf, "CHANNELS_LAST_ELEMENTS", 0)          # small inputs keep NCHW otherwise
     from actnn_b200.conf import config
     torch.manual_seed(c + k)
     layer = actnn.QConv2d(c, k, ks, stride, pad, dil, bias=bias).cuda().to(dtype)
