@@ -466,6 +466,9 @@ def _pool_args(kernel_size, stride, padding, dilation):
                     ("dilation", dilation)):
         if len(v) != 2:
             raise RuntimeError("Expected %s.size() == 2 to be true, but got false." % name)
+        least = 0 if name == "padding" else 1               # before anyone divides by a stride or narrows to a C int
+        if any(not least <= int(a) < 2 ** 31 for a in v):
+            raise RuntimeError("max_pool2d: %s must lie in %d .. 2^31 - 1, got %s" % (name, least, tuple(v)))
     return [int(a) for pair in (kernel_size, stride, padding, dilation) for a in pair]
 
 

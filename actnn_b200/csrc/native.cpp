@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <climits>
 #include <mutex>
 
 #include "../../include/actnn_b200.h"
@@ -281,9 +282,15 @@ struct Dropout : torch::autograd::Function<Dropout> {
 struct MaxPool : torch::autograd::Function<MaxPool> {
   // geom: kernel, stride, padding, dilation, two values each
   static Tensor forward(AutogradContext* ctx, const Tensor& x, std::vector<int64_t> geom) {
-    c10::cuda::CUDAGuard guard(x.device());
+    TORCH_CHECK(geom.size() == 8 && x.dim() == 4, "max_pool2d: a 4-dimensional input and eight geometry values are expected");
     int g[8];
-    for (int i = 0; i < 8; ++i) g[i] = (int)geom[i];
+    for (int i = 0; i < 8; ++i) {                      // the output size below divides by the stride
+      const int64_t least = i == 4 || i == 5 ? 0 : 1;
+      TORCH_CHECK(geom[i] >= least && geom[i] <= INT_MAX, "max_pool2d: kernel_size, stride and dilation must be positive and padding "
+                  "not negative, got ", geom[i]);
+      g[i] = (int)geom[i];
+    }
+    c10::cuda::CUDAGuard guard(x.device());
     const int64_t n = x.size(0), c = x.size(1), h = x.size(2), w = x.size(3);
     auto floordiv = [](int64_t a, int64_t b) { return a / b - (a % b != 0 && (a < 0) != (b < 0)); };
     const int64_t ho = floordiv(h + 2 * g[4] - (int64_t)g[6] * (g[0] - 1) - 1, g[2]) + 1;
