@@ -508,6 +508,11 @@ class batch_norm(Function):
             grad_input, grad_weight, grad_bias = ext_backward_func.native_batch_norm_backward(
                 grad_output, input, weight, running_mean, running_var, save_mean, save_var, training, eps,
                 [ctx.needs_input_grad[0], ctx.needs_input_grad[3], ctx.needs_input_grad[4]])
+        # an input that was None (affine=False) has no gradient; the kernels' sums are dropped then
+        if not ctx.needs_input_grad[3]:
+            grad_weight = None
+        if not ctx.needs_input_grad[4]:
+            grad_bias = None
         if ctx.scheme:
             ctx.scheme.if_allocate_perlayer()
         return grad_input, None, None, grad_weight, grad_bias, None, None, None, None

@@ -112,3 +112,24 @@ def test_layer_backward_takes_the_codes_and_agrees_with_the_decoded_path(monkeyp
         results.append(torch.autograd.grad(layer(x), [x, layer.weight, layer.bias], gy))
     for a, b in zip(*results):
         assert torch.allclose(a.float(), b.float(), rtol=2e-3, atol=2e-3 * b.float().abs().max().item())
+
+
+@pytest.mark.parametrize("hw", [14, 2])                       # from the codes; fewer than 8 positions: decoded
+@pytest.mark.parametrize("frozen", [False, True])
+def test_layer_without_trainable_weight_and_bias(hw, frozen):
+    """``affine=False``, and affine parameters that need no gradient: only the input has one, that of weight 1 and
+    bias 0."""
+    import actnn_b200 as actnn
+    x = torch.randn(12, 40, hw, hw, device="cuda", dtype=torch.float16).requires_grad_()
+    gy = torch.randn_like(x)
+    grads = []
+    for trainable in (True, False):
+        layer = actnn.QBatchNorm2d(40, affine=trainable or frozen).cuda()
+        if not trainable:
+            layer.requires_grad_(False)
+        torch.manual_seed(5)
+        x.grad = None
+        layer(x).backward(gy)
+        assert all((p.grad is not None) == trainable for p in layer.parameters())
+        grads.append(x.grad)
+    assert torch.equal(*grads)
