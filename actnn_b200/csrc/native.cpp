@@ -233,9 +233,11 @@ struct Relu : torch::autograd::Function<Relu> {
     c10::cuda::CUDAGuard guard(x.device());
     Tensor y = at::empty_like(x), mask = mask_like(x);
     const int dt = dtype_id(x.scalar_type());
-    ctx->set_materialize_grads(false);                 // no zero-filled gradients for the extrema
     variable_list out{y};
     if (with_minmax) {
+      ctx->set_materialize_grads(false);               // no zero-filled gradients for the extrema; y's is filled below
+      ctx->saved_data["sizes"] = x.sizes();
+      ctx->saved_data["dtype"] = x.scalar_type();
       Tensor mn = make({x.numel() / 256}, x.scalar_type(), x), mx = make({x.numel() / 256}, x.scalar_type(), x);
       check(actnn_relu_forward_minimax(x.data_ptr(), y.data_ptr(), mask.data_ptr<int32_t>(), mn.data_ptr(), mx.data_ptr(),
                                        x.numel(), dt, stream()),
@@ -251,8 +253,11 @@ struct Relu : torch::autograd::Function<Relu> {
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    if (!grads[0].defined()) return {Tensor(), Tensor()};
-    return {relu_backward(grads[0], ctx->get_saved_variables()[0]), Tensor()};
+    const Tensor mask = ctx->get_saved_variables()[0];
+    if (grads[0].defined()) return {relu_backward(grads[0], mask), Tensor()};
+    // the layer above gave no gradient, which counts as zeros
+    return {at::zeros(ctx->saved_data["sizes"].toIntVector(), mask.options().dtype(ctx->saved_data["dtype"].toScalarType())),
+            Tensor()};
   }
 };
 
