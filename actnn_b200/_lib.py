@@ -6,6 +6,7 @@ is raised.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from ctypes import c_char_p, c_double, c_float, c_int, c_int64, c_uint64, c_void_p
@@ -115,9 +116,15 @@ _tickets = {}
 
 
 def ticket(device: torch.device) -> torch.Tensor:
-    """256 zeroed bytes per (device, current stream) that only ``actnn_compress_mixed_prestat_kept``
-    uses: its kernels leave the ticket at zero, so it never needs clearing again."""
+    """256 zeroed bytes per (device, current stream) for the kernels of ``actnn_compress_mixed_prestat_kept`` and
+    ``actnn_batch_norm_codes_forward``, which run in stream order and leave it at zero, so it never needs clearing
+    again.  While the stream is being captured: a block of the graph's own, cleared by every replay.  A kept one
+    could not be shared with a graph: made during a capture it is only cleared when that graph runs, and a
+    replay on another stream would use it at the same time."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
+    with torch.cuda.device(idx) if idx != torch.cuda.current_device() else contextlib.nullcontext():
+        if torch.cuda.is_current_stream_capturing():
+            return torch.zeros(256, dtype=torch.uint8, device=device)
     key = (idx, stream_of_index(idx))
     buf = _tickets.get(key)
     if buf is None:
