@@ -51,3 +51,18 @@ def test_many_planes_and_unaligned_gradient(offset):
     ref = torch.zeros(64 * 96, 56 * 56, device="cuda", dtype=torch.float64)
     ref.scatter_add_(1, ri.view(64 * 96, -1), gy.double().view(64 * 96, -1))
     assert ((gx.double().view_as(ref) - ref).abs() <= 2 ** -10 * ref.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("h,w", [(9, 16), (12, 24)])
+@pytest.mark.parametrize("k,p", [(2, 0), (2, 1), (3, 0), (3, 1)])
+def test_value_is_the_first_maximum_to_the_bit(k, p, h, w, dtype):
+    """Windows whose maximum is a zero: the sign of the first zero, not that of a later one."""
+    from actnn_b200.cpp_extension import quantization as q
+    torch.manual_seed(h + k)
+    x = torch.tensor([-0.0, 0.0, -1.0])[torch.randint(3, (3, 5, h, w))].to(dtype)
+    geom = ((k, k), (2, 2), (p, p), (1, 1))
+    y, idx = q.max_pool2d_forward(x.cuda(), *geom)
+    ry, ridx = O.max_pool2d_forward(x, *geom)
+    bits = torch.int32 if dtype == torch.float32 else torch.int16
+    assert torch.equal(y.cpu().view(bits), ry.view(bits)) and torch.equal(idx.cpu(), ridx)
