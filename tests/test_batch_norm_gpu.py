@@ -269,35 +269,36 @@ def test_statistics_and_minmax_pass_declines_other_geometries(cuda_device):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
-def test_quantized_batch_norm_takes_the_one_read_path_and_matches_the_two_read_path(actnn, cuda_device, dtype):
-    """ops.batch_norm at level L3 on a covered geometry: output, gradients and the saved
-    compressed activation are the same as with the separate minimax and statistics passes."""
+def test_quantized_batch_norm_takes_the_one_read_path_and_matches_the_two_read_path(actnn, cuda_device, dtype, monkeypatch):
+    """ops.batch_norm at level L3 on a covered geometry: the saved compressed activation is that of the separate
+    minimax, statistics, compress, normalise and decode passes to the bit, output and gradients are theirs up to
+    the order of sums."""
     from actnn_b200 import ops
     from actnn_b200.cpp_extension import backward_func as bf
     actnn.set_optimization_level("L3")
     N, C, H, W = 6, 32, 16, 24
     x, gy, w, b, rm, rv = _inputs((N, C, H, W), dtype, cuda_device, seed=5)
     gen = torch.cuda.default_generators[cuda_device.index or 0]
-    results = []
+    fast = ("batch_norm_stats_minimax", "batch_norm_codes_forward", "batch_norm_codes_backward")
+    results, saved = [], []
     for fused in (True, False):
         scheme = actnn.QBNScheme()
-        real = bf.batch_norm_stats_minimax
-        calls = []
-        if fused:
-            bf.batch_norm_stats_minimax = lambda *a, **k: (calls.append(1), real(*a, **k))[1]
-        else:
-            bf.batch_norm_stats_minimax = lambda *a, **k: None
-        try:
-            gen.manual_seed(77)
-            xi = x.clone().requires_grad_(True)
-            wi, bi = w.clone().requires_grad_(True), b.clone().requires_grad_(True)
-            rmi, rvi = rm.clone(), rv.clone()
-            y = ops.batch_norm.apply(xi, rmi, rvi, wi, bi, True, 0.1, 1e-5, scheme)
-            y.backward(gy)
-        finally:
-            bf.batch_norm_stats_minimax = real
-        assert bool(calls) == fused
+        calls = set()
+        for name in fast:
+            real = getattr(bf, name)
+            monkeypatch.setattr(bf, name, (lambda *a, real=real, name=name, **k: (calls.add(name), real(*a, **k))[1])
+                                if fused else (lambda *a, **k: None))
+        gen.manual_seed(77)
+        xi = x.clone().requires_grad_(True)
+        wi, bi = w.clone().requires_grad_(True), b.clone().requires_grad_(True)
+        rmi, rvi = rm.clone(), rv.clone()
+        y = ops.batch_norm.apply(xi, rmi, rvi, wi, bi, True, 0.1, 1e-5, scheme)
+        saved.append(y.grad_fn.saved[0])
+        y.backward(gy)
+        monkeypatch.undo()
+        assert calls == (set(fast) if fused else set())
         results.append((y.detach(), xi.grad, wi.grad, bi.grad, rmi, rvi))
+    assert all(torch.equal(p, q) for p, q in zip(*saved))                   # packed, bits, scale, min
     tol = TOL[dtype]
     for a, r in zip(*results):
         assert _close(a, r, 4 * tol)

@@ -98,20 +98,57 @@ def test_forward(shape, dtype, stochastic):
     assert ((y.double() - ry).abs() <= (EPS[dtype] * 1.01 + 2048 * 2 ** -24) * big).all()
 
 
-def test_layer_backward_takes_the_codes_and_agrees_with_the_decoded_path(monkeypatch):
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("shape", [(2, 64, 3136), (9, 16, 800), (33, 3, 256), (70, 8, 288)])
+def test_forward_from_statistics_of_a_pass_before_it(shape, dtype):
+    """What maps of 256 and more whole groups take: ranges and statistics come from ``batch_norm_stats_minimax``."""
+    from actnn_b200.cpp_extension import backward_func as bf
+    from actnn_b200.cpp_extension import quantization as q
+    n, c, hw = shape
+    torch.manual_seed(2)
+    x = (torch.randn(n, c, hw, device="cuda") * 1.5 + torch.linspace(-8, 8, c, device="cuda").view(1, c, 1)).to(dtype)
+    weight, bias = torch.rand(c, device="cuda") + 0.5, torch.randn(c, device="cuda")
+    rm, rv = torch.randn(c, device="cuda"), torch.rand(c, device="cuda")
+    stats = bf.batch_norm_stats_minimax(x, weight, bias, rm, rv, 0.1, 1e-5)
+    after = rm.clone(), rv.clone()
+    gen = torch.cuda.default_generators[torch.cuda.current_device()]
+    gen.manual_seed(9)
+    gen.set_offset(4)
+    y, quantized, mean, invstd = bf.batch_norm_codes_forward(x, weight, bias, rm, rv, 0.1, 1e-5, 2 * n, 8, 0.5, True, stats)
+    assert torch.equal(rm, after[0]) and torch.equal(rv, after[1])          # updated once, by the pass before
+    assert torch.equal(mean, stats[2]) and torch.equal(invstd, stats[3])
+    stat = torch.bfloat16 if dtype == torch.float32 else dtype
+    ref = q.compress_mixed_precision(x.view(n, c * hw // 256, 256), 2 * n, 8, 0.5, philox=(9, 4), stat_dtype=stat)
+    assert all(torch.equal(a, b) for a, b in zip(quantized, ref))          # the codec to the bit
+    assert torch.equal(y, bf.batch_norm_elemt(x, weight, bias, mean, invstd, 1e-5))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,c,h,w", [(20, 48, 14, 14), (6, 5, 9, 7), (40, 16, 16, 16), (12, 24, 2, 2), (3, 8, 1, 8)])
+@pytest.mark.parametrize("affine", ["float32", "as the input"])
+def test_layer_backward_takes_the_codes_and_agrees_with_the_decoded_path(monkeypatch, n, c, h, w, dtype, affine):
+    """Maps of at least 8 positions take the codes, smaller ones the decoded path in both arms."""
     import actnn_b200 as actnn
     from actnn_b200.cpp_extension import backward_func as bf
-    layer = actnn.QBatchNorm2d(48).cuda()
-    x = torch.randn(20, 48, 14, 14, device="cuda", dtype=torch.float16).requires_grad_()
+    layer = actnn.QBatchNorm2d(c).cuda()
+    if affine != "float32":
+        layer.weight.data, layer.bias.data = layer.weight.data.to(dtype), layer.bias.data.to(dtype)
+    x = torch.randn(n, c, h, w, device="cuda", dtype=dtype).requires_grad_()
     gy = torch.randn_like(x)
-    results = []
+    real, results, taken = bf.batch_norm_codes_backward, [], []
     for use in (True, False):
-        if not use:
-            monkeypatch.setattr(bf, "batch_norm_codes_backward", lambda *a: None)
+        monkeypatch.setattr(bf, "batch_norm_codes_backward",
+                            (lambda *a: (taken.append(real(*a)), taken[-1])[1]) if use else lambda *a: None)
         torch.manual_seed(5)
         results.append(torch.autograd.grad(layer(x), [x, layer.weight, layer.bias], gy))
+    assert (taken[0] is not None) == (h * w >= 8)
+    # sums in another order: 64 float32 roundings of sums of n * h * w terms of order one; then one rounding to the
+    # type of the result, and of x's gradient another where its two sums' roundings moved it
     for a, b in zip(*results):
-        assert torch.allclose(a.float(), b.float(), rtol=2e-3, atol=2e-3 * b.float().abs().max().item())
+        assert a.dtype == b.dtype
+        big = b.double().abs().max().item()
+        bound = 2 * EPS[a.dtype] * b.double().abs() + 64 * 2 ** -24 * (big + (n * h * w) ** 0.5 * 4)
+        assert ((a.double() - b.double()).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("hw", [14, 2])                       # from the codes; fewer than 8 positions: decoded

@@ -95,6 +95,80 @@ def test_host_side_validation_needs_no_gpu(lib):
     assert lib.actnn_compress_mixed(*args) == SHAPE
 
 
+def test_host_side_validation_of_the_column_entry_points(lib):
+    """The samples codec, batch norm on the codes, the joint allocation and the transpose."""
+    OK, NULL, DTYPE, SHAPE, BITS, ALIGN, ARG, CAPACITY = 0, 1, 2, 3, 4, 5, 6, 8
+    nan = float("nan")
+
+    def changed(args, **at):
+        args = list(args)
+        for i, v in at.items():
+            args[int(i[1:])] = v
+        return args
+
+    # data packed scale mn bits offsets C workspace, bytes N F dtype stat_dtype, factors, bits target, noise, stream
+    comp = [256] * 8 + [1 << 20, 4, 700, 1, 1, 1.0, 1.0, None, 8, 8.0, 1, None, 0, 0, None]
+    call = lib.actnn_compress_mixed_samples
+    assert call(*changed(comp, _9=-1)) == SHAPE
+    assert call(*changed(comp, _9=0)) == OK
+    assert call(*changed(comp, _11=7)) == DTYPE and call(*changed(comp, _12=0)) == DTYPE
+    assert call(*changed(comp, _16=9)) == BITS and call(*changed(comp, _16=0)) == BITS
+    assert all(call(*changed(comp, **{"_%d" % i: None})) == NULL for i in range(8))
+    assert call(*changed(comp, _8=64)) == CAPACITY
+    assert call(*changed(comp, _0=257)) == ALIGN and call(*changed(comp, _7=264)) == ALIGN
+    # packed bits offsets scale mn out, N F dtype stat_dtype, stream
+    unp = [256] * 6 + [4, 700, 1, 1, None]
+    call = lib.actnn_unpack_mixed_samples
+    assert call(*changed(unp, _7=-1)) == SHAPE
+    assert call(*changed(unp, _6=0)) == OK and call(*changed(unp, _7=0)) == OK
+    assert call(*changed(unp, _8=3)) == DTYPE and call(*changed(unp, _9=2)) == DTYPE
+    assert all(call(*changed(unp, **{"_%d" % i: None})) == NULL for i in range(6))
+    assert call(*changed(unp, _5=257)) == ALIGN
+
+    size = ctypes.c_int64(0)
+    call = lib.actnn_batch_norm_codes_workspace
+    assert call(4, 3, 49, 1, None) == NULL and call(4, 3, 49, 7, ctypes.addressof(size)) == DTYPE
+    assert call(4, 3, 7, 1, ctypes.addressof(size)) == SHAPE          # fewer than 8 positions
+    assert call(4, 1 << 28, 8, 1, ctypes.addressof(size)) == SHAPE    # a sample of 2^31 elements
+    assert call(4, 3, 49, 1, ctypes.addressof(size)) == OK and size.value > 0
+    # x group_mn group_mx weight bias running_mean running_var y mean invstd packed scale mn bits offsets C, N C HW,
+    # momentum eps dtype stat_dtype, factor bits target stochastic seed offset, ticket workspace bytes stream
+    fwd = [256, None, None] + [256] * 13 + [4, 3, 49, 0.1, 1e-5, 1, 1, 1.0, 8, 8.0, 1, 0, 0, 256, 256, size.value, None]
+    call = lib.actnn_batch_norm_codes_forward
+    assert call(*changed(fwd, _18=7)) == SHAPE and call(*changed(fwd, _16=0)) == SHAPE
+    assert call(*changed(fwd, _21=5)) == DTYPE and call(*changed(fwd, _22=2)) == DTYPE
+    assert call(*changed(fwd, _24=9)) == BITS and call(*changed(fwd, _25=nan)) == ARG
+    assert all(call(*changed(fwd, **{"_%d" % i: None})) == NULL for i in (0, 7, 8, 9, 10, 11, 12, 13, 14, 15, 29, 30))
+    assert call(*changed(fwd, _1=256)) == NULL                          # minima without maxima
+    assert call(*changed(fwd, _30=264)) == ALIGN and call(*changed(fwd, _0=257)) == ALIGN
+    assert call(*changed(fwd, _18=256, _0=264)) == ALIGN                # whole groups want vector alignment
+    assert call(*changed(fwd, _31=64)) == CAPACITY
+    # packed bits offsets scale mn dy weight mean invstd dx dweight dbias, N C HW dtype stat_dtype, workspace bytes stream
+    bwd = [256] * 12 + [4, 3, 49, 1, 1, 256, size.value, None]
+    call = lib.actnn_batch_norm_codes_backward
+    assert call(*changed(bwd, _14=7)) == SHAPE and call(*changed(bwd, _15=-1)) == DTYPE and call(*changed(bwd, _16=0)) == DTYPE
+    assert all(call(*changed(bwd, **{"_%d" % i: None})) == NULL for i in (0, 1, 2, 3, 4, 5, 7, 8, 9, 17))
+    assert call(*changed(bwd, _5=257)) == ALIGN and call(*changed(bwd, _17=264)) == ALIGN
+    assert call(*changed(bwd, _18=16)) == CAPACITY
+
+    ptrs, dims = (ctypes.c_uint64 * 2)(256, 256), (ctypes.c_int32 * 2)(5, 6)
+    alloc = [ctypes.addressof(ptrs), ctypes.addressof(dims), 2, 4, 8, 80.0, 256, None]
+    call = lib.actnn_allocate_layers
+    assert call(*changed(alloc, _2=-1)) == SHAPE and call(*changed(alloc, _2=0)) == OK
+    assert call(*changed(alloc, _4=9)) == BITS and call(*changed(alloc, _5=nan)) == ARG
+    assert all(call(*changed(alloc, **{"_%d" % i: None})) == NULL for i in (0, 1, 6))
+    assert call(*changed(alloc, _2=257)) == CAPACITY and call(*changed(alloc, _3=20000)) == CAPACITY
+    ptrs[1] = 0
+    assert call(*alloc) == NULL
+    ptrs[1], dims[1] = 256, 0
+    assert call(*alloc) == ARG
+
+    call = lib.actnn_transpose16
+    assert call(256, 256, 1, -1, 8, None) == SHAPE and call(256, 256, 0, 8, 8, None) == OK
+    assert call(None, 256, 1, 8, 8, None) == NULL and call(256, None, 1, 8, 8, None) == NULL
+    assert call(257, 256, 1, 8, 8, None) == ALIGN and call(256, 257, 1, 8, 8, None) == ALIGN
+
+
 def test_missing_library_is_an_error(monkeypatch, tmp_path):
     from actnn_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)

@@ -206,3 +206,88 @@ def test_statistics_minmax_pass_stays_inside_its_outputs(env, shape, dtype):
         assert int(cm["ticket"].t[:4].view(torch.int32)) == 0
         for k, v in first.items():
             assert torch.equal(cm[k].t, v), k
+
+
+def _column_input(shape, offset, dtype, dev):
+    """An activation ``[n, c, hw]`` and a gradient of its shape, ``offset`` elements into their storage."""
+    numel = shape[0] * shape[1] * shape[2]
+    gen = torch.Generator().manual_seed(numel + offset)
+    return [torch.randn(numel + offset, generator=gen).to(dtype).to(dev)[offset:] for _ in range(2)]
+
+
+# (n, c, hw): odd maps, 8 positions (up to 129 channels a column), one sample, a column of one partial group, whole groups
+COLUMN_SHAPES = [(1, 130, 9), (3, 20, 12), (5, 3, 40), (40, 7, 49), (6, 33, 8), (1, 300, 8), (33, 5, 225), (2, 64, 784)]
+
+
+@pytest.mark.parametrize("dtype", DTS)
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("shape", COLUMN_SHAPES)
+def test_column_entry_points_stay_inside_their_outputs(env, shape, offset, dtype):
+    """actnn_compress_mixed_samples, actnn_batch_norm_codes_forward and _backward, with workspaces of exactly the
+    size they ask for."""
+    import ctypes
+    lib, _lib, q, dev = env
+    n, c, hw = shape
+    f = c * hw
+    if f % 256 == 0 and offset:
+        pytest.skip("whole groups want vector alignment")
+    g = (f + 255) // 256
+    sdt = torch.bfloat16 if dtype == torch.float32 else dtype
+    D, S = _lib.dtype_id(dtype), _lib.dtype_id(sdt)
+    st = torch.cuda.current_stream().cuda_stream
+    x, dy = _column_input(shape, offset, dtype, dev)
+    total = 2 * n
+
+    def stream_buffers():
+        return {"packed": Guarded(total * g * 8, torch.int32, dev), "scale": Guarded(n * g, sdt, dev),
+                "min": Guarded(n * g, sdt, dev), "bits": Guarded(n, torch.int32, dev),
+                "word_offsets": Guarded(n + 1, torch.int64, dev), "C": Guarded(n, torch.float32, dev)}
+
+    cm = stream_buffers()
+    ws_bytes = lib.actnn_compress_mixed_workspace(n, g, D)
+    cm["workspace"] = Guarded(ws_bytes, torch.uint8, dev)
+    _check(_lib, lib.actnn_compress_mixed_samples(x.data_ptr(), cm["packed"].ptr(), cm["scale"].ptr(), cm["min"].ptr(),
+                                                  cm["bits"].ptr(), cm["word_offsets"].ptr(), cm["C"].ptr(),
+                                                  cm["workspace"].ptr(), ws_bytes, n, f, D, S, 1.0, 1.0, None, 8,
+                                                  float(total), 1, None, 5, 0, st), "actnn_compress_mixed_samples", cm)
+    assert int(cm["bits"].t.sum()) == total
+
+    nbytes = ctypes.c_int64(0)
+    _lib.check(lib.actnn_batch_norm_codes_workspace(n, c, hw, D, ctypes.addressof(nbytes)), "workspace")
+    weight, bias = torch.rand(c, device=dev) + 0.5, torch.randn(c, device=dev)
+    fw = stream_buffers()
+    fw.update(y=Guarded(n * f, dtype, dev), mean=Guarded(c, torch.float32, dev), invstd=Guarded(c, torch.float32, dev),
+              running_mean=Guarded(c, torch.float32, dev), running_var=Guarded(c, torch.float32, dev),
+              ticket=Guarded(256, torch.uint8, dev), workspace=Guarded(nbytes.value, torch.uint8, dev))
+    for name in ("ticket", "running_mean", "running_var"):
+        fw[name].t.zero_()
+    _check(_lib, lib.actnn_batch_norm_codes_forward(
+        x.data_ptr(), None, None, weight.data_ptr(), bias.data_ptr(), fw["running_mean"].ptr(), fw["running_var"].ptr(),
+        fw["y"].ptr(), fw["mean"].ptr(), fw["invstd"].ptr(), fw["packed"].ptr(), fw["scale"].ptr(), fw["min"].ptr(),
+        fw["bits"].ptr(), fw["word_offsets"].ptr(), fw["C"].ptr(), n, c, hw, 0.1, 1e-5, D, S, 1.0, 8, float(total), 1, 5,
+        0, fw["ticket"].ptr(), fw["workspace"].ptr(), nbytes.value, st), "actnn_batch_norm_codes_forward", fw)
+    assert all(torch.equal(fw[k].t, cm[k].t) for k in ("packed", "scale", "min", "bits", "word_offsets", "C"))
+    assert not fw["ticket"].t.any()
+
+    bw = {"dx": Guarded(n * f, dtype, dev), "dweight": Guarded(c, torch.float32, dev),
+          "dbias": Guarded(c, torch.float32, dev), "workspace": Guarded(nbytes.value, torch.uint8, dev)}
+    _check(_lib, lib.actnn_batch_norm_codes_backward(
+        fw["packed"].ptr(), fw["bits"].ptr(), fw["word_offsets"].ptr(), fw["scale"].ptr(), fw["min"].ptr(),
+        dy.data_ptr(), weight.data_ptr(), fw["mean"].ptr(), fw["invstd"].ptr(), bw["dx"].ptr(), bw["dweight"].ptr(),
+        bw["dbias"].ptr(), n, c, hw, D, S, bw["workspace"].ptr(), nbytes.value, st),
+        "actnn_batch_norm_codes_backward", dict(bw, **fw))
+    assert torch.isfinite(bw["dx"].t.float()).all()
+
+
+@pytest.mark.parametrize("layers,n", [(1, 1), (3, 7), (5, 300), (256, 128)])
+def test_layer_allocation_stays_inside_its_output(env, layers, n):
+    import ctypes
+    lib, _lib, q, dev = env
+    C = torch.rand(layers, n, generator=torch.Generator().manual_seed(n)).to(dev)
+    ptrs = (ctypes.c_uint64 * layers)(*[C[i].data_ptr() for i in range(layers)])
+    dims = (ctypes.c_int32 * layers)(*[100 + i for i in range(layers)])
+    sums = Guarded(layers, torch.int32, dev)
+    _check(_lib, lib.actnn_allocate_layers(ctypes.addressof(ptrs), ctypes.addressof(dims), layers, n, 8,
+                                           2.0 * n * sum(dims), sums.ptr(), torch.cuda.current_stream().cuda_stream),
+           "actnn_allocate_layers", {"sums": sums})
+    assert (sums.t >= n).all() and (sums.t <= 8 * n).all()
