@@ -249,15 +249,10 @@ pack_single_kernel(const T* __restrict__ data, const T* __restrict__ mn, const T
   }
 }
 
-// Unpack: a warp owns (sample block, four neighbouring groups; two for float32).  Lane t reads its eight bytes of each group
-// once; the table of all wpt samples x 2^BITS codes of a group is computed by the first wpt * 2^BITS lanes
-// together (one IEEE division per lane), and for 16-bit outputs with BITS <= 2 a byte-permute selects two
-// decoded elements per instruction.
-// Bound by instruction issue: with one group per task, two tasks requested ahead, a lane spent 107 instructions on an
-// octet, most of them not on its elements (4 bits, 256 x 256 x 28 x 28 float16: 28.1 us).  Four groups share the
-// task's index arithmetic and addresses and are requested together: 21.7 us (two groups: 23.7). float32, whose octets
-// are twice as large, 2 bits, 64 x 64 x 56 x 56: one group 9.9, two 9.6, four 10.4 us.
-template <typename T> constexpr int unpack_groups() { return sizeof(T) == 2 ? 4 : 2; }
+// Unpack: a warp owns (sample block, group).  Lane t reads its eight bytes once; the table
+// of all wpt samples x 2^BITS codes is computed by the first wpt * 2^BITS lanes together
+// (one IEEE division per lane), and for 16-bit outputs with BITS <= 2 a byte-permute
+// selects two decoded elements per instruction.
 template <typename T, typename ST, int BITS>
 __global__ void __launch_bounds__(kThreads, 4)
 unpack_single_kernel(const int8_t* __restrict__ packed, const ST* __restrict__ scale,
@@ -265,22 +260,117 @@ unpack_single_kernel(const int8_t* __restrict__ packed, const ST* __restrict__ s
   constexpr int WPT = 8 / BITS;
   constexpr int E = 1 << BITS;
   constexpr bool TABLE = BITS <= 4;                        // BITS == 8: divide per element
-  constexpr int kGroups = unpack_groups<T>();
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
+  const int64_t nblocks = (N + WPT - 1) / WPT;
+
+  // The packed stream is an eighth of the output or less, so a task's loads are small; to
+  // keep enough bytes in flight each warp issues the loads of DEPTH tasks before it decodes
+  // the first of them.
+  constexpr int DEPTH = 2;
+  const int my_s = TABLE ? lane / E : lane;                // lane l serves sample no*wpt + my_s
+  PairWalker walk(warp, nwarps, nblocks, G);
+  while (walk.valid()) {
+    int64_t t_no[DEPTH], t_g[DEPTH];
+    uint2 t_w[DEPTH];
+    float t_sc[DEPTH], t_m[DEPTH];
+    bool t_ok[DEPTH];
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) {
+      t_ok[d] = walk.valid();
+      t_no[d] = walk.no;
+      t_g[d] = walk.r;
+      t_w[d] = make_uint2(0u, 0u);
+      t_sc[d] = 1.f;
+      t_m[d] = 0.f;
+      if (t_ok[d]) {
+        t_w[d] = __ldg(reinterpret_cast<const uint2*>(packed + ((t_no[d] * G + t_g[d]) * kGroup + lane * kOct)));
+        const int64_t my_n = t_no[d] * WPT + my_s;
+        if (my_s < WPT && my_n < N) {
+          t_sc[d] = load_scalar<ST>(scale, my_n * G + t_g[d]);
+          t_m[d] = load_scalar<ST>(mn, my_n * G + t_g[d]);
+        }
+        walk.next();
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) {
+      if (!t_ok[d]) break;                                 // warp-uniform
+      const int64_t no = t_no[d], g = t_g[d];
+      const uint2 w = t_w[d];
+      const float sc = t_sc[d], m = t_m[d];
+      uint32_t entry = 0u, pairs = 0u;
+      if constexpr (TABLE) {
+        entry = dequant_bits<T>((float)(lane % E), sc, m);
+        if constexpr (sizeof(T) == 2 && BITS <= 2) pairs = entry | (__shfl_down_sync(kFull, entry, 1) << 16);
+      }
+#pragma unroll
+      for (int ni = 0; ni < WPT; ++ni) {
+        const int64_t n = no * WPT + ni;
+        Oct<T> o;
+        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+        if constexpr (sizeof(T) == 2 && BITS <= 2) {
+          const uint32_t t01 = __shfl_sync(kFull, pairs, ni * E);
+          const uint32_t t23 = BITS == 2 ? __shfl_sync(kFull, pairs, ni * E + 2) : t01;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t y = ((h ? w.y : w.x) >> (ni * BITS)) & (0x01010101u * (uint32_t)(E - 1));
+            const uint32_t sel = y * 0x22u + 0x10101010u;
+            ow[2 * h] = __byte_perm(t01, t23, sel);
+            ow[2 * h + 1] = __byte_perm(t01, t23, sel >> 16);
+          }
+        } else {
+          uint32_t v[8];
+          const float sc_n = TABLE ? 0.f : __shfl_sync(kFull, sc, ni), m_n = TABLE ? 0.f : __shfl_sync(kFull, m, ni);
+          float y_n = 0.f;                                       // 16-bit statistics: one reciprocal per group
+          const bool recip = !TABLE && sizeof(ST) == 2 && group_reciprocal(sc_n, y_n);   // warp-uniform
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t code = ((((j < 4) ? w.x : w.y) >> (8 * (j & 3))) >> (ni * BITS)) & (uint32_t)(E - 1);
+            if constexpr (TABLE) v[j] = __shfl_sync(kFull, entry, ni * E + (int)code);
+            else v[j] = recip ? dequant_bits_recip<T>((float)code, sc_n, y_n, m_n) : dequant_bits<T>((float)code, sc_n, m_n);
+          }
+          if constexpr (sizeof(T) == 4) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ow[j] = v[j];
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ow[k] = v[2 * k] | (v[2 * k + 1] << 16);
+          }
+        }
+        if (n < N) store_oct_streaming<T>(out + (n * G + g) * kGroup + lane * kOct, o);
+      }
+    }
+  }
+}
+
+// Unpack of neighbouring groups: a warp task is GROUPS groups of a sample block, requested together; they share the
+// task's index arithmetic and addresses, which pays where decoding costs most (see launch_unpack).  The decoding is
+// that of the kernel above, written out again: as a function that both call it took 22.2 instead of 20.6 us there
+// (2 bits, 256 x 784 groups of float16) and 44.5 instead of 42.8 here (8 bits).
+template <typename T, typename ST, int BITS, int GROUPS>
+__global__ void __launch_bounds__(kThreads, 4)
+unpack_single_groups_kernel(const int8_t* __restrict__ packed, const ST* __restrict__ scale,
+                            const ST* __restrict__ mn, T* __restrict__ out, int64_t N, int64_t G) {
+  constexpr int WPT = 8 / BITS;
+  constexpr int E = 1 << BITS;
+  constexpr bool TABLE = BITS <= 4;                        // BITS == 8: divide per element
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
   const int64_t nblocks = (N + WPT - 1) / WPT;
   const int my_s = TABLE ? lane / E : lane;                // lane l serves sample no*wpt + my_s
-  for (PairWalker walk(warp, nwarps, nblocks, (G + kGroups - 1) / kGroups); walk.valid(); walk.next()) {
-    const int64_t g0 = (int64_t)walk.r * kGroups, n0 = walk.no * WPT;
-    const int cnt = (int)min((int64_t)kGroups, G - g0);
+  for (PairWalker walk(warp, nwarps, nblocks, (G + GROUPS - 1) / GROUPS); walk.valid(); walk.next()) {
+    const int64_t g0 = (int64_t)walk.r * GROUPS, n0 = walk.no * WPT;
+    const int cnt = (int)min((int64_t)GROUPS, G - g0);
     const int8_t* in = packed + ((walk.no * G + g0) * kGroup + lane * kOct);
     const bool mine = my_s < WPT && n0 + my_s < N;
     const int64_t q = (n0 + my_s) * G + g0;
-    uint2 w[kGroups];
-    float sc[kGroups], m[kGroups];
+    uint2 w[GROUPS];
+    float sc[GROUPS], m[GROUPS];
 #pragma unroll
-    for (int gi = 0; gi < kGroups; ++gi) {
+    for (int gi = 0; gi < GROUPS; ++gi) {
       const bool ok = gi < cnt;
       w[gi] = ok ? __ldg(reinterpret_cast<const uint2*>(in + gi * kGroup)) : make_uint2(0u, 0u);
       sc[gi] = ok && mine ? load_scalar<ST>(scale, q + gi) : 1.f;
@@ -288,7 +378,7 @@ unpack_single_kernel(const int8_t* __restrict__ packed, const ST* __restrict__ s
     }
     T* dst = out + (n0 * G + g0) * kGroup + lane * kOct;
 #pragma unroll
-    for (int gi = 0; gi < kGroups; ++gi) {
+    for (int gi = 0; gi < GROUPS; ++gi) {
       if (gi >= cnt) break;                                // warp-uniform
       uint32_t entry = 0u, pairs = 0u;
       if constexpr (TABLE) {
@@ -405,10 +495,36 @@ template <typename T, typename ST>
 int launch_unpack(int bits, const int8_t* packed, const void* scale, const void* mn, void* out, int64_t N,
                   int64_t G, cudaStream_t s) {
   const int wpt = 8 / bits;
-  const int64_t tasks = ((N + wpt - 1) / wpt) * ((G + unpack_groups<T>() - 1) / unpack_groups<T>());
-#define ACTNN_LAUNCH(BITS)                                                                        \
-  unpack_single_kernel<T, ST, BITS><<<persistent_grid(unpack_single_kernel<T, ST, BITS>, kThreads, tasks), \
-                                      kThreads, 0, s>>>(packed, (const ST*)scale, (const ST*)mn, (T*)out, N, G)
+  // us, one group a task against two and four, activations of 205 and 411 MB (of float32: of 205 and 411 MB):
+  //   16-bit types  4 bits  30.0 -> 28.8, 25.0    55.7 -> 51.9, 44.6
+  //                 8 bits  56.4 -> 42.8, 42.0   109.3 -> 81.9, 82.2
+  //                 1 bit   18.3 -> 18.5, 21.3    34.5 -> 35.2, 36.5
+  //                 2 bits  20.7 -> 20.7, 21.6    35.9 -> 36.5, 38.8
+  //   float32       4 bits  40.7 -> 43.0, 43.7    79.1 -> 84.8, 84.5
+  //                 8 bits  55.3 -> 44.4, 44.1   108.0 -> 85.0, 85.6
+  //                 2 bits  39.8 -> 41.4, 40.7    78.8 -> 80.2, 79.8
+  // Wider tasks are fewer.  At 4 bits four groups hide their own latency, so that half the resident warps are enough
+  // (8 x 3136 groups of float16, 3136 tasks: 5.2 -> 4.7; 128 x 49, 832 tasks: 2.7 against 3.6).  At 8 bits two groups
+  // want all of them (64 x 784: 16.1 -> 12.9; 512 x 3, 1024 tasks: 2.4 against 2.8) and four, which gain in bfloat16 only
+  // (16 x 7442: 32.4 -> 31.4, 256 x 784: 52.3 -> 49.4), four rounds of tasks (64 x 784, 2.6 rounds: 12.9 against 14.1).
+  const int64_t blocks = (N + wpt - 1) / wpt, resident = (int64_t)device_info().sm_count * 4 * (kThreads / 32);
+  const int64_t of_four = blocks * ((G + 3) / 4), of_two = blocks * ((G + 1) / 2);
+#define ACTNN_RUN(KERNEL, TASKS)                                                                          \
+  {                                                                                                       \
+    auto kernel = KERNEL;                                                                                 \
+    kernel<<<persistent_grid(kernel, kThreads, TASKS), kThreads, 0, s>>>(packed, (const ST*)scale, (const ST*)mn, \
+                                                                         (T*)out, N, G);                  \
+  }
+#define ACTNN_LAUNCH(BITS)                                                                                \
+  if (BITS == 4 && sizeof(T) == 2 && 2 * of_four >= resident) {                                           \
+    if constexpr (BITS == 4 && sizeof(T) == 2) ACTNN_RUN((unpack_single_groups_kernel<T, ST, BITS, 4>), of_four) \
+  } else if (BITS == 8 && of_four >= 4 * resident) {                                                      \
+    if constexpr (BITS == 8) ACTNN_RUN((unpack_single_groups_kernel<T, ST, BITS, 4>), of_four)            \
+  } else if (BITS == 8 && of_two >= resident) {                                                           \
+    if constexpr (BITS == 8) ACTNN_RUN((unpack_single_groups_kernel<T, ST, BITS, 2>), of_two)             \
+  } else {                                                                                                \
+    ACTNN_RUN((unpack_single_kernel<T, ST, BITS>), blocks * G)                                            \
+  }
   switch (bits) {
     case 1: ACTNN_LAUNCH(1); break;
     case 2: ACTNN_LAUNCH(2); break;
@@ -416,6 +532,7 @@ int launch_unpack(int bits, const int8_t* packed, const void* scale, const void*
     default: ACTNN_LAUNCH(8); break;
   }
 #undef ACTNN_LAUNCH
+#undef ACTNN_RUN
   return check_launch();
 }
 
