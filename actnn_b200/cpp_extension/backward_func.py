@@ -76,11 +76,12 @@ def channels_last_pays(input, weight, groups) -> bool:
     B200, float16, forward + backward: 3x3, 256 x 64 x 56 x 56: 742 us on NCHW, 230 on NHWC operands, 31
     per converted tensor; 256 x 256 x 28 x 28: 920 against 509.  1x1 convolutions are matrix products in
     either layout (188 against 157, less than the conversions cost) and stay; so do channel counts that
-    NHWC kernels cannot read in 16-byte vectors, grouped convolutions and float32, whose NCHW path
-    does not go through the same kernels.  Small layers are paced by the host, to which the library's own
-    conversions are cheaper than seven calls: convolution + ReLU, forward + backward, 128 x 64 x 28 x 28 (6.4 M elements)
-    265 us on NCHW against 288, 12.8 M elements 277 against 285; from 25 M elements on the conversions are GPU time
-    (bottleneck block at batch 256: 253 us of cuDNN's against 93)."""
+    NHWC kernels cannot read in 16-byte vectors, and grouped convolutions.  float32 stays because the transpose is written
+    for 16-bit elements and no case calls for another: its convolutions are converted by cuDNN, too, but in the classifier of
+    32 x 32 images that is 122 of 1019 us on the GPU in a step of 2446 that waits for the host.  Small layers are paced
+    by the host, to which the library's own conversions are cheaper than seven calls: convolution + ReLU, forward +
+    backward, 128 x 64 x 28 x 28 (6.4 M elements) 265 us on NCHW against 288, 12.8 M elements 277 against 285;
+    from 25 M elements on the conversions are GPU time (bottleneck block at batch 256: 253 us of cuDNN's against 93)."""
     return (input.dim() == 4 and input.is_cuda and input.dtype in (torch.float16, torch.bfloat16)
             and weight.dtype == input.dtype and groups == 1 and weight.shape[2] * weight.shape[3] > 1
             and weight.shape[0] % 8 == 0 and weight.shape[1] % 8 == 0 and input.shape[1] == weight.shape[1]

@@ -19,9 +19,10 @@
 //   apply   reads the codes and dy again and writes dx, walking the samples backwards so that it
 //           starts with what the reduce left in the L2.
 // Per element of a 16-bit activation that is 2 + b/8 bytes for the reduce and 4 + b/8 for the apply,
-// against 2 (decode) + 4 + 6.  What bounds it now is instruction issue (about 430 instructions a
-// bundle of 1024 elements, some 200 of them decoding), not memory: bringing dy and the words through a
-// ring of bulk copies in shared memory measured the same or slower (42.0 / 40.6 us with 3 stages).
+// against 2 (decode) + 4 + 6.  The apply moves 0.83 of the copy rate, the reduce 0.53: it is bound by its instructions
+// (393 a bundle of 1024 elements, some 200 of them decoding; issue slots 57 % busy at 16 warps an SM), not by
+// memory latency: bringing dy and the words through a ring of bulk copies in shared memory measured the same or
+// slower (42.0 / 40.6 us with 3 stages).
 // float16, 256 x 64 x 56 x 56: decode 24.9 + reduce 40.9 + apply 40.5 us -> 37.2 + 3.2 + 40.1.
 #include "column.cuh"
 
@@ -574,9 +575,9 @@ extern "C" int actnn_batch_norm_codes_forward(const void* x, const void* group_m
   const ColumnShape stats = bn_stats_shape(N, C, HW, al, es);
   if (!group_mn && workspace_bytes < bn_partial_bytes(stats, bn) + 2 * bn_range_bytes(N, F, es))
     return ACTNN_ERR_CAPACITY;
-  const BnForward f{group_mn, group_mx, (unsigned*)ticket, weight, bias, running_mean, running_var, save_mean, save_invstd, packed, bits_out, scale, mn_out,
-                    word_offsets_out, C_out, (float)momentum, (float)eps, range_factor, initial_bits, stochastic,
-                    target, seed, offset};
+  const BnForward f{group_mn, group_mx, (unsigned*)ticket, weight, bias, running_mean, running_var, save_mean,
+                    save_invstd, packed, bits_out, scale, mn_out, word_offsets_out, C_out, (float)momentum, (float)eps,
+                    range_factor, initial_bits, stochastic, target, seed, offset};
   cudaStream_t s = (cudaStream_t)stream;
   const bool edge = al != kOct || F % kGroup != 0;
 #define ACTNN_FWD(T, ST, SUB, EDGE) return launch_forward<T, ST, SUB, EDGE>(x, y, f, stats, sh, bn, workspace, s)

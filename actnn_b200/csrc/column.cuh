@@ -224,9 +224,9 @@ ACTNN_DEV void pack_column_bundle(const Oct<T> (&x)[kBundle], const Oct<T> (&nz)
   }
 }
 
-// Scale, stochastic rounding and pack of a column; each(n, octets) sees every sample's octets on the way.  Eight samples at a time: lane 4i + g prepares group g of
-// the i-th of them (one division per lane for eight bundles).  The noise octets are formed before
-// the dispatch on the width, so the eight width variants stay short.
+// Scale, stochastic rounding and pack of a column; each(n, octets) sees every sample's octets on the way.
+// Eight samples at a time: lane 4i + g prepares group g of the i-th of them (one division per lane for eight
+// bundles).  The noise octets are formed before the dispatch on the width, so the eight width variants stay short.
 template <typename T, typename ST, bool PHILOX, bool EDGE, typename Each>
 ACTNN_DEV void pack_column(const T* __restrict__ data, const ColumnShape& sh, const ColumnTask& t,
                            const ColumnOctets<EDGE>& oct, const T* __restrict__ mn, const T* __restrict__ mx,

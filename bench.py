@@ -42,6 +42,7 @@ sample: no data-path collective); value = all ranks' bytes / max-over-ranks time
 from __future__ import annotations
 
 import argparse
+import ctypes
 import json
 import os
 import sys
@@ -881,6 +882,36 @@ def run_profile(args):
         x.data_ptr(), py.data_ptr(), pidx.data_ptr(), pn, pc, ph, pw, 3, 3, 2, 2, 1, 1, 1, 1, F16, st)
     calls["max_pool_backward"] = lambda: lib.actnn_max_pool2d_backward(
         py.data_ptr(), pidx.data_ptr(), out.data_ptr(), pn, pc, ph, pw, 3, 3, 2, 2, 1, 1, 1, 1, F16, st)
+    # the column kernels: samples that are not whole groups (eight elements fewer), batch norm on the codes
+    # (16-bit types: their float32 form stores bfloat16 statistics, which the buffers above are not)
+    if F16 != _lib.F32:
+        f = G * gs - 8
+        calls["compress_mixed_samples"] = lambda: lib.actnn_compress_mixed_samples(
+            x.data_ptr(), pm.data_ptr(), scale.data_ptr(), mn.data_ptr(), bt2.data_ptr(), offs2.data_ptr(), c_out.data_ptr(),
+            ws_cm.data_ptr(), ws_cm_bytes, N, f, F16, F16, gs / 784.0, 9 / 4, None, 8, float(2 * N), 1, None, 1, 0, st)
+        calls["unpack_mixed_samples"] = lambda: lib.actnn_unpack_mixed_samples(
+            pm.data_ptr(), bt.data_ptr(), offs.data_ptr(), scale.data_ptr(), mn.data_ptr(), out.data_ptr(), N, f, F16, F16, st)
+        cc_bytes = ctypes.c_int64(0)
+        lib.actnn_batch_norm_codes_workspace(N, bn_c, bn_hw, F16, ctypes.addressof(cc_bytes))
+        cc_ws = torch.empty(cc_bytes.value, dtype=torch.uint8, device=dev)
+        ticket = torch.zeros(256, dtype=torch.uint8, device=dev)
+        calls["batch_norm_codes_forward"] = lambda: lib.actnn_batch_norm_codes_forward(
+            x.data_ptr(), None, None, w.data_ptr(), bvec.data_ptr(), rm.data_ptr(), rv.data_ptr(), out.data_ptr(),
+            sm.data_ptr(), si.data_ptr(), pm.data_ptr(), scale.data_ptr(), mn.data_ptr(), bt2.data_ptr(), offs2.data_ptr(),
+            c_out.data_ptr(), N, bn_c, bn_hw, 0.1, 1e-5, F16, F16, gs / 784.0, 8, float(2 * N), 1, 1, 0, ticket.data_ptr(),
+            cc_ws.data_ptr(), cc_bytes.value, st)
+        calls["batch_norm_codes_backward"] = lambda: lib.actnn_batch_norm_codes_backward(
+            pm.data_ptr(), bt.data_ptr(), offs.data_ptr(), scale.data_ptr(), mn.data_ptr(), dy.data_ptr(), w.data_ptr(),
+            sm.data_ptr(), si.data_ptr(), out.data_ptr(), gw.data_ptr(), gb.data_ptr(), N, bn_c, bn_hw, F16, F16,
+            cc_ws.data_ptr(), cc_bytes.value, st)
+        calls["transpose16"] = lambda: lib.actnn_transpose16(x.data_ptr(), out.data_ptr(), N, bn_c, bn_hw, st)
+        for layers in (2, 4, 54):                                        # of 256 samples each
+            c_layers = torch.exp(torch.randn(layers, 256, device=dev))
+            c_ptrs = (ctypes.c_uint64 * layers)(*[c.data_ptr() for c in c_layers])
+            c_dims, sums = (ctypes.c_int32 * layers)(*[200704] * layers), torch.empty(layers, dtype=torch.int32, device=dev)
+            calls["allocate_layers_%d" % layers] = lambda n=layers, p=c_ptrs, d=c_dims, o=sums, _keep=c_layers: \
+                lib.actnn_allocate_layers(ctypes.addressof(p), ctypes.addressof(d), n, 256, 8, 2.0 * 256 * sum(d),
+                                          o.data_ptr(), st)
     calls["max_pool_forward"]()
     calls["batch_norm_forward"]()
     torch.cuda.synchronize()

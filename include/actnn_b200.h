@@ -279,7 +279,8 @@ int actnn_batch_norm_codes_workspace(int64_t N, int64_t C, int64_t HW, int dtype
  * actnn_batch_norm_stats_minimax wrote; else both NULL) save_mean and save_invstd are inputs, too, and the running
  * statistics are left alone.  `ticket`: as in actnn_compress_mixed_prestat_kept. */
 int actnn_batch_norm_codes_forward(const void* x, const void* group_mn, const void* group_mx, const float* weight,
-                                   const float* bias, float* running_mean, float* running_var, void* y, float* save_mean, float* save_invstd, int32_t* packed,
+                                   const float* bias, float* running_mean, float* running_var, void* y,
+                                   float* save_mean, float* save_invstd, int32_t* packed,
                                    void* scale, void* mn_out, int32_t* bits_out, int64_t* word_offsets_out,
                                    float* C_out, int64_t N, int64_t C, int64_t HW, double momentum, double eps,
                                    int dtype, int stat_dtype, float range_factor, int initial_bits, double target,
