@@ -6,7 +6,6 @@ is raised.
 """
 from __future__ import annotations
 
-import contextlib
 import ctypes
 import os
 from ctypes import c_char_p, c_double, c_float, c_int, c_int64, c_uint64, c_void_p
@@ -122,9 +121,13 @@ def ticket(device: torch.device) -> torch.Tensor:
     could not be shared with a graph: made during a capture it is only cleared when that graph runs, and a
     replay on another stream would use it at the same time."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    with torch.cuda.device(idx) if idx != torch.cuda.current_device() else contextlib.nullcontext():
-        if torch.cuda.is_current_stream_capturing():
-            return torch.zeros(256, dtype=torch.uint8, device=device)
+    if idx == torch.cuda.current_device():
+        capturing = torch.cuda.is_current_stream_capturing()
+    else:
+        with torch.cuda.device(idx):
+            capturing = torch.cuda.is_current_stream_capturing()
+    if capturing:
+        return torch.zeros(256, dtype=torch.uint8, device=device)
     key = (idx, stream_of_index(idx))
     buf = _tickets.get(key)
     if buf is None:
