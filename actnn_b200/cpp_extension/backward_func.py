@@ -326,26 +326,27 @@ def batch_norm_stats_minimax(input, weight, bias, running_mean, running_var, mom
     when given; ``out``: optional float32 buffer of >= 2 * C elements for mean then invstd."""
     if not input.is_cuda or not input.is_contiguous() or input.dim() < 2:
         return None
-    N, C, HW = _bn_dims(input)
-    lib = _lib.load()
-    nbytes = lib.actnn_batch_norm_stats_minimax_workspace(N, C, HW)
-    if nbytes < 0:
-        return None
     for t in (running_mean, running_var):
         if t is not None and (t.dtype != torch.float32 or not t.is_contiguous()):
             return None
-    G = C * HW // 256
+    nat = _lib.native()
+    if nat:
+        return nat.batch_norm_stats_minimax(input, running_mean, running_var, momentum, eps, out)
+    N, C, HW = _bn_dims(input)
     dev = input.device
+    nbytes = _lib.load().actnn_batch_norm_stats_minimax_workspace(N, C, HW)
+    if nbytes < 0:
+        return None
+    if out is not None and (out.dtype != torch.float32 or not out.is_contiguous() or out.numel() < 2 * C or out.device != dev):
+        raise RuntimeError("batch_norm_stats_minimax: out must be a contiguous float32 tensor of >= 2*C elements")
+    G = C * HW // 256
     mn = torch.empty((N, G, 1), dtype=input.dtype, device=dev)
     mx = torch.empty((N, G, 1), dtype=input.dtype, device=dev)
     if out is None:
         out = torch.empty(2 * C, dtype=torch.float32, device=dev)
-    elif out.dtype != torch.float32 or not out.is_contiguous() or out.numel() < 2 * C or out.device != dev:
-        raise RuntimeError("batch_norm_stats_minimax: out must be a contiguous float32 tensor of >= 2*C elements")
-    w32, b32 = _as_f32(weight), _as_f32(bias)
     ws = _lib.scratch(dev, nbytes)
-    _lib.call("actnn_batch_norm_stats_minimax", input, _lib.ptr(input), mn.data_ptr(), mx.data_ptr(), _lib.ptr(w32),
-              _lib.ptr(b32), _lib.ptr(running_mean), _lib.ptr(running_var), out.data_ptr(), out.data_ptr() + 4 * C,
+    _lib.call("actnn_batch_norm_stats_minimax", input, _lib.ptr(input), mn.data_ptr(), mx.data_ptr(), 0, 0,
+              _lib.ptr(running_mean), _lib.ptr(running_var), out.data_ptr(), out.data_ptr() + 4 * C,
               N, C, HW, float(momentum), float(eps), _lib.dtype_id(input.dtype), ws.data_ptr(), nbytes,
               _lib.stream_of(input))
     flat = out.view(-1)

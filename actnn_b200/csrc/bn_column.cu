@@ -5,8 +5,6 @@
 //   finish  one warp per channel: mean, inverse deviation, running statistics, coefficients;
 //   (allocation of the widths, stats.cu)
 //   pack    codes and y from the same registers.
-// (Statistics and ranges of maps of 256 and more whole groups come from bn_stats_minimax_kernel in batch_norm.cu
-// instead, which the synchronised batch norm shares; see the binding.)
 // 4 + b/8 + 2 bytes an element for 16-bit types; statistics, pack and normalisation as passes of their own read x
 // three times.  float16 256 x 64 x 56 x 56: pack 28.1 + coefficients 1.6 + normalise 32.4 us -> 41.6 us (6.1 TB/s would be
 // 36, the rest is instruction issue); 128 x 256 x 14 x 14, seven launches 34 us -> four 24.6 us.
@@ -478,20 +476,26 @@ int64_t bn_range_bytes(int64_t N, int64_t F, int elem_size) {
   return (N * ((F + kGroup - 1) / kGroup) * elem_size + 255) / 256 * 256;
 }
 
+template <typename T, int SUB, bool EDGE>
+int launch_stats(const T* x, T* mn, T* mx, float* running_mean, float* running_var, float* save_mean, float* save_invstd,
+                 float momentum, float eps, const ColumnShape& sh, const BnColumns& bn, float2* partial, cudaStream_t s) {
+  bn_column_stats_kernel<T, SUB, EDGE><<<column_grid(sh), kColThreads, 0, s>>>(x, sh, bn, mn, mx, partial);
+  if (int st = check_launch()) return st;
+  bn_column_stats_finish_kernel<T><<<(bn.C + kColThreads / 32 - 1) / (kColThreads / 32), kColThreads, 0, s>>>(
+      partial, sh, bn, x, running_mean, running_var, save_mean, save_invstd, momentum, eps);
+  return check_launch();
+}
+
 template <typename T, typename ST, int SUB, bool EDGE>
 int launch_forward(const void* x, void* y, const BnForward& f, const ColumnShape& stats, const ColumnShape& sh,
                    const BnColumns& bn, void* workspace, cudaStream_t s) {
   const T *mn = (const T*)f.group_mn, *mx = (const T*)f.group_mx;
   if (!mn) {                                           // else ranges and statistics come from a pass before this call
-    float2* partial = (float2*)workspace;
-    T* own_mn = (T*)((char*)partial + bn_partial_bytes(stats, bn));
+    T* own_mn = (T*)((char*)workspace + bn_partial_bytes(stats, bn));
     T* own_mx = (T*)((char*)own_mn + bn_range_bytes(sh.N, sh.F, sizeof(T)));
-    bn_column_stats_kernel<T, SUB, EDGE><<<column_grid(stats), kColThreads, 0, s>>>((const T*)x, stats, bn, own_mn, own_mx,
-                                                                                   partial);
-    if (int st = check_launch()) return st;
-    bn_column_stats_finish_kernel<T><<<(bn.C + kColThreads / 32 - 1) / (kColThreads / 32), kColThreads, 0, s>>>(
-        partial, stats, bn, (const T*)x, f.running_mean, f.running_var, f.save_mean, f.save_invstd, f.momentum, f.eps);
-    if (int st = check_launch()) return st;
+    if (int st = launch_stats<T, SUB, EDGE>((const T*)x, own_mn, own_mx, f.running_mean, f.running_var, f.save_mean,
+                                            f.save_invstd, f.momentum, f.eps, stats, bn, (float2*)workspace, s))
+      return st;
     mn = own_mn;
     mx = own_mx;
   }
@@ -545,6 +549,45 @@ extern "C" int actnn_batch_norm_codes_workspace(int64_t N, int64_t C, int64_t HW
   *bytes = bn_coef_bytes(C) + max(bn_partial_bytes(sh, bn), bn_partial_bytes(stats, bn)) +
            2 * bn_range_bytes(N, C * HW, dtype_size(dtype));                       // ranges: forward only
   return ACTNN_OK;
+}
+
+// The statistics pass by itself, for maps of whole octets and samples of whole groups.
+// (Until it ran on columns it took tasks of up to eight groups, 15.6 instructions an element for their two channels:
+// float16 256 x 64 x 56 x 56 24.1 us against 20.1, 256 x 512 x 28 x 28 and two of 256 x 128 x 28 x 28 99.5 against 49.4.)
+extern "C" int64_t actnn_batch_norm_stats_minimax_workspace(int64_t N, int64_t C, int64_t HW) {
+  constexpr int64_t k31 = (int64_t)1 << 31;
+  if (N <= 0 || C <= 0 || N >= k31 || C >= k31 || HW >= k31 || HW < kGroup || HW % kOct != 0 || N * C >= k31 ||
+      N * C * HW >= ((int64_t)1 << 40) || C * HW % kGroup != 0 || C * HW >= 2 * k31 - kBundle * kGroup)
+    return -1;
+  const int64_t P = (C * HW / kGroup + kBundle - 1) / kBundle;
+  return (P * N * bn_columns(C, HW).kmax * (int64_t)sizeof(float2) + 255) / 256 * 256;  // a partial sum per sample, the most there are
+}
+
+extern "C" int actnn_batch_norm_stats_minimax(const void* x, void* mn, void* mx, const float* weight, const float* bias,
+                                              float* running_mean, float* running_var, float* save_mean,
+                                              float* save_invstd, int64_t N, int64_t C, int64_t HW, double momentum,
+                                              double eps, int dtype, void* workspace, int64_t workspace_bytes,
+                                              actnn_stream_t stream) {
+  (void)weight;
+  (void)bias;
+  if (dtype < ACTNN_F32 || dtype > ACTNN_BF16) return ACTNN_ERR_DTYPE;
+  const int64_t need = actnn_batch_norm_stats_minimax_workspace(N, C, HW);
+  if (need < 0) return ACTNN_ERR_SHAPE;
+  if (!x || !mn || !mx || !save_mean || !save_invstd || !workspace) return ACTNN_ERR_NULL;
+  if (workspace_bytes < need) return ACTNN_ERR_CAPACITY;
+  if (!aligned(x, dtype == ACTNN_F32 ? 32 : 16) || !aligned(workspace, 16)) return ACTNN_ERR_ALIGN;
+  const BnColumns bn = bn_columns(C, HW);
+  const ColumnShape sh = bn_stats_shape(N, C, HW, kOct, dtype_size(dtype));
+  cudaStream_t s = (cudaStream_t)stream;
+#define ACTNN_STATS(T)                                                                                             \
+  return launch_stats<T, 8, false>((const T*)x, (T*)mn, (T*)mx, running_mean, running_var, save_mean, save_invstd, \
+                                   (float)momentum, (float)eps, sh, bn, (float2*)workspace, s)
+  switch (dtype) {
+    case ACTNN_F32: ACTNN_STATS(float);
+    case ACTNN_F16: ACTNN_STATS(__half);
+    default: ACTNN_STATS(__nv_bfloat16);
+  }
+#undef ACTNN_STATS
 }
 
 extern "C" int actnn_batch_norm_codes_forward(const void* x, const void* group_mn, const void* group_mx,

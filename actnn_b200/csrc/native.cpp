@@ -131,6 +131,29 @@ py::tuple compress_single(const Tensor& data, int64_t bits, bool stochastic, boo
 }
 
 // ---------------------------------------------------------------------------------------- batch norm
+// (group minima, group maxima, mean, invstd), or None for a geometry that is not covered; `out`: room for the last two
+py::object batch_norm_stats_minimax(const Tensor& x, const OptTensor& running_mean, const OptTensor& running_var,
+                                    double momentum, double eps, const OptTensor& out) {
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t N = x.size(0), C = x.size(1), HW = N && C ? x.numel() / N / C : 0;
+  const int64_t bytes = actnn_batch_norm_stats_minimax_workspace(N, C, HW);
+  if (bytes < 0) return py::none();
+  TORCH_CHECK(!out.has_value() || (out->scalar_type() == at::kFloat && out->is_contiguous() && out->numel() >= 2 * C &&
+                                   out->device() == x.device()),
+              "batch_norm_stats_minimax: out must be a contiguous float32 tensor of >= 2*C elements");
+  const auto t = x.scalar_type();
+  Tensor mn = make({N, C * HW / 256, 1}, t, x), mx = make({N, C * HW / 256, 1}, t, x);
+  const Tensor both = out.has_value() ? out->view(-1) : make({2 * C}, at::kFloat, x);
+  Tensor mean = both.narrow(0, 0, C), invstd = both.narrow(0, C, C);
+  Tensor ws = make({bytes}, at::kByte, x);
+  check(actnn_batch_norm_stats_minimax(x.data_ptr(), mn.data_ptr(), mx.data_ptr(), nullptr, nullptr,
+                                       (float*)ptr(running_mean), (float*)ptr(running_var), mean.data_ptr<float>(),
+                                       invstd.data_ptr<float>(), N, C, HW, momentum, eps, dtype_id(t), ws.data_ptr(),
+                                       bytes, stream()),
+        "actnn_batch_norm_stats_minimax");
+  return py::make_tuple(mn, mx, mean, invstd);
+}
+
 // (y, packed, bits, scale, min, mean, invstd, word_offsets), or None for a geometry that is not covered
 py::object batch_norm_forward(const Tensor& x, const OptTensor& weight, const OptTensor& bias, const OptTensor& running_mean,
                               const OptTensor& running_var, double momentum, double eps, int64_t target_bits,
@@ -328,6 +351,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("compress_mixed", &compress_mixed);
   m.def("unpack_mixed", &unpack_mixed);
   m.def("compress_single", &compress_single);
+  m.def("batch_norm_stats_minimax", &batch_norm_stats_minimax);
   m.def("batch_norm_forward", &batch_norm_forward);
   m.def("batch_norm_backward", &batch_norm_backward);
   m.def("transpose16", &transpose16);

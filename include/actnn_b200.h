@@ -251,7 +251,7 @@ int actnn_compress_mixed_static(const void* data, int32_t* packed, void* scale, 
  *               flattened samples (what actnn_minimax returns for the same tensor)
  *   save_mean, save_invstd  float32 [C]; running_mean / running_var (may be NULL) are updated
  *               with `momentum` exactly as actnn_batch_norm_forward does
- *   weight, bias  only used to fill the coefficients kept in the workspace; may be NULL
+ *   weight, bias  not read; may be NULL
  * Geometry: HW % 8 == 0, HW >= 256 and C * HW % 256 == 0 (every layer of a ResNet down to
  * 16x16 maps); anything else returns ACTNN_ERR_SHAPE and the caller takes the two-read path.
  * actnn_batch_norm_stats_minimax_workspace returns the scratch bytes (-1: unsupported). */
