@@ -314,6 +314,7 @@ bn_codes_reduce_kernel(const int32_t* __restrict__ packed, const int32_t* __rest
   if (!t.valid) return;
   const ColumnChannels<SUB> cc(sh, bn, t, lane);
   const TransposePlan plan = make_transpose_plan(lane);
+  const WordOrder<T> order(lane);
   float neg_mean[kBundle][NS];
   float2 sg[kBundle][NS], sgx[kBundle][NS];
 #pragma unroll
@@ -348,12 +349,12 @@ bn_codes_reduce_kernel(const int32_t* __restrict__ packed, const int32_t* __rest
     const int nl = min(32, t.n1 - nb);
     ColumnStream st;
     st.open(t, nb + lane, lane < nl, bits, word_offsets);
-    BundleWords next = st.fetch<ST>(t, sh.G, nb, 0, packed, scale, mn, lane);
+    BundleWords next = st.fetch<T, ST>(t, order, sh.G, nb, 0, packed, scale, mn, lane);
     for (int i = 0; i < nl; ++i) {
       const BundleWords cur = next;
       Oct<T> g[kBundle];
       oct.template load<T>(dy + (int64_t)(nb + i) * sh.F, g);
-      if (i + 1 < nl) next = st.fetch<ST>(t, sh.G, nb + i + 1, i + 1, packed, scale, mn, lane);
+      if (i + 1 < nl) next = st.fetch<T, ST>(t, order, sh.G, nb + i + 1, i + 1, packed, scale, mn, lane);
       decode_column<T>(cur, t.count, plan, lane, [&](int gi, const Oct<T>& x) { add(gi, x, g[gi]); });
     }
   }
@@ -391,6 +392,7 @@ bn_codes_apply_kernel(const int32_t* __restrict__ packed, const int32_t* __restr
   const ColumnOctets<EDGE> oct(sh, t, lane);
   const ColumnChannels<SUB> cc(sh, bn, t, lane);
   const TransposePlan plan = make_transpose_plan(lane);
+  const WordOrder<T> order(lane);
   float4 kf[kBundle][NS];                              // (-mean, weight * invstd, -mean_dy, -q)
 #pragma unroll
   for (int gi = 0; gi < kBundle; ++gi) {
@@ -424,12 +426,12 @@ bn_codes_apply_kernel(const int32_t* __restrict__ packed, const int32_t* __restr
     const int top = t.n1 - 1 - kb;
     ColumnStream st;
     st.open(t, top - lane, lane < nl, bits, word_offsets);
-    BundleWords next = st.fetch<ST>(t, sh.G, top, 0, packed, scale, mn, lane);
+    BundleWords next = st.fetch<T, ST>(t, order, sh.G, top, 0, packed, scale, mn, lane);
     for (int i = 0; i < nl; ++i) {
       const BundleWords cur = next;
       Oct<T> g[kBundle];
       oct.template load<T>(dy + (int64_t)(top - i) * sh.F, g);
-      if (i + 1 < nl) next = st.fetch<ST>(t, sh.G, top - i - 1, i + 1, packed, scale, mn, lane);
+      if (i + 1 < nl) next = st.fetch<T, ST>(t, order, sh.G, top - i - 1, i + 1, packed, scale, mn, lane);
       T* sample = dx + (int64_t)(top - i) * sh.F;
       decode_column<T>(cur, t.count, plan, lane,
                        [&](int gi, const Oct<T>& x) { oct.template store<T>(sample, gi, gradient(gi, x, g[gi])); });

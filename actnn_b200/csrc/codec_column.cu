@@ -64,14 +64,15 @@ column_unpack_kernel(const int32_t* __restrict__ packed, const int32_t* __restri
   if (!t.valid) return;
   const ColumnOctets<EDGE> oct(sh, t, lane);
   const TransposePlan plan = make_transpose_plan(lane);
+  const WordOrder<T> order(lane);
   for (int nb = t.n0; nb < t.n1; nb += 32) {
     const int nl = min(32, t.n1 - nb);
     ColumnStream st;
     st.open(t, nb + lane, lane < nl, bits, word_offsets);
-    BundleWords next = st.fetch<ST>(t, sh.G, nb, 0, packed, scale, mn, lane);
+    BundleWords next = st.fetch<T, ST>(t, order, sh.G, nb, 0, packed, scale, mn, lane);
     for (int i = 0; i < nl; ++i) {
       const BundleWords cur = next;
-      if (i + 1 < nl) next = st.fetch<ST>(t, sh.G, nb + i + 1, i + 1, packed, scale, mn, lane);
+      if (i + 1 < nl) next = st.fetch<T, ST>(t, order, sh.G, nb + i + 1, i + 1, packed, scale, mn, lane);
       T* sample = out + (int64_t)(nb + i) * sh.F;
       decode_column<T>(cur, t.count, plan, lane,
                        [&](int gi, const Oct<T>& x) { oct.template store<T>(sample, gi, x); });

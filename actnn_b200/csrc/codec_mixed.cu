@@ -349,6 +349,7 @@ unpack_mixed_kernel(const int32_t* __restrict__ packed, const int32_t* __restric
   const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
   const TransposePlan plan = make_transpose_plan(lane);
+  const WordOrder<T> order(lane);
 
   // A bundle's input is only b * 128 bytes per warp: issue the loads of DEPTH bundles before
   // decoding the first, so that enough bytes are in flight to cover the memory latency.
@@ -374,10 +375,10 @@ unpack_mixed_kernel(const int32_t* __restrict__ packed, const int32_t* __restric
         const int b = __ldg(bits + c.n);
         if (b >= 1 && b <= 8) t_b[d] = b;
         const int32_t* in = packed + (__ldg(word_offsets + c.n) + (int64_t)c.g0 * 8 * t_b[d]);
-        const int words = c.count * 8 * t_b[d];
+        const int base = order.base(t_b[d]), step = order.step(t_b[d]), words = c.count * 8 * t_b[d];
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          if (k * 32 + lane < words) t_w[d][k] = (uint32_t)__ldg(in + k * 32 + lane);
+          if (k < t_b[d] && base + k * step < words) t_w[d][k] = (uint32_t)__ldg(in + base + k * step);
         if (lane < c.count) {
           t_sc[d] = load_scalar<ST>(scale, c.q0 + lane);
           t_m[d] = load_scalar<ST>(mn, c.q0 + lane);
@@ -468,21 +469,20 @@ ACTNN_DEV void split_group_index(int64_t q, int64_t G, int64_t& n, int64_t& r) {
 #define ACTNN_UNPACK_DIRECT_FROM 6
 #endif
 template <typename T, int B, bool FASTDIV>
-ACTNN_DEV void unpack_flat_bundle(const uint32_t (&words)[B], float sc_l, float m_l, uint32_t t01_l, uint32_t t23_l,
-                                  int first, int64_t q, T* __restrict__ out, const TransposePlan& plan, int lane) {
+ACTNN_DEV void unpack_flat_bundle(const uint32_t (&words)[B], float sc_l, float m_l, int first,
+                                  int64_t q, T* __restrict__ out, const TransposePlan& plan, int lane) {
   // from kDirect bits on every element is computed (a table of 2^B entries no longer fits a warp,
   // or costs more shuffles than the arithmetic)
   constexpr int kDirect = FASTDIV ? ACTNN_UNPACK_DIRECT_FROM : 6;
   constexpr int E = 1 << (B < kDirect ? B : 5);        // table entries per group
   constexpr int GPC = (32 / E) < kFlatBundle ? (32 / E) : kFlatBundle;   // groups served by one table
-  constexpr bool PAIRS = sizeof(T) == 2 && B <= 2;
   uint32_t S[B];
 #pragma unroll
   for (int k = 0; k < B; ++k) S[k] = warp_transpose32(words[k], plan);
   uint32_t entry = 0u;
 #pragma unroll
   for (int gi = 0; gi < kFlatBundle; ++gi) {
-    if constexpr (!PAIRS && B < kDirect) {
+    if constexpr (B < kDirect) {
       if (gi % GPC == 0) {                               // (re)build the table for groups gi .. gi+GPC-1
         const int g = first + ((gi + lane / E) & (kFlatBundle - 1));
         const float sc = __shfl_sync(kFull, sc_l, g), m = __shfl_sync(kFull, m_l, g);
@@ -496,129 +496,132 @@ ACTNN_DEV void unpack_flat_bundle(const uint32_t (&words)[B], float sc_l, float 
     if (gi == 3) { lo = get_bits<3 * 8 * B, (8 * B < 32 ? 8 * B : 32)>(S); if constexpr (8 * B > 32) hi = get_bits<3 * 8 * B + 32, 8 * B - 32>(S); }
     Oct<T> o;
     uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-    if constexpr (PAIRS) {
-      const uint32_t t01 = __shfl_sync(kFull, t01_l, first + gi);
-      const uint32_t t23 = B == 2 ? __shfl_sync(kFull, t23_l, first + gi) : t01;
+    uint32_t v[8];
+    const uint32_t S2[2] = {lo, hi};
+    uint32_t code[8];
+    get_codes<B, 0>(S2, code);
+    if constexpr (B < kDirect) {
+      const int base = (gi % GPC) * E;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {                      // four elements per step
-        const uint32_t y = spread_codes_to_bytes<B>((lo >> (4 * B * h)) & ((1u << (4 * B)) - 1u));
-        const uint32_t sel = y * 0x22u + 0x10101010u;    // byte pair (2c, 2c+1) per element
-        ow[2 * h] = __byte_perm(t01, t23, sel);
-        ow[2 * h + 1] = __byte_perm(t01, t23, sel >> 16);
-      }
+      for (int j = 0; j < 8; ++j) v[j] = __shfl_sync(kFull, entry, base + (int)code[j]);
     } else {
-      uint32_t v[8];
-      const uint32_t S2[2] = {lo, hi};
-      uint32_t code[8];
-      get_codes<B, 0>(S2, code);
-      if constexpr (B < kDirect) {
-        const int base = (gi % GPC) * E;
+      const float sc = __shfl_sync(kFull, sc_l, first + gi), m = __shfl_sync(kFull, m_l, first + gi);
+      float y = 0.f;
+      if (FASTDIV && group_reciprocal(sc, y)) {                 // warp-uniform: one scale per group
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __shfl_sync(kFull, entry, base + (int)code[j]);
-      } else {
-        const float sc = __shfl_sync(kFull, sc_l, first + gi), m = __shfl_sync(kFull, m_l, first + gi);
-        float y = 0.f;
-        if (FASTDIV && group_reciprocal(sc, y)) {                 // warp-uniform: one scale per group
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = dequant_bits_recip<T>((float)code[j], sc, y, m);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = dequant_bits<T>((float)code[j], sc, m);
-        }
-      }
-      if constexpr (sizeof(T) == 4) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) ow[j] = v[j];
+        for (int j = 0; j < 8; ++j) v[j] = dequant_bits_recip<T>((float)code[j], sc, y, m);
       } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) ow[k] = v[2 * k] | (v[2 * k + 1] << 16);
+        for (int j = 0; j < 8; ++j) v[j] = dequant_bits<T>((float)code[j], sc, m);
       }
+    }
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ow[j] = v[j];
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ow[k] = v[2 * k] | (v[2 * k + 1] << 16);
     }
     store_oct_streaming<T>(out + (q + gi) * kGroup + lane * kOct, o);
   }
 }
 
-// A run of bundles k0 .. k1-1 of one width B (see pack_flat_run): the B words per lane of
-// bundle k+1 are requested before bundle k is decoded.  `in` points at this lane's first word
-// of bundle k0; a bundle is 32 * B words.
+// The bytes of the values of codes 0..7 (2^b are used) of one group.
+template <typename T> ACTNN_DEV ByteTable byte_table(int b, float sc, float m) {
+  float y = 0.f;
+  const bool fast = group_reciprocal(sc, y);
+  auto pair = [&](int c) {
+    const uint32_t v0 = fast ? dequant_bits_recip<T>((float)c, sc, y, m) : dequant_bits<T>((float)c, sc, m);
+    const uint32_t v1 = fast ? dequant_bits_recip<T>((float)(c + 1), sc, y, m) : dequant_bits<T>((float)(c + 1), sc, m);
+    return v0 | (v1 << 16);
+  };
+  ByteTable t = {0u, 0u, 0u, 0u};
+  const uint32_t p01 = pair(0), p23 = pair(2);
+  t.lo0 = select_bytes(p01, p23, 0x6420u);
+  t.hi0 = select_bytes(p01, p23, 0x7531u);
+  if (b == 3) {
+    const uint32_t p45 = pair(4), p67 = pair(6);
+    t.lo1 = select_bytes(p45, p67, 0x6420u);
+    t.hi1 = select_bytes(p45, p67, 0x7531u);
+  }
+  return t;
+}
+
+// A run of bundles k0 .. k1-1 of one width B (see pack_flat_run), `in` its first word; a bundle is 32 * B words.
+// Widths whose codes the transpose leaves in nibbles: two bundles at a time are decoded as straight-line code
+// (four, at 1 and 2 bits: 37.5 against 37.1 us, 512 x 784 groups of bfloat16; four at 3 bits, too: 43.1; four blocks an
+// SM instead of three: 41.0).
+// The words of the next ones are requested before, the transposes of a pass are issued together, and only the
+// stores are predicated, so the scheduler always has independent work.  A run of an odd number of bundles transposes
+// a few zero words.
+template <typename T, int B>
+ACTNN_DEV void unpack_flat_nibbles(int k0, int k1, int64_t q0, const int32_t* __restrict__ in,
+                                   const WordOrder<T>& order, const ByteTable& mine, T* __restrict__ out,
+                                   const TransposePlan& plan) {
+  constexpr int PER = 2, kBundles = kFlatGroups / kFlatBundle;
+  const int lane = order.lane, step = order.step(B);
+  in += order.base(B);
+  uint32_t S[PER][B], next[PER][B];
+  auto load = [&](uint32_t (&w)[PER][B], int k) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+#pragma unroll
+      for (int kk = 0; kk < B; ++kk) w[i][kk] = k + i < k1 ? (uint32_t)__ldg(in + (k - k0 + i) * (32 * B) + kk * step) : 0u;
+    }
+  };
+  load(S, k0);
+  // kept rolled: the straight-line body of one pass is long, and the instruction cache is shared by all widths
+#pragma unroll 1
+  for (int kb = k0; kb < k1; kb += PER) {
+    load(next, kb + PER);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+#pragma unroll
+      for (int kk = 0; kk < B; ++kk) S[i][kk] = warp_transpose32(S[i][kk], plan);
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const bool live = kb + i < k1;
+      const int first = (kb + i < kBundles ? kb + i : kBundles - 1) * kFlatBundle;      // a lane of this warp in any case
+#pragma unroll
+      for (int gi = 0; gi < kFlatBundle; ++gi) {
+        ByteTable t;
+        t.lo0 = t.lo1 = __shfl_sync(kFull, mine.lo0, first + gi);
+        t.hi0 = t.hi1 = __shfl_sync(kFull, mine.hi0, first + gi);
+        if constexpr (B == 3) {
+          t.lo1 = __shfl_sync(kFull, mine.lo1, first + gi);
+          t.hi1 = __shfl_sync(kFull, mine.hi1, first + gi);
+        }
+        const Oct<T> o = decode_nibbles<T>(group_nibbles<B>(S[i], gi), t);
+        if (live) store_oct_streaming<T>(out + (q0 + (kb + i) * kFlatBundle + gi) * kGroup + lane * kOct, o);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+#pragma unroll
+      for (int kk = 0; kk < B; ++kk) S[i][kk] = next[i][kk];
+    }
+  }
+}
+
+// Other widths and float32: the B words per lane of bundle k+1 are requested before bundle k is decoded.
 template <typename T, int B, bool FASTDIV>
 ACTNN_DEV void unpack_flat_run(int k0, int k1, int64_t q0, const int32_t* __restrict__ in, float sc_l, float m_l,
-                               uint32_t t01_l, uint32_t t23_l, T* __restrict__ out, const TransposePlan& plan,
-                               int lane) {
+                               T* __restrict__ out, const TransposePlan& plan, int lane) {
   auto load = [&](uint32_t (&w)[B], const int32_t* p) {
 #pragma unroll
     for (int kk = 0; kk < B; ++kk) w[kk] = (uint32_t)__ldg(p + kk * 32);
   };
-  if constexpr (B <= 2 && sizeof(T) == 2) {
-    // Narrow widths, 16-bit outputs: four bundles at a time are decoded as straight-line code.
-    // The words of up to 8 bundles (8 * B registers) are requested up front (2 KB per warp in
-    // flight instead of 256 bytes), the transposes of four bundles are issued together
-    // (4 * B independent butterfly chains instead of B), and only the stores are predicated, so
-    // the scheduler always has independent work.  A run that is not a multiple of four bundles
-    // transposes a few zero words.
-    constexpr int kHalf = kFlatGroups / kFlatBundle / 2;         // bundles decoded per pass of the loop below
-    uint32_t S[kHalf][B], N2[kHalf][B];
-#pragma unroll
-    for (int i = 0; i < kHalf; ++i) {
-#pragma unroll
-      for (int kk = 0; kk < B; ++kk) {
-        S[i][kk] = (k0 + i < k1) ? (uint32_t)__ldg(in + (i * B + kk) * 32) : 0u;
-        N2[i][kk] = (k0 + kHalf + i < k1) ? (uint32_t)__ldg(in + ((kHalf + i) * B + kk) * 32) : 0u;
-      }
-    }
-    // two passes over the same code (kept rolled: the straight-line body of one pass is already
-    // a few thousand instructions, and the instruction cache is shared by all eight widths)
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      const int kb = k0 + half * kHalf;
-      if (kb >= k1) break;
-#pragma unroll
-      for (int i = 0; i < kHalf; ++i) {
-#pragma unroll
-        for (int kk = 0; kk < B; ++kk) S[i][kk] = warp_transpose32(S[i][kk], plan);
-      }
-#pragma unroll
-      for (int i = 0; i < kHalf; ++i) {
-        const bool live = kb + i < k1;
-        const int first = (kb + i < 2 * kHalf ? kb + i : 2 * kHalf - 1) * kFlatBundle;   // a lane of this warp in any case
-#pragma unroll
-        for (int gi = 0; gi < kFlatBundle; ++gi) {
-          const uint32_t t01 = __shfl_sync(kFull, t01_l, first + gi);
-          const uint32_t t23 = B == 2 ? __shfl_sync(kFull, t23_l, first + gi) : t01;
-          uint32_t lo = 0u;
-          if (gi == 0) lo = get_bits<0 * 8 * B, 8 * B>(S[i]);
-          if (gi == 1) lo = get_bits<1 * 8 * B, 8 * B>(S[i]);
-          if (gi == 2) lo = get_bits<2 * 8 * B, 8 * B>(S[i]);
-          if (gi == 3) lo = get_bits<3 * 8 * B, 8 * B>(S[i]);
-          Oct<T> o;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {                      // four elements per step
-            const uint32_t y = spread_codes_to_bytes<B>((lo >> (4 * B * h)) & ((1u << (4 * B)) - 1u));
-            const uint32_t sel = y * 0x22u + 0x10101010u;    // byte pair (2c, 2c+1) per element
-            o.r[2 * h] = __byte_perm(t01, t23, sel);
-            o.r[2 * h + 1] = __byte_perm(t01, t23, sel >> 16);
-          }
-          if (live) store_oct_streaming<T>(out + (q0 + (kb + i) * kFlatBundle + gi) * kGroup + lane * kOct, o);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < kHalf; ++i) {
-#pragma unroll
-        for (int kk = 0; kk < B; ++kk) S[i][kk] = N2[i][kk];
-      }
-    }
-  } else {
-    uint32_t wa[B], wb[B];
-    load(wa, in);
-    for (int k = k0; k < k1; k += 2) {
-      if (k + 1 < k1) load(wb, in + 32 * B);
-      unpack_flat_bundle<T, B, FASTDIV>(wa, sc_l, m_l, t01_l, t23_l, k * kFlatBundle, q0 + k * kFlatBundle, out, plan, lane);
-      if (k + 1 >= k1) break;
-      if (k + 2 < k1) load(wa, in + 64 * B);
-      unpack_flat_bundle<T, B, FASTDIV>(wb, sc_l, m_l, t01_l, t23_l, (k + 1) * kFlatBundle, q0 + (k + 1) * kFlatBundle, out,
-                               plan, lane);
-      in += 64 * B;
-    }
+  in += lane;
+  uint32_t wa[B], wb[B];
+  load(wa, in);
+  for (int k = k0; k < k1; k += 2) {
+    if (k + 1 < k1) load(wb, in + 32 * B);
+    unpack_flat_bundle<T, B, FASTDIV>(wa, sc_l, m_l, k * kFlatBundle, q0 + k * kFlatBundle, out, plan, lane);
+    if (k + 1 >= k1) break;
+    if (k + 2 < k1) load(wa, in + 64 * B);
+    unpack_flat_bundle<T, B, FASTDIV>(wb, sc_l, m_l, (k + 1) * kFlatBundle, q0 + (k + 1) * kFlatBundle, out, plan, lane);
+    in += 64 * B;
   }
 }
 
@@ -629,6 +632,7 @@ unpack_mixed_flat_kernel(const int32_t* __restrict__ packed, const int32_t* __re
                          const ST* __restrict__ mn, T* __restrict__ out, int64_t Q, int64_t G) {
   const int lane = threadIdx.x & 31;
   const TransposePlan plan = make_transpose_plan(lane);
+  const WordOrder<T> order(lane);
   __shared__ unsigned pool_counters[2];
   FlatPool pool;
   pool.init(pool_counters, (Q + kFlatGroups - 1) / kFlatGroups, ACTNN_UNPACK_SPLIT);
@@ -640,7 +644,7 @@ unpack_mixed_flat_kernel(const int32_t* __restrict__ packed, const int32_t* __re
     int b_l = -1;                                             // past the end of the activation
     int64_t off_l = 0;
     float sc_l = 1.f, m_l = 0.f;
-    uint32_t t01_l = 0u, t23_l = 0u;
+    ByteTable mine = {0u, 0u, 0u, 0u};
     if (q < Q) {
       int64_t n, r;
       split_group_index(q, G, n, r);
@@ -649,16 +653,7 @@ unpack_mixed_flat_kernel(const int32_t* __restrict__ packed, const int32_t* __re
       off_l = __ldg(word_offsets + n) + r * (8 * b_l);
       sc_l = load_scalar<ST>(scale, q);
       m_l = load_scalar<ST>(mn, q);
-      if constexpr (sizeof(T) == 2) {
-        if (b_l == 1 || b_l == 2) {
-          const uint32_t e0 = dequant_bits<T>(0.f, sc_l, m_l), e1 = dequant_bits<T>(1.f, sc_l, m_l);
-          t01_l = e0 | (e1 << 16);
-          if (b_l == 2) {
-            const uint32_t e2 = dequant_bits<T>(2.f, sc_l, m_l), e3 = dequant_bits<T>(3.f, sc_l, m_l);
-            t23_l = e2 | (e3 << 16);
-          }
-        }
-      }
+      if (sizeof(T) == 2 && b_l >= 1 && b_l <= 3) mine = byte_table<T>(b_l, sc_l, m_l);
     }
     int k = claim.kb;
     while (k < claim.ke) {
@@ -670,9 +665,12 @@ unpack_mixed_flat_kernel(const int32_t* __restrict__ packed, const int32_t* __re
       const int k1 = min(k + run_lanes / kFlatBundle, claim.ke);
       const uint32_t olo = __shfl_sync(kFull, (uint32_t)off_l, first);
       const uint32_t ohi = __shfl_sync(kFull, (uint32_t)((uint64_t)off_l >> 32), first);
-      const int32_t* in = packed + (int64_t)(((uint64_t)ohi << 32) | olo) + lane;
-#define ACTNN_CASE(B) \
-      case B: unpack_flat_run<T, B, sizeof(ST) == 2>(k, k1, q0, in, sc_l, m_l, t01_l, t23_l, out, plan, lane); break;
+      const int32_t* in = packed + (int64_t)(((uint64_t)ohi << 32) | olo);
+#define ACTNN_CASE(B)                                                                                             \
+      case B:                                                                                                     \
+        if constexpr (kNibbles<T, B>) unpack_flat_nibbles<T, B>(k, k1, q0, in, order, mine, out, plan);           \
+        else unpack_flat_run<T, B, sizeof(ST) == 2>(k, k1, q0, in, sc_l, m_l, out, plan, lane);                   \
+        break;
       switch (b) {
         ACTNN_CASE(1) ACTNN_CASE(2) ACTNN_CASE(3) ACTNN_CASE(4) ACTNN_CASE(5) ACTNN_CASE(6) ACTNN_CASE(7)
         ACTNN_CASE(8)

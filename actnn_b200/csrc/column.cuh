@@ -293,7 +293,7 @@ constexpr int kAhead = 4;
 struct BundleWords {
   uint32_t w[kAhead];
   float sc, m;                // statistics of group `lane`
-  const int32_t* in;          // the lane's first word
+  const int32_t* in;          // the bundle's first word
   int b;                      // 0: not a width, nothing was written
 };
 struct ColumnStream {
@@ -310,17 +310,27 @@ struct ColumnStream {
     }
   }
   // sample n, which is lane i's
-  template <typename ST>
-  ACTNN_DEV BundleWords fetch(const ColumnTask& t, int G, int n, int i, const int32_t* __restrict__ packed,
-                              const ST* __restrict__ scale, const ST* __restrict__ mn, int lane) const {
+  template <typename T, typename ST>
+  ACTNN_DEV BundleWords fetch(const ColumnTask& t, const WordOrder<T>& order, int G, int n, int i,
+                              const int32_t* __restrict__ packed, const ST* __restrict__ scale,
+                              const ST* __restrict__ mn, int lane) const {
     BundleWords r;
     r.b = __shfl_sync(kFull, b_l, i);
     const uint32_t olo = __shfl_sync(kFull, (uint32_t)off_l, i);
     const uint32_t ohi = __shfl_sync(kFull, (uint32_t)((uint64_t)off_l >> 32), i);
-    r.in = packed + (int64_t)(((uint64_t)ohi << 32) | olo) + lane;
-    const int left = t.count * 8 * r.b - lane;
+    r.in = packed + (int64_t)(((uint64_t)ohi << 32) | olo);
+    const int words = t.count * 8 * r.b;
+    if (kNibbles<T, 3> && r.b <= 3) {                      // warp-uniform
+      const int base = order.base(r.b), step = order.step(r.b);
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) r.w[k] = k * 32 < left ? (uint32_t)__ldg(r.in + k * 32) : 0u;
+      for (int k = 0; k < kAhead; ++k) {
+        const int w = base + k * step;
+        r.w[k] = k < r.b && w < words ? (uint32_t)__ldg(r.in + w) : 0u;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) r.w[k] = k * 32 < words - lane ? (uint32_t)__ldg(r.in + lane + k * 32) : 0u;
+    }
     r.sc = 1.f;
     r.m = 0.f;
     if (lane < t.count) {
@@ -336,7 +346,7 @@ ACTNN_DEV void decode_words(const BundleWords& r, int count, const TransposePlan
   uint32_t w[B];
 #pragma unroll
   for (int k = 0; k < B; ++k)
-    w[k] = k < kAhead ? r.w[k < kAhead ? k : 0] : k * 32 + lane < count * 8 * B ? (uint32_t)__ldg(r.in + k * 32) : 0u;
+    w[k] = k < kAhead ? r.w[k < kAhead ? k : 0] : k * 32 + lane < count * 8 * B ? (uint32_t)__ldg(r.in + k * 32 + lane) : 0u;
   decode_bundle<T, B>(w, r.sc, r.m, plan, lane, use);
 }
 template <typename T, typename Use>
