@@ -10,6 +10,7 @@
 // behaviour of its own.
 #include <ATen/Functions.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/CUDAGeneratorImpl.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
@@ -234,6 +235,23 @@ Tensor sample_sumsq(const Tensor& grad_in) {
   return out;
 }
 
+// A copy of a small device tensor on its way to the host: enqueued on the current stream when made, waited for (by the
+// host, without the interpreter lock) in `wait`.
+struct Readback {
+  Tensor host;
+  at::cuda::CUDAEvent copied;
+  explicit Readback(const Tensor& t) {
+    c10::cuda::CUDAGuard guard(t.device());
+    host = t.to(at::TensorOptions().device(at::kCPU), /*non_blocking=*/true);        // pinned
+    copied.record();
+  }
+  Tensor wait() {
+    py::gil_scoped_release unlocked;
+    copied.synchronize();
+    return host;
+  }
+};
+
 // ---------------------------------------------------------------------------------------- mask-saving layers
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
@@ -348,6 +366,7 @@ struct MaxPool : torch::autograd::Function<MaxPool> {
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  py::class_<Readback>(m, "Readback").def(py::init<const Tensor&>()).def("wait", &Readback::wait);
   m.def("compress_mixed", &compress_mixed);
   m.def("unpack_mixed", &unpack_mixed);
   m.def("compress_single", &compress_single);

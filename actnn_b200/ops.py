@@ -184,8 +184,9 @@ def dequantize_activation(quantized, q_input_shape, dtype=None):
     else:
         input = dequantize_and_unpack(q_input, q_input_shape, q_bits, q_scale, q_min, out_dtype=dtype)
 
-    input = input.view(N, -1)[:, :num_features]
-    return input.reshape(*q_input_shape).contiguous()
+    if input.numel() != N * num_features:
+        input = input.view(N, -1)[:, :num_features]
+    return input.reshape(q_input_shape).contiguous()
 
 
 # ---------------------------------------------------------------------------------------
@@ -204,6 +205,27 @@ def _autocast_inputs(*tensors):
     dt = torch.get_autocast_dtype("cuda")
     return tuple(t.to(dt) if isinstance(t, torch.Tensor) and t.is_floating_point() and t.is_cuda else t
                  for t in tensors)
+
+
+class _autocast_off:
+    """The body of a Function without autocast: ``torch.autocast("cuda", enabled=False)`` inside the program's own
+    context, whose weight cache it leaves alone, at a tenth of its cost, and nothing where autocast is off anyway."""
+
+    def __enter__(self):
+        self.was_on = torch.is_autocast_enabled("cuda")
+        if self.was_on:
+            torch.set_autocast_enabled("cuda", False)
+
+    def __exit__(self, *exc):
+        if self.was_on:
+            torch.set_autocast_enabled("cuda", True)
+        return False
+
+
+def _start_allocation(scheme):
+    start = getattr(scheme, "start_allocation", None)
+    if start is not None:
+        start()
 
 
 def _debug_forward(tag, quantized):
@@ -233,7 +255,7 @@ class convnd(Function):
     def run_forward(n, forward_op, ctx, input, weight, bias=None, stride=1, padding=0, dilation=1, groups=1,
                     scheme=None):
         input, weight, bias = _autocast_inputs(input, weight, bias)
-        with torch.autocast("cuda", enabled=False):
+        with _autocast_off():
             quantized = quantize_activation(input, scheme, minmax=producer_minmax(input) if scheme else None)
             ctx.scheme = scheme
             ctx.saved = quantized, weight, bias
@@ -251,6 +273,7 @@ class convnd(Function):
     def run_backward(n, ctx, grad_output, bias_reduce_dims, aug):
         if ctx.scheme:
             ctx.scheme.set_scale(grad_output)
+            _start_allocation(ctx.scheme)
         q_input_shape, stride, padding, dilation, groups, in_dtype = ctx.other_args
         padding, stride, dilation = aug(padding), aug(stride), aug(dilation)
         quantized, weight, bias = ctx.saved
@@ -310,7 +333,7 @@ class conv_transposend(Function):
     def run_forward(n, forward_op, ctx, input, weight, bias=None, stride=1, padding=0, output_padding=0,
                     groups=1, dilation=1, scheme=None):
         input, weight, bias = _autocast_inputs(input, weight, bias)
-        with torch.autocast("cuda", enabled=False):
+        with _autocast_off():
             quantized = quantize_activation(input, scheme)
             ctx.scheme = scheme
             ctx.saved = quantized, weight, bias
@@ -324,6 +347,7 @@ class conv_transposend(Function):
     def run_backward(n, ctx, grad_output, bias_reduce_dims, aug):
         if ctx.scheme:
             ctx.scheme.set_scale(grad_output)
+            _start_allocation(ctx.scheme)
         q_input_shape, stride, padding, output_padding, dilation, groups, in_dtype = ctx.other_args
         padding, output_padding, stride, dilation = aug(padding), aug(output_padding), aug(stride), aug(dilation)
         quantized, weight, bias = ctx.saved
@@ -378,7 +402,7 @@ class linear(Function):
     @staticmethod
     def forward(ctx, input, weight, bias=None, scheme=None):
         input, weight, bias = _autocast_inputs(input, weight, bias)
-        with torch.autocast("cuda", enabled=False):
+        with _autocast_off():
             quantized = quantize_activation(input, scheme)
             empty_cache(config.empty_cache_threshold)
             ctx.scheme = scheme
@@ -390,6 +414,7 @@ class linear(Function):
     def backward(ctx, grad_output):
         if ctx.scheme:
             ctx.scheme.set_scale(grad_output)
+            _start_allocation(ctx.scheme)
         quantized, weight, bias = ctx.saved
         q_input_shape, in_dtype = ctx.other_args
         input = dequantize_activation(quantized, q_input_shape, in_dtype)
@@ -397,9 +422,12 @@ class linear(Function):
         empty_cache(config.empty_cache_threshold)
 
         grad_output = grad_output.to(input.dtype)
-        go = grad_output.reshape(-1, grad_output.shape[-1])
-        x = input.reshape(-1, input.shape[-1])
-        grad_input = go.mm(weight).view(q_input_shape)
+        go, x = grad_output, input
+        if go.dim() != 2 or x.dim() != 2:
+            go, x = go.reshape(-1, go.shape[-1]), x.reshape(-1, x.shape[-1])
+        grad_input = go.mm(weight)
+        if grad_input.shape != q_input_shape:
+            grad_input = grad_input.view(q_input_shape)
         grad_weight = go.t().mm(x)
         grad_bias = go.sum(0) if bias is not None else None
         if ctx.scheme:

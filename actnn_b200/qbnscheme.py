@@ -3,7 +3,7 @@ preceding conv / linear layer (mirror of actnn/actnn/qbnscheme.py:9-60)."""
 from .conf import config
 from .cpp_extension import backward_func as ext_backward_func
 from .cpp_extension import calc_precision as ext_calc_precision
-from .qscheme import QScheme, compress_groups, group_minimax, total_bits_after_greedy
+from .qscheme import QScheme, compress_groups, group_minimax, target_bits, total_bits_after_greedy
 
 
 class QBNScheme(QScheme):
@@ -22,7 +22,7 @@ class QBNScheme(QScheme):
         groups, mn, mx = group_minimax(input)
         G = groups.shape[1]
         C = ext_calc_precision.sensitivity(mn, mx, N, config.group_size / num_pixels)
-        target = int(self.bits * N)
+        target = target_bits(self.bits, N)
         b, offsets = ext_calc_precision.allocate_bits(C, self.initial_bits, target, None, G,
                                                       config.group_size, with_offsets=True)
         b.word_offsets = offsets
@@ -38,7 +38,7 @@ class QBNScheme(QScheme):
         N, D = input.shape[0], input.shape[1]
         num_pixels = (input.numel() // N) // D
         q_input, b, q_scale, q_min, _ = compress_groups(
-            input, int(self.bits * N), int(self.initial_bits), config.group_size / num_pixels,
+            input, target_bits(self.bits, N), int(self.initial_bits), config.group_size / num_pixels,
             1.0, None, config.stochastic, stat_dtype=stat_dtype, minmax=minmax)
         return q_input, b, q_scale, q_min
 
@@ -50,7 +50,7 @@ class QBNScheme(QScheme):
         if num_pixels == 0:
             return None
         out = ext_backward_func.batch_norm_codes_forward(
-            input, weight, bias, running_mean, running_var, momentum, eps, int(self.bits * N), int(self.initial_bits),
+            input, weight, bias, running_mean, running_var, momentum, eps, target_bits(self.bits, N), int(self.initial_bits),
             config.group_size / num_pixels, config.stochastic, stats)
         if out is not None:
             self.prev_linear = QScheme.prev_layer

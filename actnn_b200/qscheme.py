@@ -7,8 +7,10 @@ priority queue and copies the bits back (three host synchronisations per layer p
 step).  Here the chain is minimax -> sensitivity -> allocate_bits, three kernel launches
 with no host round trip; the only host read left is the once-per-step per-layer
 re-allocation."""
+import numpy as np
 import torch
 
+from . import _lib
 from .conf import config
 from .cpp_extension import calc_precision as ext_calc_precision
 from .cpp_extension import minimax as ext_minimax
@@ -57,6 +59,13 @@ def total_bits_after_greedy(n: int, initial_bits: int, target: int) -> int:
     return min(initial_bits * n, max(int(target), n))
 
 
+def target_bits(bits, n: int) -> int:
+    """``int(bits * n)``, the product in float32 where ``bits`` is a float32 tensor, without a tensor operation."""
+    if isinstance(bits, torch.Tensor) and bits.dtype == torch.float32 and not bits.is_cuda and n < 1 << 24:
+        return int(np.float32(bits.item()) * np.float32(n))
+    return int(bits * n)
+
+
 class QScheme(object):
     num_samples = 1
     num_layers = 0
@@ -64,6 +73,7 @@ class QScheme(object):
     update_scale = True
     layers = []
     prev_layer = None
+    _started = None                                   # an allocation enqueued by start_allocation
 
     def __init__(self, layer, group=0, num_locations=1, depthwise_groups=1):
         self.initial_bits = config.initial_bits
@@ -123,7 +133,7 @@ class QScheme(object):
         groups, mn, mx = group_minimax(input)
         G = groups.shape[1]
         C = self._sensitivity(mn, mx, N, config.group_size / num_pixels, input.device)
-        target = int(self.bits * N)
+        target = target_bits(self.bits, N)
         b, offsets = ext_calc_precision.allocate_bits(C, self.initial_bits, target, None, G,
                                                       config.group_size, with_offsets=True)
         b.word_offsets = offsets
@@ -151,7 +161,7 @@ class QScheme(object):
         if minmax is not None and (config.group_size != 256 or (input.numel() // N) % 256 != 0):
             minmax = None                                      # padded groups: not the producer's
         q_input, b, q_scale, q_min, C = compress_groups(
-            input, int(self.bits * N), int(self.initial_bits), config.group_size / num_pixels,
+            input, target_bits(self.bits, N), int(self.initial_bits), config.group_size / num_pixels,
             self.num_locations / 4 / self.depthwise_groups, grad.reshape(1), config.stochastic,
             stat_dtype=stat_dtype, minmax=minmax)
         self.C = C
@@ -161,7 +171,12 @@ class QScheme(object):
 
     # ------------------------------------------------------------- per-layer bits
     @staticmethod
-    def allocate_perlayer():
+    def allocate_perlayer(started=None):
+        """Re-allocate the per-layer widths; ``started``: what ``start_perlayer`` returned, if it has been called."""
+        if started is not None:
+            for layers, N, sums in started:
+                QScheme._set_average_bits(layers, sums.wait(), N)      # the one host read per step
+            return
         for g, group_bits in enumerate(config.activation_compression_bits):
             layers = [layer for layer in QScheme.layers if layer.group == g and layer.C is not None]
             L = len(layers)
@@ -180,41 +195,84 @@ class QScheme(object):
             else:
                 # joint allocation over layers x samples, then the per-layer average
                 N = layers[0].C.shape[0]
-                total = float(sum(layer.dim for layer in layers) * N * group_bits)
-                sums = ext_calc_precision.allocate_layers([layer.C for layer in layers], [layer.dim for layer in layers],
-                                                          config.initial_bits, total)
-                if sums is not None:
-                    means = sums.cpu().float() / N                 # the one host read per step, see below
-                    for i, layer in enumerate(layers):
-                        layer.bits = means[i]
-                    continue
-                C = torch.cat([layer.C for layer in layers], 0).contiguous()
-                w = torch.tensor([layer.dim for layer in layers], dtype=torch.int32,
-                                 device=device).repeat_interleave(N).contiguous()
-                b, _ = ext_calc_precision.allocate_bits(C, config.initial_bits, total, w)
-                # the one host read per step.  Integer sums are exact on any device; the division
-                # is done on the host in float32 like the reference's ``bs.float().mean()``
-                means = b.view(L, N).sum(dim=1).cpu().float() / N
-                for i, layer in enumerate(layers):
-                    layer.bits = means[i]
+                sums = QScheme._joint_sums(layers, group_bits)
+                if sums is None:
+                    total = float(sum(layer.dim for layer in layers) * N * group_bits)
+                    C = torch.cat([layer.C for layer in layers], 0).contiguous()
+                    w = torch.tensor([layer.dim for layer in layers], dtype=torch.int32,
+                                     device=device).repeat_interleave(N).contiguous()
+                    b, _ = ext_calc_precision.allocate_bits(C, config.initial_bits, total, w)
+                    sums = b.view(L, N).sum(dim=1)
+                QScheme._set_average_bits(layers, sums.cpu(), N)       # the one host read per step
 
-    def if_allocate_perlayer(self):
-        """Called at the end of every layer's backward; re-allocates the per-layer widths when
-        backward has reached the first trainable layer (qscheme.py:130-147 of the reference).
-        The cheap test (is this that layer?) comes first: the scans below are O(layers)."""
+    @staticmethod
+    def _joint_sums(layers, group_bits):
+        """Sum of the widths of each layer from one launch, or ``None`` when it does not cover the problem."""
+        total = float(sum(layer.dim for layer in layers) * layers[0].C.shape[0] * group_bits)
+        return ext_calc_precision.allocate_layers([layer.C for layer in layers], [layer.dim for layer in layers],
+                                                  config.initial_bits, total)
+
+    @staticmethod
+    def _set_average_bits(layers, sums, N):
+        # integer sums are exact on any device; the division is done on the host in float32 like the
+        # reference's ``bs.float().mean()``
+        means = sums.float() / N
+        for layer, mean in zip(layers, means.unbind()):
+            layer.bits = mean
+
+    @staticmethod
+    def start_perlayer():
+        """Enqueue the joint allocation of every group and the copies of its results to the host:
+        ``[(layers, samples, sums)]``, or ``None`` when a group takes another path."""
+        native = _lib.native()
+        if not native:
+            return None
+        started = []
+        for g, group_bits in enumerate(config.activation_compression_bits):
+            layers = [layer for layer in QScheme.layers if layer.group == g and layer.C is not None]
+            if not layers:
+                continue
+            sums = None if group_bits == config.initial_bits else QScheme._joint_sums(layers, group_bits)
+            if sums is None:
+                return None
+            started.append((layers, layers[0].C.shape[0], native.Readback(sums)))
+        return started
+
+    def _closes_step(self):
+        """Whether this is the first trainable layer, which backward reaches last, and every layer has been
+        compressed.  The cheap test comes first: the scan below is O(layers)."""
         if not config.perlayer or not (config.compress_activation and config.training):
-            return
+            return False
         first_layer = None
         for layer in QScheme.layers:
             if layer.layer.weight.requires_grad:
                 first_layer = layer
                 break
-        # backward reaches the first trainable layer last: re-allocate there
-        if self is not first_layer:
+        return self is first_layer and all(layer.C is not None for layer in QScheme.layers)
+
+    def start_allocation(self):
+        """Called at the start of every layer's backward: in the one that ends the step the widths' allocation is
+        enqueued before the layer's own work.  The sensitivities it needs are from the forward pass, so the result is
+        that of an allocation at the end; but the host then waits for the copy of a few numbers while the GPU has the
+        layer's backward to do, not for all of that to finish.  A pass, float16, in one process: 3x3 convolution of
+        256 x 256 x 28 x 28 with its ReLU 1048 -> 899 us, bottleneck block at batch 256 2053 -> 1875; where the GPU waits
+        for the host anyway the event costs what it saves (classifier head at batch 256 788 -> 801)."""
+        self._started = None
+        if QScheme.allocate_perlayer is _allocate_perlayer and self._closes_step():
+            self._started = QScheme.start_perlayer()
+
+    def if_allocate_perlayer(self):
+        """Called at the end of every layer's backward; re-allocates the per-layer widths when
+        backward has reached the first trainable layer (qscheme.py:130-147 of the reference)."""
+        started, self._started = self._started, None
+        if started is None and not self._closes_step():
             return
-        for layer in QScheme.layers:
-            if layer.C is None:
-                return
         from .qbnscheme import QBNScheme
-        QScheme.allocate_perlayer()
+        if started is None:
+            QScheme.allocate_perlayer()
+        else:
+            QScheme.allocate_perlayer(started)
         QBNScheme.allocate_perlayer()
+
+
+_allocate_perlayer = QScheme.allocate_perlayer
