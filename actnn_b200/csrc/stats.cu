@@ -89,7 +89,9 @@ int launch_minimax(const void* data, void* mn, void* mx, int64_t rows, int64_t c
   const int64_t cap = (int64_t)device_info().sm_count * 8;
   if (cols == kGroup) {
     const int64_t tasks = (rows + kMinimaxRows - 1) / kMinimaxRows;
-    const int grid = (int)max((int64_t)1, min((tasks + 7) / 8, cap));
+    // a warp per task: blocks that start in order read closer together than warps that stride over the tensor do
+    // (bfloat16 512 x 784 groups after a decode of the same size 36.1 -> 34.2 us; 134 M float16 elements 40.4 -> 39.3)
+    const int grid = (int)min((tasks + 7) / 8, (int64_t)0x7fffffff);
     minimax256_kernel<T><<<grid, kThreads, 0, s>>>((const T*)data, (T*)mn, (T*)mx, rows, reverse, clear_word);
   } else {
     if (clear_word && cudaMemsetAsync(clear_word, 0, sizeof(unsigned), s) != cudaSuccess) return ACTNN_ERR_LAUNCH;
