@@ -50,7 +50,7 @@ column_pack_kernel(const T* __restrict__ data, ColumnShape sh, const T* __restri
   const ColumnTask t = column_task(sh);
   if (!t.valid) return;
   const ColumnOctets<EDGE> oct(sh, t, lane);
-  pack_column<T, ST, PHILOX>(data, sh, t, oct, mn, mx, bits, word_offsets, packed, scale, mn_out, noise, key, lane,
+  pack_column<T, ST, PHILOX>(data, sh, t, oct, mn, mx, bits, word_offsets, packed, scale, mn_out, noise, key, lane, false,
                              [](int, const Oct<T> (&)[kBundle]) {});
 }
 

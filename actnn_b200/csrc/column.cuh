@@ -154,6 +154,11 @@ template <bool EDGE> struct ColumnOctets {
       else x[gi] = gi < count ? load_oct<T>(sample + first + gi * kGroup) : zero_oct<T>();
     }
   }
+  // The column's part of a sample into the L2; one lane asks for all of it.
+  template <typename T> ACTNN_DEV void prefetch(const T* sample, const ColumnShape& sh, int lane) const {
+    if (lane != 0 || (EDGE && align != kOct)) return;
+    l2_prefetch(sample + first, (uint32_t)(min((int64_t)(kBundle * kGroup), sh.F - first) * (int64_t)sizeof(T)));
+  }
   template <typename T> ACTNN_DEV void store(T* sample, int gi, const Oct<T>& x) const {
     if constexpr (EDGE) store_octet<T, true>(sample + first + gi * kGroup, x, valid[gi], align);
     else if (gi < count) store_oct_streaming<T>(sample + first + gi * kGroup, x);
@@ -224,7 +229,8 @@ ACTNN_DEV void pack_column_bundle(const Oct<T> (&x)[kBundle], const Oct<T> (&nz)
   }
 }
 
-// Scale, stochastic rounding and pack of a column; each(n, octets) sees every sample's octets on the way.
+// Scale, stochastic rounding and pack of a column; each(n, octets) sees every sample's octets on the way.  `ahead`: the
+// octets of the sample after the one being loaded are requested into the L2.
 // Eight samples at a time: lane 4i + g prepares group g of the i-th of them (one division per lane for eight
 // bundles).  The noise octets are formed before the dispatch on the width, so the eight width variants stay short.
 template <typename T, typename ST, bool PHILOX, bool EDGE, typename Each>
@@ -232,7 +238,7 @@ ACTNN_DEV void pack_column(const T* __restrict__ data, const ColumnShape& sh, co
                            const ColumnOctets<EDGE>& oct, const T* __restrict__ mn, const T* __restrict__ mx,
                            const int32_t* __restrict__ bits, const int64_t* __restrict__ word_offsets,
                            int32_t* __restrict__ packed, ST* __restrict__ scale, ST* __restrict__ mn_out,
-                           const T* __restrict__ noise, const NoiseKey& key, int lane, Each each) {
+                           const T* __restrict__ noise, const NoiseKey& key, int lane, bool ahead, Each each) {
   const TransposePlan plan = make_transpose_plan(lane);
   Oct<T> next[kBundle];
   oct.template load<T>(data + (int64_t)t.n0 * sh.F, next);
@@ -259,6 +265,7 @@ ACTNN_DEV void pack_column(const T* __restrict__ data, const ColumnShape& sh, co
 #pragma unroll
       for (int gi = 0; gi < kBundle; ++gi) x[gi] = next[gi];
       if (n + 1 < t.n1) oct.template load<T>(data + (int64_t)(n + 1) * sh.F, next);
+      if (ahead && n + 2 < t.n1) oct.template prefetch<T>(data + (int64_t)(n + 2) * sh.F, sh, lane);
       const int64_t q0 = (int64_t)n * sh.G + t.g0;
       if constexpr (PHILOX) {
         noise_bundle<T>(key, q0, lane, nz);

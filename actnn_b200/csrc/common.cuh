@@ -103,6 +103,10 @@ ACTNN_DEV void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+// Asks for `bytes` (a multiple of 16) at `p` (16-byte aligned) to be brought into the L2; no register waits for them.
+ACTNN_DEV void l2_prefetch(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(p), "r"(bytes) : "memory");
+}
 // One attempt may sleep in hardware for up to about kBulkWaitHintNs before it reports failure.
 constexpr uint32_t kBulkWaitHintNs = 20000u;
 ACTNN_DEV bool mbar_try_wait(uint32_t bar, uint32_t parity) {
