@@ -13,10 +13,10 @@ import sys
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SOURCES = ["api.cu", "codec_mixed.cu", "codec_single.cu", "codec_generic.cu", "codec_column.cu",
+SOURCES = ["api.cu", "codec_mixed.cu", "codec_single.cu", "codec_generic.cu", "codec_column.cu", "codec_ragged.cu",
            "compress_mixed.cu", "stats.cu", "mask_ops.cu",
            "maxpool.cu", "batch_norm.cu", "bn_column.cu", "layout.cu"]
-HEADERS = ["common.cuh", "quant_math.cuh", "mixed_bundle.cuh", "column.cuh", os.path.join("..", "..", "include", "actnn_b200.h")]
+HEADERS = ["common.cuh", "quant_math.cuh", "mixed_bundle.cuh", "column.cuh", "flat_runs.cuh", os.path.join("..", "..", "include", "actnn_b200.h")]
 LIB = os.path.join(HERE, "libactnn_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",

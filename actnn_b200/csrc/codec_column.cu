@@ -1,7 +1,8 @@
 // The mixed-precision codec on [N, F] activations whose samples are not whole groups of 256, or not
 // a multiple of four groups: min / max, pack and unpack on the column mapping (column.cuh), reading
-// and writing the activation where it is.  (The reference pads every sample with a concatenation
-// and strips the padding with a copy, actnn/actnn/qscheme.py:61-71 and ops.py:137-139.)
+// and writing the activation where it is.  Large activations are packed in the order of the stream instead
+// (codec_ragged.cu).  (The reference pads every sample with a concatenation and strips the padding with a copy,
+// actnn/actnn/qscheme.py:61-71 and ops.py:137-139.)
 //
 // Bound by HBM at large sizes and by launches at small ones.  float16, compress and decompress of
 // 100 x 192 x 35 x 35 (918.75 groups a sample): 127.1 -> 60.6 us, of which the padded copy was 18 and the
@@ -139,6 +140,9 @@ int column_pack(const void* data, const void* mn, const void* mx, const int32_t*
                 int stochastic, const void* noise, uint64_t seed, uint64_t offset, cudaStream_t s) {
   if (!column_supported(N, F)) return ACTNN_ERR_SHAPE;
   if (stochastic && noise && !aligned(noise, dtype == ACTNN_F32 ? 32 : 16)) return ACTNN_ERR_ALIGN;
+  if (ragged_pays(N, F))
+    return ragged_pack(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, F, dtype, stat_dtype, stochastic,
+                       noise, seed, offset, s);
 #define ACTNN_PACK(T, ST)                                                                                         \
   return launch_pack<T, ST>(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, F, stochastic, noise, seed, \
                             offset, s)

@@ -11,7 +11,7 @@
 // string across the warp yields output words 32k .. 32k+31 of the bundle, lane w holding
 // word 32k + w, so every store is one fully coalesced 128-byte line.  No shared memory,
 // no atomics, no block-level synchronisation.
-#include "mixed_bundle.cuh"
+#include "flat_runs.cuh"
 
 namespace actnn {
 namespace {
@@ -168,8 +168,6 @@ pack_mixed_kernel(const T* __restrict__ data, const T* __restrict__ mn, const T*
 //     samples because G % 4 == 0, so its width is warp-uniform;
 //   * the octets of the next bundle (also across the task boundary) are requested before the
 //     current one is quantized: a warp always has loads in flight.
-constexpr int kFlatGroups = 32;       // groups per task
-constexpr int kFlatBundle = 4;        // groups per bundle
 #ifndef ACTNN_FLAT_BLOCKS
 #define ACTNN_FLAT_BLOCKS 2
 #endif
@@ -178,74 +176,6 @@ constexpr int kFlatBundle = 4;        // groups per bundle
 #endif
 constexpr int kFlatUnpackBlocks = ACTNN_FLAT_UNPACK_BLOCKS;
 constexpr int kFlatBlocks16 = ACTNN_FLAT_BLOCKS;   // resident blocks per SM the flat kernels are compiled for (16-bit types)
-
-template <typename T, int B, int MODE, bool CLAMP_LOW>
-ACTNN_DEV void pack_flat_bundle(const Oct<T> (&x)[kFlatBundle], const LaneParams<T>& mine, int first_lane,
-                                int64_t q, int32_t* __restrict__ out, const T* __restrict__ noise,
-                                const NoiseKey& key, const TransposePlan& plan, int lane) {
-  constexpr int GPC = NoiseShape<T>::GPC;
-  uint32_t S[B];
-#pragma unroll
-  for (int k = 0; k < B; ++k) S[k] = 0u;
-  Oct<T> nzb[GPC];
-#pragma unroll
-  for (int gi = 0; gi < kFlatBundle; ++gi) {
-    const QP<T> qp = fetch_lane_params<T>(mine, first_lane + gi);
-    Oct<T> nz;
-    if constexpr (MODE == kNoisePhilox) {
-      if (gi % GPC == 0) noise_block<T>(key, (uint64_t)(q + gi), lane, nzb);
-      nz = nzb[gi % GPC];
-    } else if constexpr (MODE == kNoiseTensor) {
-      nz = load_oct<T>(noise + (q + gi) * kGroup + lane * kOct);
-    } else {
-      nz = zero_oct<T>();
-    }
-    uint32_t lo, hi;
-    row_from_magic<T, B>(quantize_oct<T, CLAMP_LOW, B>(x[gi], nz, qp), lo, hi);
-    if (gi == 0) put_row<B, 0 * 8 * B>(S, lo, hi);
-    if (gi == 1) put_row<B, 1 * 8 * B>(S, lo, hi);
-    if (gi == 2) put_row<B, 2 * 8 * B>(S, lo, hi);
-    if (gi == 3) put_row<B, 3 * 8 * B>(S, lo, hi);
-  }
-#pragma unroll
-  for (int k = 0; k < B; ++k) out[k * 32 + lane] = (int32_t)warp_transpose32(S[k], plan);
-}
-
-// A run: bundles k0 .. k1-1 of a task, all of the same width B (a run ends where the next
-// sample has another width).  The width is a template argument here, so the loop over the
-// bundles has no dispatch in it and the octets of bundle k+1 are requested before bundle k is
-// quantized (two register buffers used alternately; nothing is copied).  `a` already holds the
-// octets of bundle k0.
-template <typename T, int B, int MODE, bool CLAMP_LOW, bool PREFETCH>
-ACTNN_DEV void pack_flat_run(Oct<T> (&a)[kFlatBundle], Oct<T> (&b)[kFlatBundle], int k0, int k1, int64_t q0,
-                             const T* __restrict__ data, const LaneParams<T>& mine, int32_t* __restrict__ out,
-                             const T* __restrict__ noise, const NoiseKey& key, const TransposePlan& plan, int lane) {
-  auto load = [&](Oct<T> (&dst)[kFlatBundle], int k) {
-#pragma unroll
-    for (int gi = 0; gi < kFlatBundle; ++gi)
-      dst[gi] = load_oct<T>(data + (q0 + k * kFlatBundle + gi) * kGroup + lane * kOct);
-  };
-  if constexpr (!PREFETCH) {
-    for (int k = k0; k < k1; ++k) {
-      if (k > k0) load(a, k);
-      pack_flat_bundle<T, B, MODE, CLAMP_LOW>(a, mine, k * kFlatBundle, q0 + k * kFlatBundle, out, noise, key, plan,
-                                              lane);
-      out += 32 * B;                                           // consecutive groups are consecutive in the stream
-    }
-  } else {
-    for (int k = k0; k < k1; k += 2) {
-      if (k + 1 < k1) load(b, k + 1);
-      pack_flat_bundle<T, B, MODE, CLAMP_LOW>(a, mine, k * kFlatBundle, q0 + k * kFlatBundle, out, noise, key, plan,
-                                              lane);
-      out += 32 * B;
-      if (k + 1 >= k1) break;
-      if (k + 2 < k1) load(a, k + 2);
-      pack_flat_bundle<T, B, MODE, CLAMP_LOW>(b, mine, (k + 1) * kFlatBundle, q0 + (k + 1) * kFlatBundle, out,
-                                              noise, key, plan, lane);
-      out += 32 * B;
-    }
-  }
-}
 
 template <typename T, typename ST, int MODE, bool CLAMP_LOW>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 2 ? kFlatBlocks16 : 2)
@@ -453,12 +383,6 @@ struct FlatPool {
     return true;
   }
 };
-// (sample, group) of group q; one 32-bit division where the activation allows it
-ACTNN_DEV void split_group_index(int64_t q, int64_t G, int64_t& n, int64_t& r) {
-  if (((uint64_t)q | (uint64_t)G) >> 32) { n = q / G; } else { n = (int64_t)((uint32_t)q / (uint32_t)G); }
-  r = q - n * G;
-}
-
 // ---------------------------------------------------------------------------- unpack, flat tasks
 // Same task shape as the flat pack: lane l owns group q0 + l of a task of 32 groups (its
 // sample, width, stream position, scale and min come from coalesced loads), and eight bundles

@@ -271,6 +271,12 @@ int column_pack(const void* data, const void* mn, const void* mx, const int32_t*
 int column_unpack(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets, const void* scale,
                   const void* mn, void* out, int64_t N, int64_t F, int dtype, int stat_dtype, cudaStream_t stream);
 
+// codec_ragged.cu: the same pack for large activations (`ragged_pays`).
+bool ragged_pays(int64_t N, int64_t F);
+int ragged_pack(const void* data, const void* mn, const void* mx, const int32_t* bits, const int64_t* word_offsets,
+                int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t F, int dtype, int stat_dtype,
+                int stochastic, const void* noise, uint64_t seed, uint64_t offset, cudaStream_t stream);
+
 // stats.cu: actnn_minimax with two extras for the one-call compress: rows walked from the
 // last to the first (`reverse`), and a word zeroed by the kernel (`clear_word`, the ticket of
 // the next kernel).
