@@ -31,6 +31,7 @@ SIGNATURES = {
     "actnn_batch_norm_codes_backward": ['P'] * 12 + ['L', 'L', 'L', 'I', 'I', 'P', 'L', 'P'],
     "actnn_range_sqr": ['P', 'P', 'L', 'L', 'I', 'F', 'F', 'P', 'P', 'P'],
     "actnn_sample_sumsq": ['P', 'P', 'L', 'L', 'I', 'P'],
+    "actnn_sample_sumsq_mean": ['P', 'P', 'P', 'P', 'L', 'L', 'I', 'P'],
     "actnn_calc_precision": ['P', 'P', 'L', 'I', 'D', 'P', 'P', 'L', 'L', 'P', 'L', 'P'],
     "actnn_allocate_layers": ['P', 'P', 'I', 'L', 'I', 'D', 'P', 'P'],
     "actnn_relu_forward": ['P', 'P', 'P', 'L', 'I', 'P'],

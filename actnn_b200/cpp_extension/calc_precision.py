@@ -92,6 +92,15 @@ def sample_sumsq(grad: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def mean_sample_sumsq(grad: torch.Tensor) -> torch.Tensor:
+    """``sample_sumsq(grad).mean()`` (actnn/actnn/qscheme.py:55), in the same launch."""
+    nat = _lib.native()
+    if not nat or not grad.is_cuda or grad.dim() == 0 or grad.shape[0] == 0 \
+            or grad.dtype not in (torch.float32, torch.float16, torch.bfloat16):
+        return sample_sumsq(grad).mean()
+    return nat.mean_sample_sumsq(grad, _lib.ticket(grad.device))
+
+
 def calc_precision(b: torch.Tensor, C: torch.Tensor, w: torch.Tensor, target) -> torch.Tensor:
     for t, name in ((b, "b"), (C, "C"), (w, "w")):
         if not t.is_contiguous():

@@ -235,6 +235,18 @@ Tensor sample_sumsq(const Tensor& grad_in) {
   return out;
 }
 
+// The mean of sample_sumsq over the samples (0-dimensional); at least one sample
+Tensor mean_sample_sumsq(const Tensor& grad_in, const Tensor& ticket) {
+  c10::cuda::CUDAGuard guard(grad_in.device());
+  const Tensor grad = grad_in.contiguous();
+  const int64_t n = grad.size(0);
+  Tensor out = make({n}, at::kFloat, grad), mean = make({}, at::kFloat, grad);
+  check(actnn_sample_sumsq_mean(grad.data_ptr(), out.data_ptr<float>(), mean.data_ptr<float>(), ticket.data_ptr(), n,
+                                grad.numel() / n, dtype_id(grad.scalar_type()), stream()),
+        "actnn_sample_sumsq_mean");
+  return mean;
+}
+
 // A copy of a small device tensor on its way to the host: enqueued on the current stream when made, waited for (by the
 // host, without the interpreter lock) in `wait`.
 struct Readback {
@@ -375,6 +387,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("batch_norm_backward", &batch_norm_backward);
   m.def("transpose16", &transpose16);
   m.def("sample_sumsq", &sample_sumsq);
+  m.def("mean_sample_sumsq", &mean_sample_sumsq);
   m.def("relu", [](const Tensor& x) { return Relu::apply(x, false)[0]; });
   m.def("relu_minmax", [](const Tensor& x) { return Relu::apply(x, true); });
   m.def("dropout", [](const Tensor& x, double p) { return Dropout::apply(x, p); });

@@ -106,12 +106,12 @@ class QScheme(object):
     def set_scale(self, grad):
         if not QScheme.update_scale:
             return
-        sq = ext_calc_precision.sample_sumsq(grad)
         if config.use_gradient:
+            sq = ext_calc_precision.sample_sumsq(grad)
             assert QScheme.batch is not None
             self.scales[QScheme.batch] = self.scales[QScheme.batch] * 0.5 + sq.cpu() * 0.5
         else:
-            self.scales = sq.mean()
+            self.scales = ext_calc_precision.mean_sample_sumsq(grad)
 
     # ------------------------------------------------------------- per-sample bits
     def _sensitivity(self, mn, mx, N, range_factor, device):

@@ -154,6 +154,10 @@ int actnn_range_sqr(const void* mn, const void* mx, int64_t N, int64_t G, int st
  * (grad.view(N, -1).float().norm(dim=1).square()) with one read of the gradient. */
 int actnn_sample_sumsq(const void* grad, float* out, int64_t N, int64_t F, int dtype,
                        actnn_stream_t stream);
+/* The same and *mean, the mean of out[0..N-1] (qscheme.py:55), N >= 1.  `ticket`: as in
+ * actnn_compress_mixed_prestat_kept. */
+int actnn_sample_sumsq_mean(const void* grad, float* out, float* mean, void* ticket, int64_t N, int64_t F, int dtype,
+                            actnn_stream_t stream);
 
 /* Replaces: calc_precision(b, C, w, target) -> b,
  * actnn/actnn/cpp_extension/calc_precision.cc:9-50 (a CPU priority queue there; here a
