@@ -233,12 +233,13 @@ max_pool_forward_row_kernel(const T* __restrict__ x, T* __restrict__ y, int8_t* 
 // Forward for 16-bit types, the same geometries with equal row and column padding P: a thread walks down
 // `rows` output rows of a segment of eight output columns.  Everything stays in packed pairs, two output columns
 // per register: pair k of tap kw holds the inputs that outputs 2k and 2k + 1 see through that tap.  An input
-// row is loaded and regrouped once, although two windows of height 3 share every other row.  The maximum
-// comes first (packed max), the arg-max by comparing the taps with it from the last to the first, so that
-// the first of equals wins; the output is that tap, not the maximum: packed max makes +0 of the two zeros, whichever comes
-// first (ReLU + pooling, both ways: 269.9 -> 271.7 us).  A window without any value above -infinity keeps code 0.
-// Bound by HBM: 205 MB in, 77 MB out for float16 128 x 64 x 112 x 112, 3 x 3 / 2.  The version that compared
-// in float32, one output at a time and every row three times, took 69.9 us; this one 57.9 (4.9 TB/s).
+// row is loaded and regrouped once, although two windows of height 3 share every other row.  The maxima of the rows
+// and of the window come first (packed max), then the first row whose maximum is the window's, then the first tap of that
+// row; the output is that tap, not the maximum: packed max makes +0 of the two zeros, whichever comes first.  A window
+// without any value above -infinity keeps code 0.
+// 205 MB in, 77 MB out for float16 128 x 64 x 112 x 112, 3 x 3 / 2.  The version that compared in float32, one output at a
+// time and every row three times, took 69.9 us; comparing all nine taps with the maximum 59.5, bound by the ALU pipe
+// (74 % busy); by rows 57.6 (54.8 -> 52.9 behind the ReLU, whose output it finds in the L2).
 template <typename T> struct Packed;
 template <> struct Packed<__half> {
   using V = __half2;
@@ -257,6 +258,8 @@ template <typename T> ACTNN_DEV uint32_t packed_equal(uint32_t a, uint32_t b) { 
   using V = typename Packed<T>::V;
   return __heq2_mask(*reinterpret_cast<const V*>(&a), *reinterpret_cast<const V*>(&b));
 }
+
+ACTNN_DEV uint32_t packed_select(uint32_t mask, uint32_t a, uint32_t b) { return (mask & a) | (~mask & b); }
 
 // Sixteen columns from c0 of an input row and one beside them, as loaded.  Ordinary cached loads: the side column is
 // in a neighbouring thread's sector.  `wide`: one 32-byte load.
@@ -333,21 +336,31 @@ max_pool_forward_packed_kernel(const T* __restrict__ x, T* __restrict__ y, int8_
     uint32_t best[4], arg[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
+      uint32_t row_max[K], t[K];
+#pragma unroll
+      for (int kh = 0; kh < K; ++kh) {
+        row_max[kh] = r[kh].tap[0][k];
+#pragma unroll
+        for (int kw = 1; kw < K; ++kw) row_max[kh] = packed_max<T>(row_max[kh], r[kh].tap[kw][k]);
+      }
       uint32_t m = Packed<T>::kLowest;
 #pragma unroll
-      for (int kh = 0; kh < K; ++kh)
+      for (int kh = 0; kh < K; ++kh) m = packed_max<T>(m, row_max[kh]);
+      // the first row that holds the maximum, then the first tap of it that does
+      const uint32_t in0 = packed_equal<T>(m, row_max[0]), in1 = K == 3 ? packed_equal<T>(m, row_max[1]) : 0u;
 #pragma unroll
-        for (int kw = 0; kw < K; ++kw) m = packed_max<T>(m, r[kh].tap[kw][k]);
-      uint32_t a = 0u, v = m;
-#pragma unroll
-      for (int c = K * K - 1; c >= 0; --c) {
-        const uint32_t t = r[c / K].tap[c % K][k], eq = packed_equal<T>(m, t);
-        a = (eq & ((uint32_t)c * 0x00010001u)) | (~eq & a);
-        v = (eq & t) | (~eq & v);                                // the tap itself: of two zeros the first keeps its sign
+      for (int kw = 0; kw < K; ++kw) {
+        t[kw] = K == 3 ? packed_select(in1, r[1].tap[kw][k], r[K - 1].tap[kw][k]) : r[1].tap[kw][k];
+        t[kw] = packed_select(in0, r[0].tap[kw][k], t[kw]);
       }
-      a &= ~packed_equal<T>(m, Packed<T>::kLowest);
-      best[k] = v;
-      arg[k] = a;
+      const uint32_t at0 = packed_equal<T>(m, t[0]), at1 = K == 3 ? packed_equal<T>(m, t[1]) : 0u;
+      const uint32_t row = ~in0 & (K == 3 ? packed_select(in1, 0x00030003u, 0x00060006u) : 0x00020002u);
+      const uint32_t col = ~at0 & (K == 3 ? packed_select(at1, 0x00010001u, 0x00020002u) : 0x00010001u);
+      uint32_t v = K == 3 ? packed_select(at1, t[1], t[K - 1]) : t[1];
+      v = packed_select(at0, t[0], v);                           // the tap itself: of two zeros the first keeps its sign
+      const uint32_t none = packed_equal<T>(m, Packed<T>::kLowest);
+      best[k] = packed_select(none, m, v);
+      arg[k] = ~none & (row + col);
     }
     const int64_t o = ((int64_t)nc * g.Ho + ho) * g.Wo + wo0;
     if (vector_store) {                                          // Wo % 8 == 0, aligned outputs
@@ -369,10 +382,10 @@ max_pool_forward_packed_kernel(const T* __restrict__ x, T* __restrict__ y, int8_
   }
 }
 
-// Rows a thread of the strip kernels walks: eight (an input row is regrouped once, the shared one at the head
+// Rows a thread of the strip kernels walks: at most `most` (an input row is regrouped once, the shared one at the head
 // of a strip twice), fewer where that would leave the chip short of threads.
-int strip_rows(int64_t planes, int segs, int row_count) {
-  int rows = 8;
+int strip_rows(int64_t planes, int segs, int row_count, int most) {
+  int rows = most;
   while (rows > 1 && planes * segs * ((row_count + rows - 1) / rows) < (int64_t)device_info().sm_count * 2048) rows >>= 1;
   return rows;
 }
@@ -388,7 +401,10 @@ int launch_forward(const void* x, void* y, int8_t* idx, int64_t planes, const Po
     const int vec = g.Wo % 8 == 0 && aligned(y, sizeof(T) * 8) && aligned(idx, 8);
     if constexpr (sizeof(T) == 2) {
       if (g.PH == g.PW && g.SH == 2) {
-        const int rows = strip_rows(planes, segs, g.Ho), chunks = (g.Ho + rows - 1) / rows;
+        // us at 8 / 4 / 2 / 1 rows, float16: 3 x 3 on 128 x 64 x 112 x 112 57.6 / 57.6 / 59.1 / 66.2, 256 x 256 x 32 x 32 41.0 / 40.9 /
+        // 42.1 / 45.3, 2 x 2 there 35.8 / 34.7 / 33.0 / 34.1; output rows that are no whole octets are stored element by
+        // element, and neighbouring threads should then be on neighbouring rows: 256 x 64 x 56 x 56 110 / 110 / 98 / 64
+        const int rows = strip_rows(planes, segs, g.Ho, vec ? 4 : 1), chunks = (g.Ho + rows - 1) / rows;
         const int64_t total = planes * segs * chunks;            // <= total_segments
         const int pgrid = (int)((total + 255) / 256);
         const int wide = g.W % 16 == 0 && aligned(x, 32);
@@ -804,6 +820,161 @@ max_pool_backward_strip_kernel(const T* __restrict__ gy, const int8_t* __restric
   }
 }
 
+// The same for 16-bit types in packed pairs of windows.  Of the positions a pair of rows has, an odd column has one
+// window per row, an even one two (columns counted from the padding's edge), and the first row has two window rows:
+// gradients are picked by comparing two codes at once, one or two of them add up in the type itself, which rounds as
+// float32 and one rounding do, and only the positions with four are added in float32.  128 x 64 x 112 x 112, 3 x 3 / 2:
+// 63.9 us, bound by instruction issue (265 a pair of rows, ALU 72 % busy) -> 55.3 with strips of
+// four pairs.
+template <typename T, int K, int P> struct PackedWindows {
+  using Windows = PoolWindows<T, K, P>;
+  // codes (as float16 numbers 1024 + code) and gradients of window columns b0 .. b0 + 3, and of the four one to the
+  // side (b0 + 1 .. b0 + 4 with padding, b0 - 1 .. b0 + 2 without)
+  uint32_t code[2], grad[2], side_code[2], side_grad[2];
+  ACTNN_DEV void set(const typename Windows::Raw& raw) {
+    const uint2 g = *reinterpret_cast<const uint2*>(raw.grads);
+    grad[0] = g.x;
+    grad[1] = g.y;
+    code[0] = __byte_perm(raw.codes, 0x64646464u, 0x4140);
+    code[1] = __byte_perm(raw.codes, 0x64646464u, 0x4342);
+    if constexpr (P == 1 || K == 3) {
+      const uint32_t c = raw.side_code | 0x6400u, s = *reinterpret_cast<const uint16_t*>(&raw.side_grad);
+      if constexpr (P == 1) {
+        side_code[0] = __byte_perm(raw.codes, 0x64646464u, 0x4241);
+        side_code[1] = __byte_perm(raw.codes, c, 0x5453);
+        side_grad[0] = __byte_perm(g.x, g.y, 0x5432);
+        side_grad[1] = __byte_perm(g.y, s, 0x5432);
+      } else {
+        side_code[0] = __byte_perm(raw.codes, c, 0x5054);
+        side_code[1] = __byte_perm(raw.codes, 0x64646464u, 0x4241);
+        side_grad[0] = __byte_perm(s, g.x, 0x5410);
+        side_grad[1] = __byte_perm(g.x, g.y, 0x5432);
+      }
+    }
+  }
+  // the gradients that go through tap (KH, KW), in the order of the columns they reach
+  template <int KH, int KW> ACTNN_DEV void pick(uint32_t (&o)[2]) const {
+    constexpr bool kBeside = P == 1 ? KW == 0 : KW == 2;
+    constexpr uint32_t want = (0x6400u | (KH * K + KW)) * 0x00010001u;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if constexpr (kBeside) o[i] = side_grad[i] & packed_equal<__half>(side_code[i], want);
+      else o[i] = grad[i] & packed_equal<__half>(code[i], want);
+    }
+  }
+};
+// (0 + a) + b: the zero in front makes +0 of a -0, as an accumulator does
+template <typename T> ACTNN_DEV uint32_t packed_sum(uint32_t a) {
+  using V = typename Packed<T>::V;
+  const uint32_t zero = 0u;
+  const V r = __hadd2(*reinterpret_cast<const V*>(&a), *reinterpret_cast<const V*>(&zero));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+template <typename T> ACTNN_DEV uint32_t packed_sum(uint32_t a, uint32_t b) {
+  using V = typename Packed<T>::V;
+  const uint32_t x = packed_sum<T>(a);
+  const V r = __hadd2(*reinterpret_cast<const V*>(&x), *reinterpret_cast<const V*>(&b));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+template <typename T> ACTNN_DEV float half_plus(uint16_t v, float acc) {
+  float r;
+  if constexpr (DType<T>::id == ACTNN_F16) asm("add.rn.f32.f16 %0, %1, %2;" : "=f"(r) : "h"(v), "f"(acc));
+  else asm("add.rn.f32.bf16 %0, %1, %2;" : "=f"(r) : "h"(v), "f"(acc));
+  return r;
+}
+template <typename T> ACTNN_DEV uint32_t packed_sum(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  float f[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int s = 16 * h;
+    f[h] = half_plus<T>((uint16_t)(b >> s), half_plus<T>((uint16_t)(a >> s), 0.f));
+    f[h] = half_plus<T>((uint16_t)(d >> s), half_plus<T>((uint16_t)(c >> s), f[h]));
+  }
+  uint32_t r;
+  if constexpr (DType<T>::id == ACTNN_F16) {
+    const __half2 v = __floats2half2_rn(f[0], f[1]);
+    r = *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(f[0], f[1]);
+    r = *reinterpret_cast<const uint32_t*>(&v);
+  }
+  return r;
+}
+
+template <typename T, int K, int P>
+__global__ void __launch_bounds__(256)
+max_pool_backward_packed_kernel(const T* __restrict__ gy, const int8_t* __restrict__ idx, T* __restrict__ gx,
+                                uint32_t total, int segs, int chunks, int rows, PoolGeom g, int vector_load) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  const uint32_t strip = t / (uint32_t)segs;
+  const int seg = (int)(t - strip * (uint32_t)segs);
+  const uint32_t nc = strip / (uint32_t)chunks;
+  const int pairs = (g.H - 1 + P) / 2 + 1;
+  const int r0 = (int)(strip - nc * (uint32_t)chunks) * rows, r1 = min(pairs, r0 + rows);
+  const T* gy_p = gy + (int64_t)nc * g.Ho * g.Wo;
+  const int8_t* idx_p = idx + (int64_t)nc * g.Ho * g.Wo;
+  T* out = gx + (int64_t)nc * g.H * g.W + seg * 8;
+  // odd[i], even[i]: positions with one window column and with two
+  auto store = [&](int h, const uint32_t (&odd)[2], const uint32_t (&even)[2]) {
+    if (h < 0 || h >= g.H) return;
+    Oct<T> o;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t a = P == 1 ? odd[i] : even[i], b = P == 1 ? even[i] : odd[i];
+      o.r[2 * i] = __byte_perm(a, b, 0x5410);
+      o.r[2 * i + 1] = __byte_perm(a, b, 0x7632);
+    }
+    store_oct<T>(out + (int64_t)h * g.W, o);
+  };
+  using Windows = PoolWindows<T, K, P>;
+  PackedWindows<T, K, P> here;
+  typename Windows::Raw next;                                    // requested a pair ahead
+  uint32_t up[3][2];                                             // what the window row above gives through its last row
+  if constexpr (K == 3) {
+    Windows::request(next, gy_p, idx_p, r0 - 1, seg * 4, g, vector_load);
+    here.set(next);
+    here.template pick<2, 0>(up[0]);
+    here.template pick<2, 1>(up[1]);
+    here.template pick<2, 2>(up[2]);
+  }
+  Windows::request(next, gy_p, idx_p, r0, seg * 4, g, vector_load);
+  for (int r = r0; r < r1; ++r) {
+    here.set(next);
+    if (r + 1 < r1) Windows::request(next, gy_p, idx_p, r + 1, seg * 4, g, vector_load);
+    uint32_t a0[2], a1[2], a2[2], odd[2], even[2];
+    here.template pick<0, 0>(a0);
+    here.template pick<0, 1>(a1);
+    if constexpr (K == 3) here.template pick<0, 2>(a2);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if constexpr (K == 3) {
+        odd[i] = packed_sum<T>(up[1][i], a1[i]);
+        even[i] = packed_sum<T>(up[2][i], up[0][i], a2[i], a0[i]);
+      } else {
+        odd[i] = packed_sum<T>(a1[i]);
+        even[i] = packed_sum<T>(a0[i]);
+      }
+    }
+    store(2 * r - P, odd, even);
+    here.template pick<1, 0>(a0);
+    here.template pick<1, 1>(a1);
+    if constexpr (K == 3) here.template pick<1, 2>(a2);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      odd[i] = packed_sum<T>(a1[i]);
+      if constexpr (K == 3) even[i] = packed_sum<T>(a2[i], a0[i]);
+      else even[i] = packed_sum<T>(a0[i]);
+    }
+    store(2 * r + 1 - P, odd, even);
+    if constexpr (K == 3) {
+      here.template pick<2, 0>(up[0]);
+      here.template pick<2, 1>(up[1]);
+      here.template pick<2, 2>(up[2]);
+    }
+  }
+}
+
 template <typename T>
 int launch_backward(const void* gy, const int8_t* idx, void* gx, int64_t planes, const PoolGeom& g, cudaStream_t s) {
   const int plane_elems = g.H * g.W;
@@ -819,16 +990,23 @@ int launch_backward(const void* gy, const int8_t* idx, void* gx, int64_t planes,
     const int vec = g.Wo % 4 == 0 && aligned(gy, sizeof(T) * 4) && aligned(idx, 4);
     if (g.PH == g.PW) {
       const int pairs = (g.H - 1 + g.PH) / 2 + 1;
-      const int rows = strip_rows(planes, segs, pairs), chunks = (pairs + rows - 1) / rows;
+      // 16-bit types at 8 / 4 / 2 / 1 pairs: the shapes above 58.3 / 55.3 / 59.8 / 77.6, 41.0 / 38.0 / 42.6 / 52.8, 30.9 / 27.4 /
+      // 27.1 / 31.0 and 33.0 / 29.5 / 32.4 / 40.5
+      const int rows = strip_rows(planes, segs, pairs, sizeof(T) == 2 ? 4 : 8), chunks = (pairs + rows - 1) / rows;
       const int64_t total = planes * segs * chunks;              // <= total_segments + planes * segs
       const int sgrid = (int)((total + 255) / 256);
 #define ACTNN_STRIP(K, P)                                                                                          \
-      max_pool_backward_strip_kernel<T, K, P><<<sgrid, 256, 0, s>>>((const T*)gy, idx, (T*)gx, (uint32_t)total, segs, \
-                                                                    chunks, rows, g, vec)
-      if (g.KH == 3 && g.PW == 1) ACTNN_STRIP(3, 1);
-      else if (g.KH == 3) ACTNN_STRIP(3, 0);
-      else if (g.PW == 1) ACTNN_STRIP(2, 1);
-      else ACTNN_STRIP(2, 0);
+      {                                                                                                            \
+        auto kernel = [] {                                                                                         \
+          if constexpr (sizeof(T) == 2) return max_pool_backward_packed_kernel<T, K, P>;                           \
+          else return max_pool_backward_strip_kernel<T, K, P>;                                                     \
+        }();                                                                                                       \
+        kernel<<<sgrid, 256, 0, s>>>((const T*)gy, idx, (T*)gx, (uint32_t)total, segs, chunks, rows, g, vec);      \
+      }
+      if (g.KH == 3 && g.PW == 1) ACTNN_STRIP(3, 1)
+      else if (g.KH == 3) ACTNN_STRIP(3, 0)
+      else if (g.PW == 1) ACTNN_STRIP(2, 1)
+      else ACTNN_STRIP(2, 0)
 #undef ACTNN_STRIP
       return check_launch();
     }
