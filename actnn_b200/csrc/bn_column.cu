@@ -6,8 +6,8 @@
 //   (allocation of the widths, stats.cu)
 //   pack    codes and y from the same registers.
 // 4 + b/8 + 2 bytes an element for 16-bit types; statistics, pack and normalisation as passes of their own read x
-// three times.  float16 256 x 64 x 56 x 56: pack 28.1 + coefficients 1.6 + normalise 32.4 us -> 41.6 us (6.1 TB/s would be
-// 36, the rest is instruction issue); 128 x 256 x 14 x 14, seven launches 34 us -> four 24.6 us.
+// three times.  float16 256 x 64 x 56 x 56: pack 28.1 + coefficients 1.6 + normalise 32.4 us -> 37.6 us (6.1 TB/s would be
+// 36); 128 x 256 x 14 x 14, seven launches 34 us -> four 24.6 us.
 //
 // Backward: both passes decode the saved codes in registers, so the decoded activation is never
 // written to memory (the reference decodes it, ops.py:470-476, and cuDNN reads it back, ops.py:490-493):
@@ -17,11 +17,11 @@
 //   apply   reads the codes and dy again and writes dx, walking the samples backwards so that it
 //           starts with what the reduce left in the L2.
 // Per element of a 16-bit activation that is 2 + b/8 bytes for the reduce and 4 + b/8 for the apply,
-// against 2 (decode) + 4 + 6.  The apply moves 0.83 of the copy rate, the reduce 0.53: it is bound by its instructions
-// (393 a bundle of 1024 elements, some 200 of them decoding; issue slots 57 % busy at 16 warps an SM), not by
-// memory latency: bringing dy and the words through a ring of bulk copies in shared memory measured the same or
-// slower (42.0 / 40.6 us with 3 stages).
-// float16, 256 x 64 x 56 x 56: decode 24.9 + reduce 40.9 + apply 40.5 us -> 37.2 + 3.2 + 40.1.
+// against 2 (decode) + 4 + 6.  The apply moves 0.83 of the copy rate, the reduce 0.53.  With 16 warps an SM it issues 57 % of
+// the time, and nothing tried moved that: a ring of bulk copies for dy and the words 42.0 / 40.6 us (reduce / apply),
+// a ring of per-lane asynchronous copies without barriers 35.0 - 36.0 / 39.3 - 39.9, dy requested into the L2 ahead
+// 35.1 / 37.7, a third block an SM 36.2 / 47.6, a decode of half the instructions 32.5 / 39.4 against 32.7 / 39.5.
+// float16, 256 x 64 x 56 x 56: decode 24.9 + reduce 40.9 + apply 40.5 us -> 32.5 + 2.6 + 39.4.
 #include "column.cuh"
 
 namespace actnn {

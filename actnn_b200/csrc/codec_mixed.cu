@@ -261,8 +261,7 @@ pack_mixed_flat_kernel(const T* __restrict__ data, const T* __restrict__ mn, con
 // ---------------------------------------------------------------------------- unpack
 // Decoding a group needs only 2^B distinct outputs, code / scale + min for code = 0..2^B-1.
 // Lanes compute those once (one IEEE division per lane for up to four groups at a time)
-// and the elements look theirs up: for 16-bit types and B <= 2 the table of a group fits
-// two registers and a byte-permute picks two elements per instruction; otherwise a warp
+// and the elements look theirs up: for 16-bit types up to 3 bits by byte permutes (mixed_bundle.cuh); otherwise a warp
 // shuffle fetches the entry; from 6 bits on the division is done per element.
 // Unpack of whole groups whose count per sample is no multiple of four, or below 32: a warp task is a bundle of four
 // groups (the last one of a sample may be shorter), in the order of the stream, so that the bundles of a wide sample
@@ -387,8 +386,8 @@ struct FlatPool {
 // Same task shape as the flat pack: lane l owns group q0 + l of a task of 32 groups (its
 // sample, width, stream position, scale and min come from coalesced loads), and eight bundles
 // of four groups are decoded with the words of the next bundle already requested.  For 16-bit
-// outputs at 1 or 2 bits the lane also computes the 2^B decoded values of its own group once
-// per task (packed in two registers); a bundle then fetches them with two shuffles per group.
+// outputs of up to 3 bits the lane also computes the 2^B decoded values of its own group once
+// per task (their low and high bytes in two registers, four at 3 bits); a bundle then fetches them with a shuffle each.
 #ifndef ACTNN_UNPACK_DIRECT_FROM
 #define ACTNN_UNPACK_DIRECT_FROM 6
 #endif
