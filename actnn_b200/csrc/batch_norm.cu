@@ -72,25 +72,6 @@ struct BnShape {
   FastDiv vecs_per_plane;                                    // HW / VEC
 };
 
-// Sums (a, b) over the block in a fixed order; the result is valid in thread 0.
-ACTNN_DEV float2 block_sum2(float a, float b) {
-  __shared__ float2 warp_part[kBnThreads / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(kFull, a, o);
-    b += __shfl_xor_sync(kFull, b, o);
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) warp_part[wid] = make_float2(a, b);
-  __syncthreads();
-  float2 r = make_float2(0.f, 0.f);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int w = 0; w < kBnThreads / 32; ++w) { r.x += warp_part[w].x; r.y += warp_part[w].y; }
-  }
-  return r;
-}
-
 // Publishes this block's partial and tells whether it was the channel's last; if so, warp 0
 // of the block returns (in lane 0) the sums over the S partials in index order.
 ACTNN_DEV bool publish_and_collect(float2 mine, float2* partial, unsigned* tickets, int c, int s, int S,
@@ -157,7 +138,7 @@ bn_forward_reduce_kernel(const T* __restrict__ x, BnShape sh, float2* __restrict
     }
   }
   float2 tot;
-  if (!publish_and_collect(block_sum2(sum, sq), partial, tickets, c, s, sh.S, &tot)) return;
+  if (!publish_and_collect(block_sum2<kBnThreads>(sum, sq), partial, tickets, c, s, sh.S, &tot)) return;
   const float M = (float)sh.N * (float)sh.HW;
   const float m_s = tot.x / M;
   const float var = fmaxf(tot.y / M - m_s * m_s, 0.f);
@@ -241,7 +222,7 @@ bn_backward_reduce_kernel(const T* __restrict__ x, const T* __restrict__ dy, BnS
     }
   }
   float2 tot;
-  if (!publish_and_collect(block_sum2(sdy, sdyx), partial, tickets, c, s, sh.S, &tot)) return;
+  if (!publish_and_collect(block_sum2<kBnThreads>(sdy, sdyx), partial, tickets, c, s, sh.S, &tot)) return;
   const float M = (float)sh.N * (float)sh.HW;
   const float invstd = save_invstd[c];
   if (dbias) dbias[c] = tot.x;

@@ -3,6 +3,7 @@
 // Forward: one read of x gives the statistics and the group ranges, the second packs AND normalises:
 //   stats   min / max of the bundle's groups, sums of (x - shift) and its square per octet in registers;
 //   finish  one warp per channel: mean, inverse deviation, running statistics, coefficients;
+//           (maps of a group and more: both from the pass of bn_stats_minimax_kernel, called before)
 //   (allocation of the widths, stats.cu)
 //   pack    codes and y from the same registers.
 // 4 + b/8 + 2 bytes an element for 16-bit types; statistics, pack and normalisation as passes of their own read x
@@ -101,6 +102,11 @@ template <typename T> ACTNN_DEV float2 octet_pair_plus(const Oct<T>& o, int k, f
     }
     return r;
   }
+}
+// Element e plus a, likewise.
+template <typename T> ACTNN_DEV float octet_plus(const Oct<T>& o, int e, float a) {
+  if constexpr (sizeof(T) == 4) return o.f[e] + a;
+  else return e % 2 ? octet_pair_plus<T>(o, e / 2, 0.f, a).y : octet_pair_plus<T>(o, e / 2, a, 0.f).x;
 }
 template <typename T> ACTNN_DEV void set_octet_pair(Oct<T>& o, int k, float2 v) {
   if constexpr (sizeof(T) == 4) {
@@ -224,6 +230,25 @@ bn_column_stats_kernel(const T* __restrict__ x, ColumnShape sh, BnColumns bn, T*
   write_partials<SUB>(cc, sum, sq, partial + ((int64_t)split * sh.P + t.p) * bn.kmax, lane);
 }
 
+// Statistics of channel c from the sums of its (x - shift) and their squares.
+template <typename T>
+ACTNN_DEV void finish_channel(float2 tot, int N, int HW, int c, const T* __restrict__ x, float* __restrict__ running_mean,
+                              float* __restrict__ running_var, float* __restrict__ save_mean,
+                              float* __restrict__ save_invstd, float momentum, float eps) {
+  const float M = (float)N * (float)HW;
+  const float m_s = tot.x / M;
+  const float var = fmaxf(tot.y / M - m_s * m_s, 0.f);
+  const float mean = load_scalar<T>(x, (int64_t)c * HW) + m_s;
+  const float invstd = 1.0f / sqrtf(var + eps);
+  save_mean[c] = mean;
+  save_invstd[c] = invstd;
+  if (running_mean) running_mean[c] = (1.f - momentum) * running_mean[c] + momentum * mean;
+  if (running_var) {
+    const float unbiased = M > 1.f ? var * (M / (M - 1.f)) : var;
+    running_var[c] = (1.f - momentum) * running_var[c] + momentum * unbiased;
+  }
+}
+
 // One warp per channel.
 template <typename T>
 __global__ void __launch_bounds__(kColThreads)
@@ -235,21 +260,165 @@ bn_column_stats_finish_kernel(const float2* __restrict__ partial, ColumnShape sh
   const int c = (int)(blockIdx.x * (kColThreads / 32) + (threadIdx.x >> 5));
   if (c >= bn.C) return;
   const float2 tot = collect_partials(sh, bn, partial, c, lane);
-  if (lane != 0) return;
-  const float M = (float)sh.N * (float)bn.HW;
-  const float m_s = tot.x / M;
-  const float var = fmaxf(tot.y / M - m_s * m_s, 0.f);
-  const float mean = load_scalar<T>(x, (int64_t)c * bn.HW) + m_s;
-  const float invstd = 1.0f / sqrtf(var + eps);
-  save_mean[c] = mean;
-  save_invstd[c] = invstd;
-  if (running_mean) running_mean[c] = (1.f - momentum) * running_mean[c] + momentum * mean;
-  if (running_var) {
-    const float unbiased = M > 1.f ? var * (M / (M - 1.f)) : var;
-    running_var[c] = (1.f - momentum) * running_var[c] + momentum * unbiased;
+  if (lane == 0)
+    finish_channel<T>(tot, sh.N, bn.HW, c, x, running_mean, running_var, save_mean, save_invstd, momentum, eps);
+}
+
+// ------------------------------------------------------------------ statistics by themselves
+// Statistics and group ranges for the entry point that returns only these: maps of at least a group, whole octets and
+// samples of whole groups.  The work of a warp is the same R = min(8, HW / 256) consecutive groups of every sample of
+// its split: no more than two channels, and which of them an element belongs to does not change from sample to
+// sample.  Sums are closed once a sample: eight elements of a row, the rows, the lanes, then a partial sum per
+// channel, added up below in a fixed order.  So no chain of additions grows with the number of elements a warp
+// happens to get, and the result does not depend on the number of SMs.  (Accumulators carried down all samples of a
+// split, as in the kernel above, cost the variance of 1024 x 256 x 56 x 56 a root mean square error of 8.5e-7, against 2.1e-7.)
+// Bound by instruction issue (69 instructions a group and warp at R = 8, 87 at R = 3).  us, both launches, float16: tasks
+// strided over by persistent warps, both channels' sums kept for every octet -> this; in brackets sums down the samples:
+// 256 x 64 x 56 x 56 29.2 -> 28.0 (25.3), 256 x 512 x 28 x 28 71.0 -> 52.3 (41.3), 256 x 128 x 28 x 28 24.9 -> 19.9 (16.9),
+// 128 x 256 x 16 x 16 18.7 -> 12.8 (12.6); one task of one group a warp there: 20.8.
+struct StatShape {
+  int N, C, HW, G;
+  int R, T;           // groups per task, tasks per sample
+  int M, U;           // tasks a warp takes together, units of that per sample
+  int step;           // groups loaded at a time
+  int S, spp;         // splits of the samples, samples per split
+};
+
+constexpr int kStatRowsMax = 8;
+
+// M: four tasks of a group, two of two groups, or one of more; STEP: groups loaded at a time, three or four.
+template <typename T, int M, int STEP>
+__global__ void __launch_bounds__(kColThreads, sizeof(T) == 2 ? 3 : 2)
+bn_stats_minimax_kernel(const T* __restrict__ x, StatShape sh, T* __restrict__ mn, T* __restrict__ mx,
+                        float4* __restrict__ partial) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t warp = blockIdx.x * (kColThreads / 32) + __shfl_sync(kFull, threadIdx.x >> 5, 0);
+  const int split = (int)(warp / (uint32_t)sh.U), u = (int)(warp - (uint32_t)split * (uint32_t)sh.U);
+  if (split >= sh.S) return;
+  const int n0 = split * sh.spp, n1 = min(sh.N, n0 + sh.spp);
+  const int row0 = u * (M * sh.R), rows = min(M * sh.R, sh.G - row0);
+  const int64_t F = (int64_t)sh.G * kGroup;
+  int other[M];                    // the lane's rows of the task from which on its elements are the second channel's
+  float neg0[M], neg1[M];          // shifts: the channels' first elements
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const uint32_t e0 = (uint32_t)(row0 + m * sh.R) * kGroup, c0 = e0 / (uint32_t)sh.HW;
+    const int left = (int)min((c0 + 1) * (int64_t)sh.HW - e0, (int64_t)kStatRowsMax * kGroup);
+    other[m] = (left - lane * kOct + kGroup - 1) / kGroup;                       // HW % 8 == 0: whole octets
+    neg0[m] = c0 < (uint32_t)sh.C ? -load_scalar<T>(x, (int64_t)c0 * sh.HW) : 0.f;
+    neg1[m] = c0 + 1 < (uint32_t)sh.C ? -load_scalar<T>(x, (int64_t)(c0 + 1) * sh.HW) : 0.f;
+  }
+  auto task = [](int i) { return i * M / kBundle; };                             // of row i of a bundle
+  auto second = [&](int r0, int i) { return (M == 1 ? r0 + i : i % (kBundle / M)) >= other[task(i)]; };
+  // a row past the end reads as zeros with a shift of zero and adds nothing
+  auto shift = [&](int r0, int i) { return r0 + i >= rows ? 0.f : second(r0, i) ? neg1[task(i)] : neg0[task(i)]; };
+  auto load = [&](Oct<T> (&v)[kBundle], const T* p, int r0) {
+#pragma unroll
+    for (int i = 0; i < STEP; ++i) v[i] = r0 + i < rows ? load_oct<T>(p + (r0 + i) * kGroup) : zero_oct<T>();
+  };
+  // the samples from the last to the first: the pack starts with what is read here last
+  const T* p = x + (n1 - 1) * F + (int64_t)row0 * kGroup + lane * kOct;
+  int64_t q0 = (int64_t)(n1 - 1) * sh.G + row0 + lane;
+  float* dst = reinterpret_cast<float*>(partial + (int64_t)(n1 - 1) * sh.T + u * M) + (lane >> 3);
+  Oct<T> next[kBundle];
+#pragma unroll
+  for (int i = 0; i < kBundle; ++i) next[i] = zero_oct<T>();
+  load(next, p, 0);
+  for (int n = n1 - 1; n >= n0; --n) {
+    float2 a0[M], a1[M];           // (sum, sum of squares) of a task's two channels
+#pragma unroll
+    for (int m = 0; m < M; ++m) a0[m] = a1[m] = both(0.f);
+    for (int r0 = 0; r0 < rows; r0 += STEP) {
+      Oct<T> v[kBundle];
+#pragma unroll
+      for (int i = 0; i < kBundle; ++i) v[i] = next[i];
+      if (M == 1 && r0 + STEP < rows) {
+        load(next, p, r0 + STEP);
+      } else if (n > n0) {
+        p -= F;
+        load(next, p, 0);
+      }
+      float lo = 0.f, hi = 0.f;
+      bundle_minmax<T, STEP>(v, lane, lo, hi);
+      if (lane < min(STEP, rows - r0)) {
+        store_scalar<T>(mn, q0 + r0, lo);
+        store_scalar<T>(mx, q0 + r0, hi);
+      }
+      auto add_row = [&](int i, float2 row) {
+        const bool other_channel = second(r0, i);
+        a0[task(i)] = add2(a0[task(i)], other_channel ? both(0.f) : row);
+        a1[task(i)] = add2(a1[task(i)], other_channel ? row : both(0.f));
+      };
+#pragma unroll
+      for (int i = 0; i + 1 < STEP; i += 2) {                   // two rows, one in each half of a pair
+        const float na = shift(r0, i), nb = shift(r0, i + 1);
+        float2 s = both(0.f), q = both(0.f);
+#pragma unroll
+        for (int e = 0; e < kOct; ++e) {
+          const float2 d = make_float2(octet_plus<T>(v[i], e, na), octet_plus<T>(v[i + 1], e, nb));
+          s = add2(s, d);
+          q = fma2(d, d, q);
+        }
+        add_row(i, make_float2(s.x, q.x));
+        add_row(i + 1, make_float2(s.y, q.y));
+      }
+      if constexpr (STEP % 2) {
+        const float na = shift(r0, STEP - 1);
+        float s = 0.f, q = 0.f;
+#pragma unroll
+        for (int e = 0; e < kOct; ++e) {
+          const float d = octet_plus<T>(v[STEP - 1], e, na);
+          s += d;
+          q = fmaf(d, d, q);
+        }
+        add_row(STEP - 1, make_float2(s, q));
+      }
+    }
+    // the four sums over the warp: halves of it specialise on a channel, then quarters on sum or sum of squares;
+    // lanes 0, 8, 16, 24 end with them
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const bool hi16 = lane & 16, hi8 = lane & 8;
+      const float2 keep = hi16 ? a1[m] : a0[m], give = hi16 ? a0[m] : a1[m];
+      const float a = keep.x + __shfl_xor_sync(kFull, give.x, 16);
+      const float b = keep.y + __shfl_xor_sync(kFull, give.y, 16);
+      float t = (hi8 ? b : a) + __shfl_xor_sync(kFull, hi8 ? a : b, 8);
+      t += __shfl_xor_sync(kFull, t, 4);
+      t += __shfl_xor_sync(kFull, t, 2);
+      t += __shfl_xor_sync(kFull, t, 1);
+      if ((lane & 7) == 0 && (M == 1 || m * sh.R < rows)) dst[4 * m] = t;
+    }
+    q0 -= sh.G;
+    dst -= 4 * (int64_t)sh.T;
   }
 }
 
+// One block per channel: adds the partial sums of every task that touches it, sample after sample and task after task.
+template <typename T>
+__global__ void __launch_bounds__(kColThreads)
+bn_stats_finish_kernel(const float4* __restrict__ partial, StatShape sh, const T* __restrict__ x,
+                       float* __restrict__ running_mean, float* __restrict__ running_var, float* __restrict__ save_mean,
+                       float* __restrict__ save_invstd, float momentum, float eps) {
+  const int c = blockIdx.x;
+  const uint32_t span = (uint32_t)sh.R * kGroup, hw = (uint32_t)sh.HW;
+  const uint32_t first = (uint32_t)c * hw, last = first + hw - 1;
+  const int j_lo = (int)(first / span), j_hi = min((int)(last / span), sh.T - 1);
+  const int lo_is_second = (uint32_t)j_lo * span < first;       // only the first task can begin in the channel before
+  float sum = 0.f, sq = 0.f;
+  for (int n = threadIdx.x; n < sh.N; n += kColThreads) {
+    for (int j = j_lo; j <= j_hi; ++j) {
+      const float4 p = __ldg(partial + (int64_t)n * sh.T + j);
+      const bool second = j == j_lo && lo_is_second;
+      sum += second ? p.z : p.x;
+      sq += second ? p.w : p.y;
+    }
+  }
+  const float2 tot = block_sum2<kColThreads>(sum, sq);
+  if (threadIdx.x == 0)
+    finish_channel<T>(tot, sh.N, sh.HW, c, x, running_mean, running_var, save_mean, save_invstd, momentum, eps);
+}
+
+// ------------------------------------------------------------------ pack and normalise
 template <typename T, typename ST, int SUB, bool PHILOX, bool EDGE>
 __global__ void __launch_bounds__(kColThreads, kBnBlocks)
 bn_column_pack_kernel(const T* __restrict__ x, ColumnShape sh, BnColumns bn, const T* __restrict__ mn,
@@ -557,16 +726,31 @@ extern "C" int actnn_batch_norm_codes_workspace(int64_t N, int64_t C, int64_t HW
   return ACTNN_OK;
 }
 
-// The statistics pass by itself, for maps of whole octets and samples of whole groups.
-// (Until it ran on columns it took tasks of up to eight groups, 15.6 instructions an element for their two channels:
-// float16 256 x 64 x 56 x 56 24.1 us against 20.1, 256 x 512 x 28 x 28 and two of 256 x 128 x 28 x 28 99.5 against 49.4.)
-extern "C" int64_t actnn_batch_norm_stats_minimax_workspace(int64_t N, int64_t C, int64_t HW) {
+// The statistics pass by itself.
+static bool stats_minimax_shape(int64_t N, int64_t C, int64_t HW, StatShape& sh) {
   constexpr int64_t k31 = (int64_t)1 << 31;
   if (N <= 0 || C <= 0 || N >= k31 || C >= k31 || HW >= k31 || HW < kGroup || HW % kOct != 0 || N * C >= k31 ||
-      N * C * HW >= ((int64_t)1 << 40) || C * HW % kGroup != 0 || C * HW >= 2 * k31 - kBundle * kGroup)
-    return -1;
-  const int64_t P = (C * HW / kGroup + kBundle - 1) / kBundle;
-  return (P * N * bn_columns(C, HW).kmax * (int64_t)sizeof(float2) + 255) / 256 * 256;  // a partial sum per sample, the most there are
+      N * C * HW >= ((int64_t)1 << 40) || C * HW % kGroup != 0 || C * HW >= 2 * k31 - kStatRowsMax * kGroup)
+    return false;
+  sh.N = (int)N;
+  sh.C = (int)C;
+  sh.HW = (int)HW;
+  sh.G = (int)(C * HW / kGroup);
+  sh.R = (int)min((int64_t)kStatRowsMax, HW / kGroup);
+  sh.T = (sh.G + sh.R - 1) / sh.R;
+  sh.M = sh.R <= 2 ? kBundle / sh.R : 1;
+  sh.U = (sh.T + sh.M - 1) / sh.M;
+  const int rows = sh.M * sh.R, steps = (rows + kBundle - 1) / kBundle;
+  sh.step = (rows + steps - 1) / steps;
+  return true;
+}
+static int64_t stats_minimax_bytes(const StatShape& sh) {
+  return ((int64_t)sh.N * sh.T * (int64_t)sizeof(float4) + 255) / 256 * 256;
+}
+
+extern "C" int64_t actnn_batch_norm_stats_minimax_workspace(int64_t N, int64_t C, int64_t HW) {
+  StatShape sh;
+  return stats_minimax_shape(N, C, HW, sh) ? stats_minimax_bytes(sh) : -1;
 }
 
 extern "C" int actnn_batch_norm_stats_minimax(const void* x, void* mn, void* mx, const float* weight, const float* bias,
@@ -577,21 +761,33 @@ extern "C" int actnn_batch_norm_stats_minimax(const void* x, void* mn, void* mx,
   (void)weight;
   (void)bias;
   if (dtype < ACTNN_F32 || dtype > ACTNN_BF16) return ACTNN_ERR_DTYPE;
-  const int64_t need = actnn_batch_norm_stats_minimax_workspace(N, C, HW);
-  if (need < 0) return ACTNN_ERR_SHAPE;
+  StatShape sh;
+  if (!stats_minimax_shape(N, C, HW, sh)) return ACTNN_ERR_SHAPE;
   if (!x || !mn || !mx || !save_mean || !save_invstd || !workspace) return ACTNN_ERR_NULL;
-  if (workspace_bytes < need) return ACTNN_ERR_CAPACITY;
+  if (workspace_bytes < stats_minimax_bytes(sh)) return ACTNN_ERR_CAPACITY;
   if (!aligned(x, dtype == ACTNN_F32 ? 32 : 16) || !aligned(workspace, 16)) return ACTNN_ERR_ALIGN;
-  const BnColumns bn = bn_columns(C, HW);
-  const ColumnShape sh = bn_stats_shape(N, C, HW, kOct, dtype_size(dtype));
+  const SampleSplits splits = split_samples(N, sh.U, (dtype == ACTNN_F32 ? 2 : 3) * kColThreads / 32);
+  sh.S = splits.S;
+  sh.spp = splits.spp;
+  const int grid = (int)(((int64_t)sh.U * sh.S + kColThreads / 32 - 1) / (kColThreads / 32));
   cudaStream_t s = (cudaStream_t)stream;
-#define ACTNN_STATS(T)                                                                                             \
-  return launch_stats<T, 8, false>((const T*)x, (T*)mn, (T*)mx, running_mean, running_var, save_mean, save_invstd, \
-                                   (float)momentum, (float)eps, sh, bn, (float2*)workspace, s)
+#define ACTNN_STATS(T)                                                                                              \
+  {                                                                                                                 \
+    auto kernel = sh.M == 4 ? bn_stats_minimax_kernel<T, 4, 4>                                                      \
+                            : sh.M == 2 ? bn_stats_minimax_kernel<T, 2, 4>                                          \
+                                        : sh.step == 4 ? bn_stats_minimax_kernel<T, 1, 4>                           \
+                                                       : bn_stats_minimax_kernel<T, 1, 3>;                          \
+    kernel<<<grid, kColThreads, 0, s>>>((const T*)x, sh, (T*)mn, (T*)mx, (float4*)workspace);                       \
+    if (int st = check_launch()) return st;                                                                         \
+    bn_stats_finish_kernel<T><<<sh.C, kColThreads, 0, s>>>((const float4*)workspace, sh, (const T*)x, running_mean, \
+                                                           running_var, save_mean, save_invstd, (float)momentum,    \
+                                                           (float)eps);                                             \
+    return check_launch();                                                                                          \
+  }
   switch (dtype) {
-    case ACTNN_F32: ACTNN_STATS(float);
-    case ACTNN_F16: ACTNN_STATS(__half);
-    default: ACTNN_STATS(__nv_bfloat16);
+    case ACTNN_F32: ACTNN_STATS(float)
+    case ACTNN_F16: ACTNN_STATS(__half)
+    default: ACTNN_STATS(__nv_bfloat16)
   }
 #undef ACTNN_STATS
 }

@@ -26,6 +26,21 @@ struct ColumnShape {
 // Splits of the samples: a warp per (column, split).  The resident warps should all be busy and the
 // last wave should not be nearly empty, so the candidates are one to four waves' worth of warps and
 // the one with the fewest bundles on the critical path (plus a bundle's worth of start-up) is taken.
+struct SampleSplits { int S, spp; };
+inline SampleSplits split_samples(int64_t N, int64_t P, int warps_per_sm) {
+  const int64_t resident = (int64_t)device_info().sm_count * warps_per_sm;
+  SampleSplits r = {1, (int)N};
+  int64_t best = -1;
+  for (int k = 1; k <= 4; ++k) {
+    int64_t S = resident * k / P;
+    S = S < 1 ? 1 : S > N ? N : S;
+    const int64_t spp = (N + S - 1) / S;
+    S = (N + spp - 1) / spp;
+    const int64_t cost = (P * S + resident - 1) / resident * (spp + 1);
+    if (best < 0 || cost < best) { best = cost; r.S = (int)S; r.spp = (int)spp; }
+  }
+  return r;
+}
 inline ColumnShape column_shape(int64_t N, int64_t F, int align, int warps_per_sm) {
   ColumnShape sh;
   sh.F = F;
@@ -33,16 +48,9 @@ inline ColumnShape column_shape(int64_t N, int64_t F, int align, int warps_per_s
   sh.G = (int)((F + kGroup - 1) / kGroup);
   sh.P = (sh.G + kBundle - 1) / kBundle;
   sh.align = align;
-  const int64_t resident = (int64_t)device_info().sm_count * warps_per_sm;
-  int64_t best = -1;
-  for (int k = 1; k <= 4; ++k) {
-    int64_t S = resident * k / sh.P;
-    S = S < 1 ? 1 : S > N ? N : S;
-    const int64_t spp = (N + S - 1) / S;
-    S = (N + spp - 1) / spp;
-    const int64_t cost = (sh.P * S + resident - 1) / resident * (spp + 1);
-    if (best < 0 || cost < best) { best = cost; sh.S = (int)S; sh.spp = (int)spp; }
-  }
+  const SampleSplits splits = split_samples(N, sh.P, warps_per_sm);
+  sh.S = splits.S;
+  sh.spp = splits.spp;
   return sh;
 }
 inline int column_grid(const ColumnShape& sh) {
@@ -166,10 +174,11 @@ template <bool EDGE> struct ColumnOctets {
 };
 
 // ------------------------------------------------------------------ group min / max of a bundle
-// Lane gi (< 4) ends with the extrema of group gi.
-template <typename T> ACTNN_DEV void bundle_minmax(const Oct<T> (&x)[kBundle], int lane, float& mn, float& mx) {
+// Lane gi (< COUNT) ends with the extrema of group gi.
+template <typename T, int COUNT = kBundle>
+ACTNN_DEV void bundle_minmax(const Oct<T> (&x)[kBundle], int lane, float& mn, float& mx) {
 #pragma unroll
-  for (int gi = 0; gi < kBundle; ++gi) {
+  for (int gi = 0; gi < COUNT; ++gi) {
     float lo, hi;
     oct_minmax<T>(x[gi], lo, hi);
     lo = warp_min(lo);

@@ -152,6 +152,25 @@ ACTNN_DEV float warp_max(float v) {
   return r;
 }
 
+// Sums (a, b) over a block of THREADS in a fixed order; the result is valid in thread 0.
+template <int THREADS> ACTNN_DEV float2 block_sum2(float a, float b) {
+  __shared__ float2 warp_part[THREADS / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(kFull, a, o);
+    b += __shfl_xor_sync(kFull, b, o);
+  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) warp_part[wid] = make_float2(a, b);
+  __syncthreads();
+  float2 r = make_float2(0.f, 0.f);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) { r.x += warp_part[w].x; r.y += warp_part[w].y; }
+  }
+  return r;
+}
+
 // ------------------------------------------------------------------ 32x32 bit transpose
 // Lane r holds row r of a 32x32 bit matrix (bit c = column c).  Afterwards lane r holds
 // column r of the original (bit c = original lane c, bit r).  Five butterfly stages; per

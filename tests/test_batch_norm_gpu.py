@@ -304,3 +304,40 @@ def test_quantized_batch_norm_takes_the_one_read_path_and_matches_the_two_read_p
         assert _close(a, r, 4 * tol)
     ref = torch.nn.functional.batch_norm(x.float(), rm.clone(), rv.clone(), w, b, True, 0.1, 1e-5)
     assert _close(results[0][0].float(), ref, 4 * tol)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_error_of_the_statistics_does_not_grow_with_the_samples(cuda_device, dtype):
+    """Deviations of +-v, whose square one accumulator adds up with a rounding to the same side each time once it has
+    some hundred of them: the chains of additions stay short however many samples there are."""
+    from actnn_b200.cpp_extension import backward_func as bf
+    n, c, hw, v = 2322, 784, 256, 1 + 993 / 1024
+    x = torch.tensor([v, -v], dtype=dtype, device=cuda_device).repeat(n * c * hw // 2).view(n, c, 16, 16)
+    x[0, :, 0, 0] = 0                                         # the kernel's shift: deviations are the values themselves
+    invstd = bf.batch_norm_stats_minimax(x, None, None, None, None, 0.1, 1e-5)[3].double()
+    m = n * hw
+    var = (m - 1) / m * v * v - (v / m) ** 2
+    # positive terms: 8 additions in a row, 5 over the lanes, ceil(n / 256) + 13 over the samples, a rounding each; half
+    # of that for the root, and four roundings to the result
+    bound = ((8 + 5 + -(-n // 256) + 13) / 2 + 4) * 2 ** -24
+    assert ((invstd * (var + 1e-5) ** 0.5 - 1).abs() <= bound).all()
+
+
+# maps of 1, 2, 3 .. 8 and more whole groups, last tasks of a sample that are shorter, one sample and several a warp
+@pytest.mark.parametrize("shape", [(3, 7, 16, 16), (2, 3, 16, 32), (5, 6, 24, 32), (4, 1, 32, 32), (3, 5, 32, 40), (2, 2, 48, 32),
+                                   (6, 4, 32, 56), (9, 1, 48, 48), (700, 128, 16, 16), (900, 40, 24, 24), (700, 64, 32, 24)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_statistics_and_group_minmax_of_all_task_lengths(cuda_device, shape, dtype):
+    from actnn_b200.cpp_extension import backward_func as bf
+    gen = torch.Generator(device=cuda_device).manual_seed(shape[0])
+    shift = torch.linspace(-3, 3, shape[1], device=cuda_device).view(1, -1, 1, 1)
+    x = (torch.randn(shape, device=cuda_device, generator=gen) + shift).to(dtype)
+    mn, mx, mean, invstd = bf.batch_norm_stats_minimax(x, None, None, None, None, 0.1, 1e-5)
+    groups = x.view(shape[0], -1, 256)
+    assert torch.equal(mn.view(groups.shape[:2]), groups.amin(2)) and torch.equal(mx.view(groups.shape[:2]), groups.amax(2))
+    xd = x.double()
+    m, var = xd.mean((0, 2, 3)), xd.var((0, 2, 3), unbiased=False)
+    # sums of |x - shift| and its square (the shift within six deviations) in chains and trees of under 48 roundings
+    dev = torch.sqrt(var) + 6 * torch.sqrt(var)
+    assert ((mean.double() - m).abs() <= 48 * 2 ** -24 * (dev + m.abs())).all()
+    assert ((invstd.double() * torch.sqrt(var + 1e-5) - 1).abs() <= 48 * 2 ** -24 * (dev ** 2 / var)).all()
