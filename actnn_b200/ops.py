@@ -222,10 +222,27 @@ class _autocast_off:
         return False
 
 
-def _start_allocation(scheme):
-    start = getattr(scheme, "start_allocation", None)
-    if start is not None:
-        start()
+class _scheme_step:
+    """What the scheme of a layer does around the layer's backward: the gradient scale and, in the layer that ends the
+    step, the start of the widths' allocation before it, the allocation's end after it.  When the backward fails, the
+    widths stay and nothing of the allocation is kept."""
+
+    def __init__(self, scheme, grad_output):
+        self.scheme, self.grad_output = scheme, grad_output
+
+    def __enter__(self):
+        if self.scheme:
+            self.scheme.set_scale(self.grad_output)
+            start = getattr(self.scheme, "start_allocation", None)
+            if start is not None:
+                start()
+
+    def __exit__(self, failure, *exc):
+        if self.scheme and failure is None:
+            self.scheme.if_allocate_perlayer()
+        elif getattr(self.scheme, "_started", None) is not None:
+            self.scheme._started = None
+        return False
 
 
 def _debug_forward(tag, quantized):
@@ -271,41 +288,37 @@ class convnd(Function):
 
     @staticmethod
     def run_backward(n, ctx, grad_output, bias_reduce_dims, aug):
-        if ctx.scheme:
-            ctx.scheme.set_scale(grad_output)
-            _start_allocation(ctx.scheme)
-        q_input_shape, stride, padding, dilation, groups, in_dtype = ctx.other_args
-        padding, stride, dilation = aug(padding), aug(stride), aug(dilation)
-        quantized, weight, bias = ctx.saved
-        input = dequantize_activation(quantized, q_input_shape, in_dtype)
-        del quantized, ctx.saved
-        empty_cache(config.empty_cache_threshold)
-        if config.debug_memory_op_backward:
-            global conv2d_layer_ct
-            print("========== conv%dd backward %d ==========" % (n, conv2d_layer_ct))
-            get_memory_usage(True)
-            conv2d_layer_ct += 1
-            print("WS: %.2f MB" % (compute_tensor_bytes([grad_output, input, input]) / 1024 ** 2))
+        with _scheme_step(ctx.scheme, grad_output):
+            q_input_shape, stride, padding, dilation, groups, in_dtype = ctx.other_args
+            padding, stride, dilation = aug(padding), aug(stride), aug(dilation)
+            quantized, weight, bias = ctx.saved
+            input = dequantize_activation(quantized, q_input_shape, in_dtype)
+            del quantized, ctx.saved
+            empty_cache(config.empty_cache_threshold)
+            if config.debug_memory_op_backward:
+                global conv2d_layer_ct
+                print("========== conv%dd backward %d ==========" % (n, conv2d_layer_ct))
+                get_memory_usage(True)
+                conv2d_layer_ct += 1
+                print("WS: %.2f MB" % (compute_tensor_bytes([grad_output, input, input]) / 1024 ** 2))
 
-        grad_output = grad_output.to(input.dtype)
-        needs = [ctx.needs_input_grad[0], ctx.needs_input_grad[1]]
-        use_pipeline = bool(config.pipeline_threshold) and all(needs) and \
-            compute_tensor_bytes([grad_output, input, input]) > config.pipeline_threshold
-        args = (padding, stride, dilation, groups)
-        if use_pipeline:
-            grad_input, grad_weight = _chunked_conv_backward(
-                ext_backward_func.cudnn_convolution_backward, input, grad_output, weight, args, needs)
-        elif n == 2 and ext_backward_func.channels_last_pays(input, weight, groups):
-            grad_input, grad_weight = (g if g is None else ext_backward_func.to_planes(g) for g in
-                                       ext_backward_func.cudnn_convolution_backward(
-                ext_backward_func.to_channels_last(input), ext_backward_func.to_channels_last(grad_output.contiguous()),
-                ext_backward_func.to_channels_last(weight), *args, config.cudnn_benchmark_conv2d, False, False, needs))
-        else:
-            grad_input, grad_weight = ext_backward_func.cudnn_convolution_backward(
-                input, grad_output, weight, *args, config.cudnn_benchmark_conv2d, False, False, needs)
-        grad_bias = grad_output.sum(bias_reduce_dims) if bias is not None and ctx.needs_input_grad[2] else None
-        if ctx.scheme:
-            ctx.scheme.if_allocate_perlayer()
+            grad_output = grad_output.to(input.dtype)
+            needs = [ctx.needs_input_grad[0], ctx.needs_input_grad[1]]
+            use_pipeline = bool(config.pipeline_threshold) and all(needs) and \
+                compute_tensor_bytes([grad_output, input, input]) > config.pipeline_threshold
+            args = (padding, stride, dilation, groups)
+            if use_pipeline:
+                grad_input, grad_weight = _chunked_conv_backward(
+                    ext_backward_func.cudnn_convolution_backward, input, grad_output, weight, args, needs)
+            elif n == 2 and ext_backward_func.channels_last_pays(input, weight, groups):
+                grad_input, grad_weight = (g if g is None else ext_backward_func.to_planes(g) for g in
+                                           ext_backward_func.cudnn_convolution_backward(
+                    ext_backward_func.to_channels_last(input), ext_backward_func.to_channels_last(grad_output.contiguous()),
+                    ext_backward_func.to_channels_last(weight), *args, config.cudnn_benchmark_conv2d, False, False, needs))
+            else:
+                grad_input, grad_weight = ext_backward_func.cudnn_convolution_backward(
+                    input, grad_output, weight, *args, config.cudnn_benchmark_conv2d, False, False, needs)
+            grad_bias = grad_output.sum(bias_reduce_dims) if bias is not None and ctx.needs_input_grad[2] else None
         return grad_input, grad_weight, grad_bias, None, None, None, None, None
 
 
@@ -345,36 +358,32 @@ class conv_transposend(Function):
 
     @staticmethod
     def run_backward(n, ctx, grad_output, bias_reduce_dims, aug):
-        if ctx.scheme:
-            ctx.scheme.set_scale(grad_output)
-            _start_allocation(ctx.scheme)
-        q_input_shape, stride, padding, output_padding, dilation, groups, in_dtype = ctx.other_args
-        padding, output_padding, stride, dilation = aug(padding), aug(output_padding), aug(stride), aug(dilation)
-        quantized, weight, bias = ctx.saved
-        input = dequantize_activation(quantized, q_input_shape, in_dtype)
-        del quantized, ctx.saved
-        empty_cache(config.empty_cache_threshold)
-        if config.debug_memory_op_backward:
-            global conv2d_layer_ct
-            print("========== conv%dd_transpose backward %d ==========" % (n, conv2d_layer_ct))
-            get_memory_usage(True)
-            conv2d_layer_ct += 1
-            print("WS: %.2f MB" % (compute_tensor_bytes([grad_output, input, input]) / 1024 ** 2))
+        with _scheme_step(ctx.scheme, grad_output):
+            q_input_shape, stride, padding, output_padding, dilation, groups, in_dtype = ctx.other_args
+            padding, output_padding, stride, dilation = aug(padding), aug(output_padding), aug(stride), aug(dilation)
+            quantized, weight, bias = ctx.saved
+            input = dequantize_activation(quantized, q_input_shape, in_dtype)
+            del quantized, ctx.saved
+            empty_cache(config.empty_cache_threshold)
+            if config.debug_memory_op_backward:
+                global conv2d_layer_ct
+                print("========== conv%dd_transpose backward %d ==========" % (n, conv2d_layer_ct))
+                get_memory_usage(True)
+                conv2d_layer_ct += 1
+                print("WS: %.2f MB" % (compute_tensor_bytes([grad_output, input, input]) / 1024 ** 2))
 
-        grad_output = grad_output.to(input.dtype)
-        needs = [ctx.needs_input_grad[0], ctx.needs_input_grad[1]]
-        use_pipeline = bool(config.pipeline_threshold) and all(needs) and \
-            compute_tensor_bytes([grad_output, input, input]) > config.pipeline_threshold
-        args = (padding, output_padding, stride, dilation, groups)
-        if use_pipeline:
-            grad_input, grad_weight = _chunked_conv_backward(
-                ext_backward_func.cudnn_convolution_transpose_backward, input, grad_output, weight, args, needs)
-        else:
-            grad_input, grad_weight = ext_backward_func.cudnn_convolution_transpose_backward(
-                input, grad_output, weight, *args, config.cudnn_benchmark_conv2d, False, False, needs)
-        grad_bias = grad_output.sum(bias_reduce_dims) if bias is not None and ctx.needs_input_grad[2] else None
-        if ctx.scheme:
-            ctx.scheme.if_allocate_perlayer()
+            grad_output = grad_output.to(input.dtype)
+            needs = [ctx.needs_input_grad[0], ctx.needs_input_grad[1]]
+            use_pipeline = bool(config.pipeline_threshold) and all(needs) and \
+                compute_tensor_bytes([grad_output, input, input]) > config.pipeline_threshold
+            args = (padding, output_padding, stride, dilation, groups)
+            if use_pipeline:
+                grad_input, grad_weight = _chunked_conv_backward(
+                    ext_backward_func.cudnn_convolution_transpose_backward, input, grad_output, weight, args, needs)
+            else:
+                grad_input, grad_weight = ext_backward_func.cudnn_convolution_transpose_backward(
+                    input, grad_output, weight, *args, config.cudnn_benchmark_conv2d, False, False, needs)
+            grad_bias = grad_output.sum(bias_reduce_dims) if bias is not None and ctx.needs_input_grad[2] else None
         return grad_input, grad_weight, grad_bias, None, None, None, None, None, None
 
 
@@ -412,26 +421,22 @@ class linear(Function):
 
     @staticmethod
     def backward(ctx, grad_output):
-        if ctx.scheme:
-            ctx.scheme.set_scale(grad_output)
-            _start_allocation(ctx.scheme)
-        quantized, weight, bias = ctx.saved
-        q_input_shape, in_dtype = ctx.other_args
-        input = dequantize_activation(quantized, q_input_shape, in_dtype)
-        del quantized, ctx.saved
-        empty_cache(config.empty_cache_threshold)
+        with _scheme_step(ctx.scheme, grad_output):
+            quantized, weight, bias = ctx.saved
+            q_input_shape, in_dtype = ctx.other_args
+            input = dequantize_activation(quantized, q_input_shape, in_dtype)
+            del quantized, ctx.saved
+            empty_cache(config.empty_cache_threshold)
 
-        grad_output = grad_output.to(input.dtype)
-        go, x = grad_output, input
-        if go.dim() != 2 or x.dim() != 2:
-            go, x = go.reshape(-1, go.shape[-1]), x.reshape(-1, x.shape[-1])
-        grad_input = go.mm(weight)
-        if grad_input.shape != q_input_shape:
-            grad_input = grad_input.view(q_input_shape)
-        grad_weight = go.t().mm(x)
-        grad_bias = go.sum(0) if bias is not None else None
-        if ctx.scheme:
-            ctx.scheme.if_allocate_perlayer()
+            grad_output = grad_output.to(input.dtype)
+            go, x = grad_output, input
+            if go.dim() != 2 or x.dim() != 2:
+                go, x = go.reshape(-1, go.shape[-1]), x.reshape(-1, x.shape[-1])
+            grad_input = go.mm(weight)
+            if grad_input.shape != q_input_shape:
+                grad_input = grad_input.view(q_input_shape)
+            grad_weight = go.t().mm(x)
+            grad_bias = go.sum(0) if bias is not None else None
         return grad_input, grad_weight, grad_bias, None
 
 

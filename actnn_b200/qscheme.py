@@ -258,7 +258,7 @@ class QScheme(object):
         256 x 256 x 28 x 28 with its ReLU 1048 -> 899 us, bottleneck block at batch 256 2053 -> 1875; where the GPU waits
         for the host anyway the event costs what it saves (classifier head at batch 256 788 -> 801)."""
         self._started = None
-        if QScheme.allocate_perlayer is _allocate_perlayer and self._closes_step():
+        if QScheme.allocate_perlayer is _allocate_perlayer and self._closes_step():    # a program's own: at the end
             self._started = QScheme.start_perlayer()
 
     def if_allocate_perlayer(self):
@@ -275,4 +275,6 @@ class QScheme(object):
         QBNScheme.allocate_perlayer()
 
 
+# A program may put its own function in the place of QScheme.allocate_perlayer (the reference calls it by that name,
+# actnn/actnn/qscheme.py:146): it is then called without arguments, after the last backward, and nothing starts before.
 _allocate_perlayer = QScheme.allocate_perlayer
