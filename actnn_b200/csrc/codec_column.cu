@@ -137,10 +137,10 @@ int column_minimax(const void* data, void* mn, void* mx, int64_t N, int64_t F, i
 
 int column_pack(const void* data, const void* mn, const void* mx, const int32_t* bits, const int64_t* word_offsets,
                 int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t F, int dtype, int stat_dtype,
-                int stochastic, const void* noise, uint64_t seed, uint64_t offset, cudaStream_t s) {
+                int stochastic, const void* noise, uint64_t seed, uint64_t offset, double width, cudaStream_t s) {
   if (!column_supported(N, F)) return ACTNN_ERR_SHAPE;
   if (stochastic && noise && !aligned(noise, dtype == ACTNN_F32 ? 32 : 16)) return ACTNN_ERR_ALIGN;
-  if (ragged_pays(N, F))
+  if (ragged_pays(N, F, dtype, width))
     return ragged_pack(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, F, dtype, stat_dtype, stochastic,
                        noise, seed, offset, s);
 #define ACTNN_PACK(T, ST)                                                                                         \

@@ -742,7 +742,7 @@ namespace actnn {
 int pack_mixed_impl(const void* data, const void* mn, const void* mx, const int32_t* bits,
                     const int64_t* word_offsets, int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t G,
                     int64_t group_size, int dtype, int stat_dtype, int stochastic, const void* noise, uint64_t seed,
-                    uint64_t offset, bool min_is_exact, cudaStream_t s) {
+                    uint64_t offset, bool min_is_exact, double width, cudaStream_t s) {
   if (int st = check_common(N, G, group_size, dtype, stat_dtype)) return st;
   if (N == 0 || G == 0) return ACTNN_OK;
   if (!data || !mn || !mx || !bits || !word_offsets || !packed || !scale) return ACTNN_ERR_NULL;
@@ -755,7 +755,7 @@ int pack_mixed_impl(const void* data, const void* mn, const void* mx, const int3
   // take the column kernels, which the step-by-step entry (min not known to be exact) does not have
   if (min_is_exact && mn_out && (G % kFlatBundle != 0 || G < kFlatGroups))
     return column_pack(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, G * kGroup, dtype, stat_dtype,
-                       stochastic, noise, seed, offset, s);
+                       stochastic, noise, seed, offset, width, s);
   switch (dtype) {
     case ACTNN_F16:
       return launch_pack<__half, __half>(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, G,
@@ -779,7 +779,7 @@ extern "C" int actnn_pack_mixed(const void* data, const void* mn, const void* mx
                                 int stochastic, const void* noise, uint64_t seed, uint64_t offset,
                                 actnn_stream_t stream) {
   return pack_mixed_impl(data, mn, mx, bits, word_offsets, packed, scale, mn_out, N, G, group_size, dtype,
-                         stat_dtype, stochastic, noise, seed, offset, false, (cudaStream_t)stream);
+                         stat_dtype, stochastic, noise, seed, offset, false, 8.0, (cudaStream_t)stream);
 }
 
 extern "C" int actnn_bad_width_bundles(uint32_t* count) {

@@ -4,8 +4,8 @@
 // The bundles are the aligned groups 4k .. 4k+3 of the flat [N * G] list, as in the kernels for whole groups, so that a
 // call of the noise generator serves each (columns of an odd G need two), and a bundle inside a sample is
 // addressed and packed as there: only the sample's offset differs.  What is special happens in one bundle or two a
-// sample, those that hold its last, partial group or groups of two samples; they are taken group by group.  Every warp
-// gets an equal share of consecutive bundles and prepares up to 32 groups at a time, a group a lane.
+// sample, those that hold its last, partial group or groups of two samples; they are taken group by group.  A warp
+// prepares up to 32 groups at a time, a group a lane.
 // What bounds it: instruction issue (the generator, rounding); it runs at the pace of the pack of whole groups.
 #include "flat_runs.cuh"
 
@@ -20,23 +20,31 @@ struct RaggedShape {
   int64_t pad;                // elements missing in the last group of a sample
 };
 
-// The warp's share of the bundles, up to eight at a time.
-struct BundleShare {
-  int64_t next, left;
-  ACTNN_DEV BundleShare(int64_t Q) {
-    const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * kThreads) >> 5;
+// The bundles in tasks of up to eight, all of the same length or one less and as many for every warp; the warps take
+// them in turn.  So the warps of a block are on neighbouring groups, mostly of one sample and one width, and share its
+// code in the instruction caches, and every warp meets all parts of the activation.  (One run of consecutive bundles a
+// warp had the warps of a block on different samples, and was slower than the columns where widths are many: float16
+// compress of 512 x 785 groups, columns / runs / tasks in turn, 2 bits on average 120 / 103 / 96 us, 4 bits 128 / 147 /
+// 113, 6 bits 136 / 158 / 129; float32 170 / 162 / 157, 178 / 211 / 165, 185 / 210 / 171.)
+// FROM_END: the last task first, for float32: 200 x 900 groups 79.9 -> 74.0 us; float16 49.4 -> 49.0, 512 x 785 95.0 -> 97.1.
+template <bool FROM_END> struct BundleTasks {
+  int64_t next, stride, tasks, base, rem;
+  ACTNN_DEV BundleTasks(int64_t Q) {
     const int64_t total = (Q + kFlatBundle - 1) / kFlatBundle;
-    const int64_t base = total / nwarps, rem = total - base * nwarps;
-    next = warp * base + min(warp, rem);
-    left = base + (warp < rem ? 1 : 0);
+    constexpr int kMost = kFlatGroups / kFlatBundle;
+    next = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
+    stride = ((int64_t)gridDim.x * kThreads) >> 5;
+    tasks = min((total + stride * kMost - 1) / (stride * kMost) * stride, total);
+    base = total / tasks;
+    rem = total - base * tasks;
   }
+  // Bundles of the next task, which begins with group q0; zero: no more.
   ACTNN_DEV int take(int64_t& q0) {
-    const int n = (int)min(left, (int64_t)(kFlatGroups / kFlatBundle));
-    q0 = next * kFlatBundle;
-    next += n;
-    left -= n;
-    return n;
+    if (next >= tasks) return 0;
+    const int64_t t = FROM_END ? tasks - 1 - next : next;
+    q0 = (t * base + min(t, rem)) * kFlatBundle;
+    next += stride;
+    return (int)(base + (t < rem ? 1 : 0));
   }
 };
 
@@ -97,10 +105,9 @@ pack_ragged_kernel(const T* __restrict__ data, const T* __restrict__ mn, const T
   const int lane = threadIdx.x & 31;
   const TransposePlan plan = make_transpose_plan(lane);
   Oct<T> bufA[kFlatBundle], bufB[kFlatBundle];                  // bufB stays unused without PREFETCH
-  BundleShare share(sh.Q);
-  while (share.left > 0) {
-    int64_t q0;
-    const int bundles = share.take(q0);
+  BundleTasks<sizeof(T) == 4> tasks(sh.Q);
+  int64_t q0;
+  while (const int bundles = tasks.take(q0)) {
     const LaneGroup g(sh, q0, bundles, lane);
     int b_l = 0;
     int64_t off_l = 0;
@@ -214,14 +221,26 @@ int launch_pack(const void* data, const void* mn, const void* mx, const int32_t*
 
 }  // namespace
 
-// Where the bundles inside a sample outweigh its last one or two, and every warp gets a few of them.  us, columns against
-// this, widths around 2 bits, whole octets: float16 100 x 919 groups 20.0 / 14.5, 50 x 919 11.1 / 9.2, 30 x 919 7.7 / 7.9, 200 x 259
-// 13.0 / 10.0, 300 x 919 (octets on 4 elements) 61.9 / 43.2, 16 x 7442 24.3 / 16.7; 200 x 130 7.3 / 7.9, 1000 x 130 26.4 / 23.7
-// but 28.5 / 35.5 around 4 bits, 4000 x 33 30.2 / 32.5; float32 100 x 919 24.9 / 21.7, 200 x 259 15.6 / 12.7, 30 x 919 9.2 / 8.9.
+// Where the bundles inside a sample outweigh its last one or two, and every warp gets a few of them.  How many groups a
+// sample that takes depends on how many widths the warps of a block meet, of which the host knows the average (`width`; 1:
+// all the same): the columns keep all warps on one sample.  us of a compress, columns / this, float16 except where noted;
+// the samples' scales spread as exp(0.7 randn):
+//   2 bits   160 x 256 groups 20.3 / 19.7, 200 x 259 24.8 / 22.1, 400 x 300 39.3 / 39.5, 512 x 257 48.9 / 42.9, 1024 x 257 91.3 /
+//            83.3, 50 x 919 22.3 / 20.1, 100 x 919 33.6 / 28.1, 16 x 7442 46.5 / 35.8; but 300 x 130 23.4 / 23.2, 1000 x 130 53.3 / 55.1
+//   3 bits   200 x 259 25.4 / 23.9, 300 x 400 41.6 / 39.7, 400 x 440 54.5 / 53.3, 512 x 401 72.9 / 62.6; but 256 x 256 27.0 / 29.5,
+//            400 x 300 40.8 / 43.3; float32 400 x 440 82.9 / 78.0, 400 x 300 59.2 / 59.2
+//   4 bits   256 x 515 50.0 / 43.4, 512 x 401 72.3 / 69.4, 400 x 440 56.9 / 57.9, 2000 x 401 555 / 560 (spread as exp(0.3 randn) 55.7 /
+//            53.2 and 551 / 508); but 200 x 300 26.6 / 29.1, 400 x 300 41.8 / 46.3; float32 400 x 440 85.4 / 81.1, 400 x 300 61.0 / 62.9
+//   6 bits   64 x 641 23.4 / 21.5, 512 x 785 136 / 129; but 512 x 401 77.8 / 75.5, 400 x 440 60.2 / 67.4, 1024 x 513 180 / 188; float32
+//            512 x 401 105.9 / 96.9, 400 x 440 89.5 / 85.0
+//   all of 8 200 x 259 25.4 / 23.1, 512 x 785 135 / 113, 400 x 300 42.4 / 41.8
 // (The unpack has no generator to save and stays with the columns: 13.3 against 17.5, 100 x 919.)
-bool ragged_pays(int64_t N, int64_t F) {
+bool ragged_pays(int64_t N, int64_t F, int dtype, double width) {
   const int64_t G = (F + kGroup - 1) / kGroup;
-  return G >= 256 && N * G >= 40960 && N * G < ((int64_t)1 << 31);
+  int64_t least = 256;
+  if (width > 2 && (width > 3 || N > 200)) least = 384;
+  if (width > 4 && dtype != ACTNN_F32) least = 640;
+  return G >= least && N * G >= 40960 && N * G < ((int64_t)1 << 31);
 }
 
 int ragged_pack(const void* data, const void* mn, const void* mx, const int32_t* bits, const int64_t* word_offsets,

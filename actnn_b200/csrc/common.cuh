@@ -274,11 +274,11 @@ int check_launch();                                // api.cu: cudaPeekAtLastErro
 unsigned* bulk_wait_counter();                     // api.cu: device counter of bulk-copy waits that gave up
 
 // codec_mixed.cu: actnn_pack_mixed with one more promise from the caller, `min_is_exact`
-// (every mn[q] is the true minimum of its group, as after actnn_minimax).
+// (every mn[q] is the true minimum of its group, as after actnn_minimax), and the `allocation_width`.
 int pack_mixed_impl(const void* data, const void* mn, const void* mx, const int32_t* bits,
                     const int64_t* word_offsets, int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t G,
                     int64_t group_size, int dtype, int stat_dtype, int stochastic, const void* noise, uint64_t seed,
-                    uint64_t offset, bool min_is_exact, cudaStream_t stream);
+                    uint64_t offset, bool min_is_exact, double width, cudaStream_t stream);
 
 // codec_column.cu: min / max, pack and unpack of [N, F] activations, any F (groups of 256; elements past
 // the end of a sample count as zeros in its last group).  `mn` must be the true group minima.
@@ -286,12 +286,16 @@ int column_minimax(const void* data, void* mn, void* mx, int64_t N, int64_t F, i
                    cudaStream_t stream);
 int column_pack(const void* data, const void* mn, const void* mx, const int32_t* bits, const int64_t* word_offsets,
                 int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t F, int dtype, int stat_dtype,
-                int stochastic, const void* noise, uint64_t seed, uint64_t offset, cudaStream_t stream);
+                int stochastic, const void* noise, uint64_t seed, uint64_t offset, double width, cudaStream_t stream);
 int column_unpack(const int32_t* packed, const int32_t* bits, const int64_t* word_offsets, const void* scale,
                   const void* mn, void* out, int64_t N, int64_t F, int dtype, int stat_dtype, cudaStream_t stream);
 
-// codec_ragged.cu: the same pack for large activations (`ragged_pays`).
-bool ragged_pays(int64_t N, int64_t F);
+// codec_ragged.cu: the same pack for large activations (`ragged_pays`).  `width`: the average of the allocation, as far as
+// it says how many widths there are; all the same count as 1.
+inline double allocation_width(int64_t N, int initial_bits, double target) {
+  return target >= (double)N * initial_bits ? 1.0 : target / (double)N;
+}
+bool ragged_pays(int64_t N, int64_t F, int dtype, double width);
 int ragged_pack(const void* data, const void* mn, const void* mx, const int32_t* bits, const int64_t* word_offsets,
                 int32_t* packed, void* scale, void* mn_out, int64_t N, int64_t F, int dtype, int stat_dtype,
                 int stochastic, const void* noise, uint64_t seed, uint64_t offset, cudaStream_t stream);

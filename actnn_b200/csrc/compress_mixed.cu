@@ -55,7 +55,8 @@ extern "C" int actnn_compress_mixed(const void* data, int32_t* packed, void* sca
     if (st) return st;
   }
   return pack_mixed_impl(data, mn, mx, bits_out, word_offsets_out, packed, scale, mn_out, N, G, group_size, dtype,
-                         stat_dtype, stochastic, noise, seed, offset, true, (cudaStream_t)stream);
+                         stat_dtype, stochastic, noise, seed, offset, true,
+                         allocation_width(N, initial_bits, target), (cudaStream_t)stream);
 }
 
 // The same compress of [N, F] samples that need not be whole groups: the last group of a sample is
@@ -100,7 +101,7 @@ extern "C" int actnn_compress_mixed_samples(const void* data, int32_t* packed, v
       return st;
   }
   return column_pack(data, mn, mx, bits_out, word_offsets_out, packed, scale, mn_out, N, F, dtype, stat_dtype,
-                     stochastic, noise, seed, offset, s);
+                     stochastic, noise, seed, offset, allocation_width(N, initial_bits, target), s);
 }
 
 // The same compress when the per-group min / max already exist (actnn_batch_norm_stats_minimax
@@ -136,7 +137,8 @@ static int compress_prestat(const void* data, const void* mn, const void* mx, in
     if (st) return st;
   }
   return pack_mixed_impl(data, mn, mx, bits_out, word_offsets_out, packed, scale, mn_out, N, G, group_size, dtype,
-                         stat_dtype, stochastic, noise, seed, offset, true, s);
+                         stat_dtype, stochastic, noise, seed, offset, true,
+                         allocation_width(N, initial_bits, target), s);
 }
 
 extern "C" int actnn_compress_mixed_prestat(const void* data, const void* mn, const void* mx, int32_t* packed,
