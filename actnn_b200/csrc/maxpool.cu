@@ -705,8 +705,9 @@ max_pool_backward_s2_kernel(const T* __restrict__ gy, const int8_t* __restrict__
 // reach the first through their last row (window row r - 1) and their first (r), the second through their middle
 // row (r) only, so every window row is loaded once per strip, kept for the next pair, and only the
 // 9 / 4 candidates a position has on average are compared (the segment kernel compares 2 rows of 5 for every row).
-// The order of additions is that of the general kernel.  float16 128 x 64 x 112 x 112, 3 x 3 / 2 (282 MB): segment
-// kernel 128.0 us, bound by instruction issue; strips 71.7, with the next window row requested ahead 63.8.
+// The order of additions is that of the general kernel.  float16 128 x 64 x 112 x 112, 3 x 3 / 2 (282 MB), when this
+// kernel took it: segment kernel 128.0 us, bound by instruction issue; strips 71.7, with the next window row requested ahead
+// 63.8.  Now float32's alone: 16-bit types take the packed kernel below.
 template <typename T, int K, int P> struct PoolWindows {
   static constexpr int BLO = (K == 3 && P == 0) ? -1 : 0, BHI = P == 1 ? 4 : 3, NB = BHI - BLO + 1;
   static constexpr bool kSide = NB == 5;                         // a fifth window column, left (BLO) or right (BHI) of the four
@@ -774,6 +775,7 @@ template <typename T, int K, int P>
 __global__ void __launch_bounds__(256)
 max_pool_backward_strip_kernel(const T* __restrict__ gy, const int8_t* __restrict__ idx, T* __restrict__ gx,
                                uint32_t total, int segs, int chunks, int rows, PoolGeom g, int vector_load) {
+  static_assert(sizeof(T) == 4, "16-bit types take the packed kernel below");
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= total) return;
   const uint32_t strip = t / (uint32_t)segs;
@@ -787,14 +789,8 @@ max_pool_backward_strip_kernel(const T* __restrict__ gy, const int8_t* __restric
   auto store = [&](int h, const float (&acc)[8]) {
     if (h < 0 || h >= g.H) return;
     Oct<T> o;
-    if constexpr (sizeof(T) == 4) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o.f[j] = acc[j];
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        o.r[k] = bits_of<T>(round_to<T>(acc[2 * k])) | (bits_of<T>(round_to<T>(acc[2 * k + 1])) << 16);
-    }
+    for (int j = 0; j < 8; ++j) o.f[j] = acc[j];
     store_oct<T>(out + (int64_t)h * g.W, o);
   };
   using Windows = PoolWindows<T, K, P>;
