@@ -681,8 +681,7 @@ int launch_forward(const void* x, void* y, const BnForward& f, const ColumnShape
       return st;
   }
   auto pack = f.stochastic ? bn_column_pack_kernel<T, ST, SUB, true, EDGE> : bn_column_pack_kernel<T, ST, SUB, false, EDGE>;
-  // Large 16-bit activations: requested into the L2 a sample ahead of the loads, while y goes out.  The line lies between
-  // the sizes that were measured, 15 MB and 40 MB.
+  // 16-bit activations that do not stay in the L2: requested there a sample ahead of the loads, while y goes out.
   // float16 256 x 64 x 56 x 56 41.5 -> 37.6 us (two samples ahead 38.0, three 38.3), 256 x 128 x 28 x 28 21.8 -> 19.8, 200 x
   // 64 x 40 x 40 18.1 -> 16.8; at 15 MB (64 x 100 x 35 x 35) 19.3 -> 19.6, and float32 pays: 76.5 -> 80.
   const bool ahead = sizeof(T) == 2 && (int64_t)sh.N * sh.F >= ((int64_t)16 << 20);

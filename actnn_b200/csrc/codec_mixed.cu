@@ -304,17 +304,10 @@ unpack_mixed_kernel(const int32_t* __restrict__ packed, const int32_t* __restric
         const int b = __ldg(bits + c.n);
         if (b >= 1 && b <= 8) t_b[d] = b;
         const int32_t* in = packed + (__ldg(word_offsets + c.n) + (int64_t)c.g0 * 8 * t_b[d]);
-        const int words = c.count * 8 * t_b[d];
-        if (kNibbles<T, 3> && t_b[d] <= 3) {                  // warp-uniform
-          const int base = order.base(t_b[d]), step = order.step(t_b[d]);
+        const int base = order.base(t_b[d]), step = order.step(t_b[d]), words = c.count * 8 * t_b[d];
 #pragma unroll
-          for (int k = 0; k < 3; ++k)
-            if (k < t_b[d] && base + k * step < words) t_w[d][k] = (uint32_t)__ldg(in + base + k * step);
-        } else {
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (k * 32 + lane < words) t_w[d][k] = (uint32_t)__ldg(in + k * 32 + lane);
-        }
+        for (int k = 0; k < 8; ++k)
+          if (k < t_b[d] && base + k * step < words) t_w[d][k] = (uint32_t)__ldg(in + base + k * step);
         if (lane < c.count) {
           t_sc[d] = load_scalar<ST>(scale, c.q0 + lane);
           t_m[d] = load_scalar<ST>(mn, c.q0 + lane);
