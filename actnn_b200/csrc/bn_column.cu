@@ -445,7 +445,8 @@ bn_column_pack_kernel(const T* __restrict__ x, ColumnShape sh, BnColumns bn, con
     }
   }
   pack_column<T, ST, PHILOX>(
-      x, sh, t, oct, mn, mx, bits, word_offsets, packed, scale, mn_out, (const T*)nullptr, key, lane, ahead,
+      x, sh, t, oct, mn, mx, bits, word_offsets, packed, scale, mn_out, (const T*)nullptr, key, lane,
+      PHILOX && sizeof(T) == 2 && ahead,
       [&](int n, const Oct<T> (&v)[kBundle]) {
         T* sample = y + (int64_t)n * sh.F;
 #pragma unroll
@@ -681,7 +682,9 @@ int launch_forward(const void* x, void* y, const BnForward& f, const ColumnShape
       return st;
   }
   auto pack = f.stochastic ? bn_column_pack_kernel<T, ST, SUB, true, EDGE> : bn_column_pack_kernel<T, ST, SUB, false, EDGE>;
-  // 16-bit activations that do not stay in the L2: requested there a sample ahead of the loads, while y goes out.
+  // Large 16-bit activations: requested into the L2 a sample ahead of the loads, while y goes out.  The line lies between
+  // the sizes that were measured, 15 MB and 40 MB.  The kernels of float32 and of rounding to nearest are compiled without it:
+  // its branch alone cost 512 x 256 x 28 x 28 of float32 240 -> 250 us (whole pass), and rounding to nearest 123.7 -> 126.5.
   // float16 256 x 64 x 56 x 56 41.5 -> 37.6 us (two samples ahead 38.0, three 38.3), 256 x 128 x 28 x 28 21.8 -> 19.8, 200 x
   // 64 x 40 x 40 18.1 -> 16.8; at 15 MB (64 x 100 x 35 x 35) 19.3 -> 19.6, and float32 pays: 76.5 -> 80.
   const bool ahead = sizeof(T) == 2 && (int64_t)sh.N * sh.F >= ((int64_t)16 << 20);
