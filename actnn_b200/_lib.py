@@ -115,9 +115,9 @@ _tickets = {}
 
 
 def ticket(device: torch.device) -> torch.Tensor:
-    """256 zeroed bytes per (device, current stream) for the kernels of ``actnn_compress_mixed_prestat_kept`` and
-    ``actnn_batch_norm_codes_forward``, which run in stream order and leave it at zero, so it never needs clearing
-    again.  While the stream is being captured: a block of the graph's own, cleared by every replay.  A kept one
+    """256 zeroed bytes per (device, current stream) for the kernels of ``actnn_compress_mixed_prestat_kept``,
+    ``actnn_batch_norm_codes_forward`` and ``actnn_sample_sumsq_mean``, which run in stream order and leave it at zero,
+    so it never needs clearing again.  While the stream is being captured: a block of the graph's own, cleared by every replay.  A kept one
     could not be shared with a graph: made during a capture it is only cleared when that graph runs, and a
     replay on another stream would use it at the same time."""
     idx = device.index if device.index is not None else torch.cuda.current_device()

@@ -323,7 +323,8 @@ def batch_norm_stats_minimax(input, weight, bias, running_mean, running_var, mom
     Returns ``(mn, mx, mean, invstd)`` -- ``mn`` / ``mx`` shaped ``[N, G, 1]`` in the input's
     dtype, ``mean`` / ``invstd`` float32 ``[C]`` -- or ``None`` when the geometry is not covered
     (then the caller takes the two-read path).  ``running_mean`` / ``running_var`` are updated
-    when given; ``out``: optional float32 buffer of >= 2 * C elements for mean then invstd."""
+    when given; ``out``: optional float32 buffer of >= 2 * C elements for mean then invstd.
+    ``weight`` and ``bias`` are not looked at (they are in the calls programs have)."""
     if not input.is_cuda or not input.is_contiguous() or input.dim() < 2:
         return None
     for t in (running_mean, running_var):
