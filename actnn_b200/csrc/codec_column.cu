@@ -6,7 +6,7 @@
 //
 // Bound by HBM at large sizes and by launches at small ones.  float16, compress and decompress of
 // 100 x 192 x 35 x 35 (918.75 groups a sample): 127.1 -> 60.6 us, of which the padded copy was 18 and the
-// cut-out copy 49 (54.3 with the pack in the order of the stream); 8 x 16 x 14 x 14: 81.1 -> 46.4 us (seven kernels -> four).
+// cut-out copy 49 (52.1 with the pack in the order of the stream); 8 x 16 x 14 x 14: 81.1 -> 46.4 us (seven kernels -> four).
 #include "column.cuh"
 
 namespace actnn {
